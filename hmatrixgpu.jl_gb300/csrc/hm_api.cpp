@@ -81,7 +81,18 @@ int upload_units(HMatrix &H) {
   H.dfree(H.dp.warp_begin);
   int rc;
   if ((rc = upload(H, &H.dp.units, p.units))) return rc;
-  if ((rc = upload(H, &H.dp.vunits, p.vunits))) return rc;
+  if (H.dp.v_dynamic) {
+    // tickets: larger units first (by 8 KB, so that units of one source stay
+    // together), because the longest rows, one unit each, would end the pass alone
+    const int64_t es = 16 / p.vec;
+    std::vector<VUnit> vs = p.vunits;
+    std::stable_sort(vs.begin(), vs.end(), [&](const VUnit &a, const VUnit &b) {
+      return static_cast<int64_t>(a.stride) * a.nrows * es / 8192 > static_cast<int64_t>(b.stride) * b.nrows * es / 8192;
+    });
+    if ((rc = upload(H, &H.dp.vunits, vs))) return rc;
+  } else if ((rc = upload(H, &H.dp.vunits, p.vunits))) {
+    return rc;
+  }
   if ((rc = upload(H, &H.dp.warp_begin, p.warp_begin))) return rc;
   H.dp.nunits = static_cast<int32_t>(p.units.size());
   H.dp.nvunits = static_cast<int32_t>(p.vunits.size());

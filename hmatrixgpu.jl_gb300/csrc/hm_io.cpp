@@ -308,8 +308,8 @@ extern "C" int hmgpu_hmatrix_load(const char *path, hmgpu_hmatrix **out) {
   uint64_t sum = 0;
   r.val(sum);
   if (!r.ok || sum != want) return hm::fail(HMGPU_ERR_INVALID, std::string(path) + ": checksum mismatch");
-  if ((rc = hm::upload_plan(*H, tmap0, smap0, zero_row))) return rc;
   H->dp.v_dynamic = v_dynamic != 0;
+  if ((rc = hm::upload_plan(*H, tmap0, smap0, zero_row))) return rc;
   if (H->opt.precision == HMGPU_MIXED && (rc = hm::build_tc(*H))) return rc;
   cudaError_t e = cudaDeviceSynchronize();
   if (e != cudaSuccess) return hm::cuda_fail(e, "loading an H-matrix");

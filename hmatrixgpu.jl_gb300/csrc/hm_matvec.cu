@@ -46,6 +46,12 @@ __device__ __forceinline__ double2 ld_stream(const double2 *p) {
   return v;
 }
 
+// Programmatic dependent launch: a kernel of the product may start while the one
+// before it ends. It waits here, before it touches anything that earlier kernels
+// write (or still read), until they are complete; from then on the next may start.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 __device__ __forceinline__ float fma_(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 __device__ __forceinline__ double fma_(double a, double b, double c) { return __fma_rn(a, b, c); }
 
@@ -106,6 +112,8 @@ __global__ void permute_x_kernel(const T *__restrict__ x, const int32_t *__restr
                                  int64_t n, int64_t x_len, T *__restrict__ xt,
                                  int32_t *__restrict__ counter) {
   int64_t j = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
+  pdl_wait();
+  pdl_trigger();
   if (j == 0) {
     counter[0] = 0;  // near/U row units
     counter[8] = 0;  // V units (dynamic schedule)
@@ -117,11 +125,13 @@ __global__ void permute_x_kernel(const T *__restrict__ x, const int32_t *__restr
 // ---------------------------------------------------------------------------
 // V pass. A unit is a run of rank rows of one block; `lanes` lanes share a
 // row and 32/lanes rows run side by side. Row storage is phase-aligned with
-// XT, so element p of the row pairs with XT[x_off + p]. Two schedules, picked
-// per matrix by the autotuner: each warp owns a contiguous, byte-balanced
-// range of units (planned on the host), or warps take units one at a time
-// from a ticket counter (the next ticket is drawn before the current unit
-// runs), which evens out uneven speeds on matrices with long rows.
+// XT, so element p of the row pairs with XT[x_off + p]. Warps take units one at
+// a time from a ticket counter, largest first (the first one is the warp's own
+// number, the next ticket is drawn before the current unit runs). The other
+// schedule, which a caller or the autotuner may set: each warp owns a
+// contiguous, byte-balanced range of units, planned on the host. Measured in us
+// with tickets / ranges: film 2^20 FP32 507 / 540, 40,960-point cube FP64
+// 372 / 427, batch of 12 spheres 77 / 96, one sphere of 20,011 points 31 / 29.
 // ---------------------------------------------------------------------------
 // Six CTAs per SM (40 registers) and four loads in flight per lane: the pass
 // is bound by memory latency, like the near/U pass.
@@ -183,61 +193,13 @@ __global__ void __launch_bounds__(kThreads, 6) v_pass_kernel(const T *__restrict
                                                           const VUnit *__restrict__ units,
                                                           const int32_t *__restrict__ warp_begin,
                                                           T *__restrict__ xt) {
-  using VT = typename Vec16<T>::type;
-  constexpr int VEC = Vec16<T>::N;
   const int warp = static_cast<int>((blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x) >> 5);
   const int lane = threadIdx.x & 31;
   const int u0 = warp_begin[warp], u1 = warp_begin[warp + 1];
-  for (int u = u0; u < u1; u++) {
-    const VUnit U = units[u];
-    const int g = U.lanes, slot = lane / g, sub = lane - slot * g, per = 32 / g;
-    const int nv = U.stride / VEC;
-    const VT *X = reinterpret_cast<const VT *>(xt + U.x_off);
-    for (int k0 = 0; k0 < U.nrows; k0 += per) {
-      const int k = k0 + slot;
-      T acc = T(0);
-      if (k < U.nrows) {
-        const VT *row = reinterpret_cast<const VT *>(V + U.v_off + static_cast<int64_t>(k) * U.stride);
-        int p = sub;
-        for (; p + 3 * g < nv; p += 4 * g) {  // four 16-byte loads of V in flight per lane
-          VT a0 = ld_stream(row + p), a1 = ld_stream(row + p + g);
-          VT a2 = ld_stream(row + p + 2 * g), a3 = ld_stream(row + p + 3 * g);
-          VT b0 = __ldg(X + p), b1 = __ldg(X + p + g), b2 = __ldg(X + p + 2 * g), b3 = __ldg(X + p + 3 * g);
-          const T *ea0 = reinterpret_cast<const T *>(&a0), *eb0 = reinterpret_cast<const T *>(&b0);
-          const T *ea1 = reinterpret_cast<const T *>(&a1), *eb1 = reinterpret_cast<const T *>(&b1);
-          const T *ea2 = reinterpret_cast<const T *>(&a2), *eb2 = reinterpret_cast<const T *>(&b2);
-          const T *ea3 = reinterpret_cast<const T *>(&a3), *eb3 = reinterpret_cast<const T *>(&b3);
-#pragma unroll
-          for (int q = 0; q < VEC; q++) acc = fma_(ea0[q], eb0[q], acc);
-#pragma unroll
-          for (int q = 0; q < VEC; q++) acc = fma_(ea1[q], eb1[q], acc);
-#pragma unroll
-          for (int q = 0; q < VEC; q++) acc = fma_(ea2[q], eb2[q], acc);
-#pragma unroll
-          for (int q = 0; q < VEC; q++) acc = fma_(ea3[q], eb3[q], acc);
-        }
-        for (; p + g < nv; p += 2 * g) {
-          VT a0 = ld_stream(row + p), a1 = ld_stream(row + p + g);
-          VT b0 = __ldg(X + p), b1 = __ldg(X + p + g);
-          const T *ea0 = reinterpret_cast<const T *>(&a0), *eb0 = reinterpret_cast<const T *>(&b0);
-          const T *ea1 = reinterpret_cast<const T *>(&a1), *eb1 = reinterpret_cast<const T *>(&b1);
-#pragma unroll
-          for (int q = 0; q < VEC; q++) acc = fma_(ea0[q], eb0[q], acc);
-#pragma unroll
-          for (int q = 0; q < VEC; q++) acc = fma_(ea1[q], eb1[q], acc);
-        }
-        if (p < nv) {
-          VT a0 = ld_stream(row + p);
-          VT b0 = __ldg(X + p);
-          const T *ea0 = reinterpret_cast<const T *>(&a0), *eb0 = reinterpret_cast<const T *>(&b0);
-#pragma unroll
-          for (int q = 0; q < VEC; q++) acc = fma_(ea0[q], eb0[q], acc);
-        }
-      }
-      for (int o = g >> 1; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-      if (sub == 0 && k < U.nrows) xt[U.t_off + k] = acc;
-    }
-  }
+  if (u0 >= u1) return;
+  pdl_wait();  // XT holds the permuted x
+  pdl_trigger();
+  for (int u = u0; u < u1; u++) v_unit(V, units[u], xt, lane);
 }
 
 template <typename T>
@@ -246,20 +208,24 @@ __global__ void __launch_bounds__(kThreads, 6) v_pass_dyn_kernel(const T *__rest
                                                               int32_t nunits, T *__restrict__ xt,
                                                               int32_t *__restrict__ ticket) {
   const int lane = threadIdx.x & 31;
-  int u = 0;
-  if (lane == 0) u = atomicAdd(ticket, 1);
-  u = __shfl_sync(0xffffffffu, u, 0);
+  const int nwarps = static_cast<int>((gridDim.x * blockDim.x) >> 5);
+  int u = static_cast<int>((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+  if (u >= nunits) return;
+  pdl_wait();  // XT holds the permuted x, the ticket is zero
+  pdl_trigger();
   while (u < nunits) {
     int next = 0;
-    if (lane == 0) next = atomicAdd(ticket, 1);
+    if (lane == 0) next = nwarps + atomicAdd(ticket, 1);
     v_unit(V, units[u], xt, lane);
     u = __shfl_sync(0xffffffffu, next, 0);
   }
 }
 
 // ---------------------------------------------------------------------------
-// Near/U pass. CTAs take row units (rows of one tile) from a ticket counter,
-// tiles with the most columns first. The CTA gathers the tile's vector
+// Near/U pass. CTAs take row units (rows of one tile) from a ticket counter
+// (the first one is the CTA's own number, its tables are read while the V pass
+// ends, and the next ticket is drawn while the current unit streams), tiles
+// with the most columns first. The CTA gathers the tile's vector
 // entries (x for dense columns, t for rank columns) into shared memory once
 // per unit (once per 16 rows when the tile needs several chunks of entries);
 // then each warp streams one or two whole rows of the tile's
@@ -297,19 +263,21 @@ __global__ void __launch_bounds__(kThreads, 6) du_rows_kernel(DuArgs<T> a) {
   constexpr int CH = DuCols<T>::value;
   __shared__ __align__(16) T vals[CH];
   __shared__ Seg ssegs[kDuSegs];
-  __shared__ int32_t s_ticket[2];
+  __shared__ int32_t s_ticket;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  for (int it = 0;; it++) {
-    if (tid == 0) s_ticket[it & 1] = atomicAdd(a.counter, 1);
-    __syncthreads();
-    const int32_t u = s_ticket[it & 1];
-    if (u >= a.nunits) break;
+  for (int32_t u = blockIdx.x; u < a.nunits;) {
     const RowUnit U = a.units[u];
     const TileDesc d = a.tiles[U.tile];
     const bool seg_smem = d.nseg <= kDuSegs;
     if (seg_smem)
       for (int s = tid; s < d.nseg; s += kThreads) ssegs[s] = a.segs[d.seg0 + s];
     const Seg *S = seg_smem ? ssegs : a.segs + d.seg0;
+    if (u == static_cast<int32_t>(blockIdx.x)) {
+      pdl_wait();  // t is complete, the ticket is zero
+      pdl_trigger();
+    }
+    int32_t next = 0;
+    if (tid == 0) next = static_cast<int32_t>(gridDim.x) + atomicAdd(a.counter, 1);
     // Rows 16 at a time (a warp per row pair); a unit has more than 16 rows
     // only when its tile fits one chunk of entries, which are then gathered
     // once for all its rows.
@@ -394,6 +362,9 @@ __global__ void __launch_bounds__(kThreads, 6) du_rows_kernel(DuArgs<T> a) {
         if (hb) a.y[a.tmap0[d.row0 + ib]] = yb;
       }
     }
+    if (tid == 0) s_ticket = next;
+    __syncthreads();  // the entries and segments are no longer read
+    u = s_ticket;
   }
 }
 
@@ -417,6 +388,22 @@ int occupancy_du(bool f64, bool comp) {
   return n > 0 ? n : 1;
 }
 
+// A launch that may overlap the end of the kernel before it on the stream; the
+// kernel calls pdl_wait().
+template <typename... P, typename... A>
+static cudaError_t launch_pdl(void (*k)(P...), int grid, cudaStream_t s, A... args) {
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t c{};
+  c.gridDim = dim3(static_cast<unsigned>(grid));
+  c.blockDim = dim3(kThreads);
+  c.stream = s;
+  c.attrs = &at;
+  c.numAttrs = 1;
+  return cudaLaunchKernelEx(&c, k, static_cast<P>(args)...);
+}
+
 template <typename T, bool COMP>
 static cudaError_t run(const DevPlan &p, const T *panels, const T *vdata, T *xt, const T *x, T *y,
                        int grid_v, int grid_du, cudaStream_t s, cudaEvent_t *ev, int *launches) {
@@ -424,19 +411,22 @@ static cudaError_t run(const DevPlan &p, const T *panels, const T *vdata, T *xt,
   if (gp > 4096) gp = 4096;
   int nl = 0;
   if (ev) cudaEventRecord(ev[0], s);
-  permute_x_kernel<T><<<gp, kThreads, 0, s>>>(x, p.smap0, p.n, p.x_len, xt, p.counter);
+  cudaError_t e = launch_pdl(permute_x_kernel<T>, gp, s, x, p.smap0, p.n, p.x_len, xt, p.counter);
+  if (e != cudaSuccess) return e;
   nl++;
   if (ev) cudaEventRecord(ev[1], s);
   if (!p.warp_begin_empty) {
     if (p.v_dynamic)
-      v_pass_dyn_kernel<T><<<grid_v, kThreads, 0, s>>>(vdata, p.vunits, p.nvunits, xt, p.counter + 8);
+      e = launch_pdl(v_pass_dyn_kernel<T>, grid_v, s, vdata, p.vunits, p.nvunits, xt, p.counter + 8);
     else
-      v_pass_kernel<T><<<grid_v, kThreads, 0, s>>>(vdata, p.vunits, p.warp_begin, xt);
+      e = launch_pdl(v_pass_kernel<T>, grid_v, s, vdata, p.vunits, p.warp_begin, xt);
+    if (e != cudaSuccess) return e;
     nl++;
   }
   if (ev) cudaEventRecord(ev[2], s);
   DuArgs<T> a{panels, p.tiles, p.units, p.nunits, p.segs, xt, p.tmap0, y, p.counter};
-  du_rows_kernel<T, COMP><<<grid_du, kThreads, 0, s>>>(a);
+  e = launch_pdl(du_rows_kernel<T, COMP>, grid_du, s, a);
+  if (e != cudaSuccess) return e;
   nl++;
   if (ev) cudaEventRecord(ev[3], s);
   if (launches) *launches = nl;

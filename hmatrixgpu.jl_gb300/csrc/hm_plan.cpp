@@ -10,10 +10,10 @@
 //     rows (dense-block columns, then low-rank U columns), rows padded to 16
 //     bytes, with a list of segments telling where each column's vector entry
 //     lives in XT = [x | t];
-//   * row units: runs of at most kUnitRows rows of one tile, largest first;
+//   * row units: runs of 16 to 64 rows of one tile, largest first;
 //   * the V factors row by row, each row phase-aligned with the permuted x so
 //     that a 16-byte load of V pairs with a 16-byte load of x;
-//   * a static, byte-balanced split of the V rows over the resident warps.
+//   * units of V rows, and their byte-balanced split over the resident warps.
 #include <algorithm>
 #include <numeric>
 
@@ -23,7 +23,6 @@ namespace hm {
 
 static constexpr int kMaxTileRows = 128;
 static constexpr int64_t kVUnitBytes = 64 * 1024;
-static constexpr int32_t kUnitRows = 16;  // rows per near/U unit (2 per warp of 8)
 // multi-RHS V items: at most kMVRows rows (the tensor-core items' limit) and
 // about kMVEntries stored entries
 static constexpr int32_t kMVRows = 64;
@@ -53,18 +52,45 @@ void make_units(Plan &p, int32_t unit_rows) {
   }
 }
 
+// Rows per near/U unit: the most (a tile's entries are gathered once per unit)
+// that still give each of the resident CTAs two units; 16, two rows per warp, at
+// least. Near/U pass in us with 16 / 64 rows: film 2^20 1427 / 1284, batch of 12
+// spheres 125 / 107; with 24 tiles (1000 points, FP64) 8.2 / 14.
+static int32_t default_unit_rows(Plan &p, int nwarps) {
+  for (int32_t rows : {64, 32}) {
+    make_units(p, rows);
+    if (static_cast<int64_t>(p.units.size()) >= 2 * (nwarps / 8)) return rows;
+  }
+  return 16;
+}
+
 void make_vunits(Plan &p, int64_t unit_bytes, int nwarps) {
   const int esize = 16 / p.vec;
   p.vunits.clear();
   p.vunit_bytes = unit_bytes;
   std::vector<int64_t> uweight;
+  int64_t bytes = 0;
+  for (const VGroup &g : p.vgroups) bytes += static_cast<int64_t>(g.stride) * esize * g.rows;
+  // Units of a quarter of a resident warp's share of the bytes, at least 8 KB (a
+  // ticket each: all of them come from one address), or the whole share where that
+  // is less; unit_bytes at most. With 64 KB units for every size, most warps had
+  // none on small matrices (V pass of a 20,011-point sphere 96 us, now 31 us).
+  const int64_t share = bytes / std::max(1, nwarps);
+  unit_bytes = std::min(unit_bytes, std::max<int64_t>(1024, std::min(share, std::max<int64_t>(8192, share / 4))));
+  // Lanes per row: a power of two leaving each lane at least this many 16-byte
+  // vectors of the row (at most a warp per row). Fewer lanes per row leave less
+  // idle at the row's end and in the sum over the lanes; in FP64 that counts
+  // more, since the FP64 pipe takes as long for one active lane as for 32. V pass
+  // in us with 4 / 8 / 16 vectors a lane: film 2^20 FP32 580 / 507 / 512, batch of
+  // 12 spheres 113 / 77 / 81; 40,960-point cube FP64 673 / 497 / 372.
+  const int32_t lane_vecs = p.vec == 2 ? 16 : 8;
   for (const VGroup &g : p.vgroups) {
-    // lanes per row: a power of two leaving each lane at least four 16-byte
-    // vectors of the row, so that loads overlap (at most a warp per row)
     int32_t nv = g.stride / p.vec, lanes = 1;
-    while (lanes * 4 < nv && lanes < 32) lanes *= 2;
+    while (lanes * lane_vecs < nv && lanes < 32) lanes *= 2;
     const int64_t row_bytes = static_cast<int64_t>(g.stride) * esize;
-    const int32_t rows_per = static_cast<int32_t>(std::max<int64_t>(1, unit_bytes / row_bytes));
+    // whole steps of 32 / lanes rows
+    const int32_t step = 32 / lanes;
+    const int32_t rows_per = static_cast<int32_t>(std::max<int64_t>(1, (unit_bytes / row_bytes + step - 1) / step)) * step;
     for (int32_t k0 = 0; k0 < g.rows; k0 += rows_per) {
       VUnit u{};
       u.v_off = g.v_off + static_cast<int64_t>(k0) * g.stride;
@@ -252,7 +278,7 @@ void make_plan(const BlockSet &bs, int vec, int nwarps, const std::vector<int64_
     return static_cast<int64_t>(p.tiles[a].ncols) > static_cast<int64_t>(p.tiles[b].ncols);
   });
   p.tile_order = order;
-  make_units(p, kUnitRows);
+  make_units(p, default_unit_rows(p, nwarps));
 
   // ---- V pass -----------------------------------------------------------------------
   p.v_off.assign(na, 0);
@@ -485,7 +511,7 @@ int combine_plans(const std::vector<const Plan *> &plans, const std::vector<cons
   std::iota(P.tile_order.begin(), P.tile_order.end(), 0);
   std::stable_sort(P.tile_order.begin(), P.tile_order.end(),
                    [&](int32_t a, int32_t b) { return P.tiles[a].ncols > P.tiles[b].ncols; });
-  make_units(P, plans[0]->unit_rows);
+  make_units(P, default_unit_rows(P, nwarps));
   make_vunits(P, plans[0]->vunit_bytes, nwarps);
   std::stable_sort(P.mv_items.begin(), P.mv_items.end(), [](const MVItem &a, const MVItem &b) {
     return static_cast<int64_t>(a.nrows) * a.ncols > static_cast<int64_t>(b.nrows) * b.ncols;

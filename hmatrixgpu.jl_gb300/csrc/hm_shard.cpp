@@ -131,8 +131,8 @@ static int make_shard(const HMatrix &H, int32_t rank, int32_t world, HMatrix &S)
   std::vector<int32_t> smap0(static_cast<size_t>(n)), tmap0(static_cast<size_t>(m), -1);
   std::iota(smap0.begin(), smap0.end(), 0);
   for (int64_t r = S.shard_row0; r < S.shard_row1; r++) tmap0[r] = static_cast<int32_t>(r - S.shard_row0);
-  if ((rc = upload_plan(S, tmap0, smap0, H.dp.zero_row))) return rc;
   S.dp.v_dynamic = H.dp.v_dynamic;
+  if ((rc = upload_plan(S, tmap0, smap0, H.dp.zero_row))) return rc;
   S.plan.unit_rows = p.unit_rows;
   return setup_grids(S);
 }

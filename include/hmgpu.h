@@ -386,9 +386,10 @@ int hmgpu_graph_free(hmgpu_graph *G);
  * threshold (1 << 30: never), 1 if it came from the cache. */
 int hmgpu_hmatrix_autotune(hmgpu_hmatrix *H, const char *cache_path, int32_t *result);
 /* The product parameters in force (no counterpart in the reference): rows per
- * near/U unit, V unit KiB, multi-RHS threshold, V schedule (0: each warp owns
- * a byte-balanced range of V units, 1: warps take V units from a ticket
- * counter; the autotuner times both). Writes min(n, 4) values. */
+ * near/U unit, V unit KiB at most (small matrices take smaller units), multi-RHS
+ * threshold, V schedule (0: each warp owns a byte-balanced range of V units, 1:
+ * warps take V units from a ticket counter, the default; the autotuner times
+ * both). Writes min(n, 4) values. */
 int hmgpu_hmatrix_tuning(const hmgpu_hmatrix *H, int32_t *values, int32_t n);
 /* Sets those four parameters directly (for instance from an earlier autotune
  * on the same structure); n must be 4. Results do not depend on them. */
