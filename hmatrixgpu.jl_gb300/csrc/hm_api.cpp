@@ -111,7 +111,6 @@ int upload_plan(HMatrix &H, const std::vector<int32_t> &tmap0, const std::vector
   if ((rc = H.dalloc(&H.xt, p.xt_len * es))) return rc;
   cudaMemset(H.xt, 0, p.xt_len * es);
   if ((rc = upload(H, &H.dp.tiles, p.tiles))) return rc;
-  if ((rc = upload(H, &H.dp.tile_order, p.tile_order))) return rc;
   if ((rc = upload(H, &H.dp.segs, p.segs))) return rc;
   if ((rc = upload_units(H))) return rc;
   if ((rc = upload(H, &H.dp.tmap0, tmap0))) return rc;
@@ -131,9 +130,40 @@ int upload_plan(HMatrix &H, const std::vector<int32_t> &tmap0, const std::vector
   cudaMemset(H.dp.counter, 0, 64);
   H.dp.status = H.dp.counter + 4;  // its own 16-byte slot of the same allocation
   H.dp.ntiles = static_cast<int32_t>(p.tiles.size());
+  {  // rows of a tile in near-equal parts of at most 64, or 32 or 16 where that is
+    // what gives each SM four (the smallest parts re-read the XT rows most often)
+    const int64_t want = 4 * static_cast<int64_t>(H.num_sms);
+    std::vector<int64_t> map0(p.tiles.size());
+    int64_t ncm = 0;
+    for (size_t t = 0; t < map0.size(); t++) {
+      map0[t] = ncm;
+      ncm += p.tiles[t].ncols;
+    }
+    std::vector<MUnit> mu;
+    for (int32_t rows = 64; rows >= 16; rows /= 2) {
+      mu.clear();
+      for (int32_t ti : p.tile_order) {
+        const TileDesc &d = p.tiles[ti];
+        const int32_t parts = (d.m + rows - 1) / rows;
+        for (int32_t q = 0; q < parts; q++) {
+          const int32_t i0 = static_cast<int32_t>(static_cast<int64_t>(d.m) * q / parts);
+          const int32_t i1 = static_cast<int32_t>(static_cast<int64_t>(d.m) * (q + 1) / parts);
+          mu.push_back(MUnit{d.data_off + static_cast<int64_t>(i0) * d.ld, map0[ti], d.row0 + i0, i1 - i0, d.ld, d.ncols});
+        }
+      }
+      if (static_cast<int64_t>(mu.size()) >= want) break;
+    }
+    if ((rc = upload(H, &H.dp.munits, mu))) return rc;
+    H.dp.nmunits = static_cast<int32_t>(mu.size());
+  }
   {  // device order: by first XT row, so pieces reading the same x rows share them in L2
     std::vector<MVItem> ms = p.mv_items;
-    std::stable_sort(ms.begin(), ms.end(), [](const MVItem &a, const MVItem &b) { return a.x_off < b.x_off; });
+    std::stable_sort(ms.begin(), ms.end(), [](const MVItem &a, const MVItem &b) {
+      const bool wa = a.ncols > kMvWarpCols, wb = b.ncols > kMvWarpCols;
+      return wa != wb ? wa : a.x_off < b.x_off;
+    });
+    H.dp.nmv_big = static_cast<int32_t>(
+        std::count_if(ms.begin(), ms.end(), [](const MVItem &a) { return a.ncols > kMvWarpCols; }));
     if ((rc = upload(H, &H.dp.mv_items, ms))) return rc;
   }
   if ((rc = upload(H, &H.dp.mv_reduce, p.mv_reduce))) return rc;
@@ -530,11 +560,21 @@ extern "C" int hmgpu_matvec(hmgpu_hmatrix *h, const void *x, void *y, int64_t nr
       if (cudaError_t e = hm::encode_xts_map(H.tc, 64)) return hm::cuda_fail(e, "tensor map of XTS");
     }
     if (!tc && !H.xt_multi) {
+      std::vector<int64_t> col0(H.plan.tiles.size());
+      int64_t ncm = 0;
+      for (size_t t = 0; t < col0.size(); t++) {
+        col0[t] = ncm;
+        ncm += H.plan.tiles[t].ncols;
+      }
+      if ((rc = hm::upload(H, &H.dp.mcol0, col0)) ||
+          (rc = H.dalloc(reinterpret_cast<void **>(&H.dp.mcolmap), ncm * sizeof(int32_t))))
+        return rc;
+      if (cudaError_t e = hm::launch_colmap(H.dp.tiles, H.dp.ntiles, H.dp.segs, H.dp.mcol0, H.dp.mcolmap, s))
+        return hm::cuda_fail(e, "column map");
       if ((rc = H.dalloc(&H.xt_multi, H.plan.xt_len * per * es)) ||
           (rc = H.dalloc(&H.p_multi, std::max<int64_t>(H.plan.p_rows, 1) * per * es)))
         return rc;
       cudaMemsetAsync(H.xt_multi, 0, H.plan.xt_len * per * es, s);
-      H.grid_du_multi = H.num_sms * hm::occupancy_du_multi(f64);
     }
     for (int64_t k0 = 0; k0 < nrhs; k0 += per) {
       cudaEvent_t *ev;
@@ -561,7 +601,7 @@ extern "C" int hmgpu_matvec(hmgpu_hmatrix *h, const void *x, void *y, int64_t nr
         }
         e = hm::launch_matvec_multi(f64, H.dp, H.panels, H.vdata, xt, H.p_multi,
                                     static_cast<const char *>(x) + k0 * ldx * es, ldx, nr,
-                                    static_cast<char *>(y) + k0 * ldy * es, ldy, H.grid_du_multi, s, ev, &nl);
+                                    static_cast<char *>(y) + k0 * ldy * es, ldy, H.num_sms, s, ev, &nl);
       }
       if (e != cudaSuccess) return hm::cuda_fail(e, "multi-RHS matvec launch");
       if (H.profiling) H.prof_launches += nl;

@@ -14,15 +14,19 @@ struct DevPlan {
   int32_t ntiles = 0;
   RowUnit *units = nullptr;      // near/U pass work
   int32_t nunits = 0;
-  int32_t *tile_order = nullptr; // tiles by decreasing work (multi-RHS pass)
+  MUnit *munits = nullptr;       // multi-RHS near/U work: at most 64 rows of a tile, widest tiles first
+  int32_t nmunits = 0;
+  int32_t *mcolmap = nullptr;    // XT row of every tile column, tile after tile (first multi-RHS product)
+  int64_t *mcol0 = nullptr;      // first entry of each tile
   VUnit *vunits = nullptr;
   int32_t nvunits = 0;
   int32_t *warp_begin = nullptr;
   int32_t nwarps = 0;
   bool warp_begin_empty = true;  // no V units (no low-rank blocks)
   bool v_dynamic = true;         // V units from a ticket counter instead of warp ranges
-  MVItem *mv_items = nullptr;  // multi-RHS V items, largest first
+  MVItem *mv_items = nullptr;  // multi-RHS V items: those of many columns first
   int32_t nmv = 0;
+  int32_t nmv_big = 0;         // items of more than kMvWarpCols columns
   MVReduce *mv_reduce = nullptr;
   int32_t nmvr = 0;
   int64_t p_rows = 0;
@@ -37,6 +41,7 @@ struct DevPlan {
 };
 
 constexpr int kThreads = 256;  // threads per CTA of the product kernels
+constexpr int kMvWarpCols = 128;  // a multi-RHS V item of at most this many columns goes to one warp (FP32)
 
 // Resident CTAs per SM of the V pass and of the near/U pass for an element type.
 int occupancy_v(bool f64);
@@ -113,10 +118,12 @@ cudaError_t launch_pack_tc(const TcPack *jobs, int64_t njobs, const float *src, 
 cudaError_t launch_matvec_tc(const DevPlan &p, const DevTc &t, const float *X, int64_t ldx, int nr,
                              float *Y, int64_t ldy, cudaStream_t s, cudaEvent_t *ev, int *launches);
 
-int occupancy_du_multi(bool f64);
+// XT row of every tile column (tile t's at colmap[col0[t]]...), from the segments.
+cudaError_t launch_colmap(const TileDesc *tiles, int32_t ntiles, const Seg *segs, const int64_t *col0, int32_t *colmap,
+                          cudaStream_t s);
 // P: partial rows of cut V groups (p_rows x rhs_per_pass() values).
 cudaError_t launch_matvec_multi(bool f64, const DevPlan &p, const void *panels, const void *vdata,
                                 void *xt, void *P, const void *X, int64_t ldx, int nr, void *Y,
-                                int64_t ldy, int grid_du, cudaStream_t s, cudaEvent_t *ev,
+                                int64_t ldy, int num_sms, cudaStream_t s, cudaEvent_t *ev,
                                 int *launches);
 }  // namespace hm

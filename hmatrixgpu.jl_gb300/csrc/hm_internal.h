@@ -93,6 +93,15 @@ struct RowUnit {
   int32_t tile, i0, i1, pad;
 };
 
+// A unit of the multi-right-hand-side near/U pass: m <= 64 rows of one tile.
+struct MUnit {
+  int64_t data_off;  // element offset of the first row
+  int64_t map;       // first entry of the tile in the column map
+  int32_t row0;      // first permuted row
+  int32_t m, ld, ncols;
+};
+static_assert(sizeof(MUnit) == 32, "MUnit layout");
+
 // A unit of the V pass: rows [0, nrows) of one low-rank block, each row a
 // phase-aligned run of `stride` elements dotted with XT[x_off : x_off+stride).
 struct VUnit {

@@ -14,6 +14,7 @@
 #include <cuda_runtime.h>
 
 #include "hm_device.h"
+#include "hm_launch.cuh"
 
 namespace hm {
 
@@ -45,12 +46,6 @@ __device__ __forceinline__ double2 ld_stream(const double2 *p) {
                : "l"(p));
   return v;
 }
-
-// Programmatic dependent launch: a kernel of the product may start while the one
-// before it ends. It waits here, before it touches anything that earlier kernels
-// write (or still read), until they are complete; from then on the next may start.
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 __device__ __forceinline__ float fma_(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 __device__ __forceinline__ double fma_(double a, double b, double c) { return __fma_rn(a, b, c); }
@@ -388,22 +383,6 @@ int occupancy_du(bool f64, bool comp) {
   return n > 0 ? n : 1;
 }
 
-// A launch that may overlap the end of the kernel before it on the stream; the
-// kernel calls pdl_wait().
-template <typename... P, typename... A>
-static cudaError_t launch_pdl(void (*k)(P...), int grid, cudaStream_t s, A... args) {
-  cudaLaunchAttribute at{};
-  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at.val.programmaticStreamSerializationAllowed = 1;
-  cudaLaunchConfig_t c{};
-  c.gridDim = dim3(static_cast<unsigned>(grid));
-  c.blockDim = dim3(kThreads);
-  c.stream = s;
-  c.attrs = &at;
-  c.numAttrs = 1;
-  return cudaLaunchKernelEx(&c, k, static_cast<P>(args)...);
-}
-
 template <typename T, bool COMP>
 static cudaError_t run(const DevPlan &p, const T *panels, const T *vdata, T *xt, const T *x, T *y,
                        int grid_v, int grid_du, cudaStream_t s, cudaEvent_t *ev, int *launches) {
@@ -411,21 +390,21 @@ static cudaError_t run(const DevPlan &p, const T *panels, const T *vdata, T *xt,
   if (gp > 4096) gp = 4096;
   int nl = 0;
   if (ev) cudaEventRecord(ev[0], s);
-  cudaError_t e = launch_pdl(permute_x_kernel<T>, gp, s, x, p.smap0, p.n, p.x_len, xt, p.counter);
+  cudaError_t e = launch_pdl(permute_x_kernel<T>, gp, kThreads, 0, s, x, p.smap0, p.n, p.x_len, xt, p.counter);
   if (e != cudaSuccess) return e;
   nl++;
   if (ev) cudaEventRecord(ev[1], s);
   if (!p.warp_begin_empty) {
     if (p.v_dynamic)
-      e = launch_pdl(v_pass_dyn_kernel<T>, grid_v, s, vdata, p.vunits, p.nvunits, xt, p.counter + 8);
+      e = launch_pdl(v_pass_dyn_kernel<T>, grid_v, kThreads, 0, s, vdata, p.vunits, p.nvunits, xt, p.counter + 8);
     else
-      e = launch_pdl(v_pass_kernel<T>, grid_v, s, vdata, p.vunits, p.warp_begin, xt);
+      e = launch_pdl(v_pass_kernel<T>, grid_v, kThreads, 0, s, vdata, p.vunits, p.warp_begin, xt);
     if (e != cudaSuccess) return e;
     nl++;
   }
   if (ev) cudaEventRecord(ev[2], s);
   DuArgs<T> a{panels, p.tiles, p.units, p.nunits, p.segs, xt, p.tmap0, y, p.counter};
-  e = launch_pdl(du_rows_kernel<T, COMP>, grid_du, s, a);
+  e = launch_pdl(du_rows_kernel<T, COMP>, grid_du, kThreads, 0, s, a);
   if (e != cudaSuccess) return e;
   nl++;
   if (ev) cudaEventRecord(ev[3], s);

@@ -5,78 +5,58 @@
 // the pass's columns). XT holds, for every permuted source index and every
 // rank row, the W values of that row contiguously (row-major, 4W bytes per row
 // in FP32). The matrix is read once per pass and every element feeds W FMAs,
-// so the 32-wide form is bound by the CUDA cores' FMA rate and the 8-wide one
-// by HBM.
+// so the 32-wide form is bound by the CUDA cores' FMA rate (FP64: by the FP64
+// pipe at every width) and the 8-wide FP32 one by HBM.
 //
-// Both passes run the same register-tiled micro-kernel over panels of at most
-// 128 rows (multi_panel below); partial sums of the column slices meet in
-// shared memory in a fixed order, so results are deterministic.
+// Both passes run the same micro-kernel (slice_product): one warp multiplies
+// panels of at most 64 rows with W right-hand sides, a register tile of up to
+// 8 x 8 per lane, its operands copied into its own two stages of shared memory,
+// so that warps never wait for one another inside a panel. The warps of a CTA
+// share a panel by column slices, whose sums meet in shared memory in warp order;
+// V items of few columns go to single warps. Results are deterministic.
+//
+// Measured on a film of 262,144 points (633 M stored entries, FP32), us per product with 32,
+// 16 and 8 right-hand sides: 1039, 647 and 558, against 2336 for the form before (CTA-wide
+// stages, 4 x 8 or 2 x 16 tiles, panel entries straight from global memory: L1-bound). The
+// FMAs alone take 580 at the card's FP32 rate, the entries' bytes 374.
 #include <cuda_runtime.h>
 
+#include <type_traits>
+
 #include "hm_device.h"
+#include "hm_launch.cuh"
 
 namespace hm {
 
 constexpr int kRhs = 32;  // right-hand sides per pass at most (row length of XT)
-
-template <typename T, int W>
-struct Cols {
-  static constexpr int value = 16384 / (W * sizeof(T));  // XT rows staged at once
-};
-
-template <typename T>
-struct V4;
-template <>
-struct V4<float> {
-  using type = float4;
-};
-template <>
-struct V4<double> {
-  struct type {
-    double x, y, z, w;
-  };
-};
-
-template <typename T>
-__device__ __forceinline__ void ld4(const T *p, T (&v)[4]) {
-  if constexpr (sizeof(T) == 4) {
-    const float4 a = __ldcs(reinterpret_cast<const float4 *>(p));
-    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
-  } else {
-    const double2 a = __ldcs(reinterpret_cast<const double2 *>(p));
-    const double2 b = __ldcs(reinterpret_cast<const double2 *>(p) + 1);
-    v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
-  }
+// Warps per CTA of the V pass and of the near/U pass, and CTAs per SM (16 warps of 128
+// registers a thread in FP32; FP64 needs more registers for the same tile, and 8 warps keep
+// the FP64 pipe busy). More CTAs hide one another's panel starts and ends better, more warps
+// read longer runs of each panel row: V pass of a 40,960-point cube, 32 wide, FP32, in us with
+// 4 / 8 warps 355 / 400, near/U pass 812 / 663 (film of 262,144: 695 / 719).
+constexpr int kVWarps = 4, kDuWarps = 8;
+template <typename T, int NW>
+constexpr int multi_ctas() {
+  return (sizeof(T) == 4 ? 16 : 8) / NW;
 }
+constexpr int kPanelRows = 64;  // rows of a panel at most
 
-template <typename T, int N>
-__device__ __forceinline__ void ldsn(const T *p, T (&v)[N]) {
-  if constexpr (sizeof(T) == 4) {
-#pragma unroll
-    for (int q = 0; q < N / 4; q++) {
-      const float4 a = reinterpret_cast<const float4 *>(p)[q];
-      v[4 * q] = a.x; v[4 * q + 1] = a.y; v[4 * q + 2] = a.z; v[4 * q + 3] = a.w;
-    }
-  } else {
-#pragma unroll
-    for (int q = 0; q < N / 2; q++) {
-      const double2 a = reinterpret_cast<const double2 *>(p)[q];
-      v[2 * q] = a.x;
-      v[2 * q + 1] = a.y;
-    }
-  }
-}
+// ticket counters (slots of DevPlan::counter): near/U units, V items of CTAs, of warps
+constexpr int kTickets = 3;
+__device__ constexpr int kTicket[kTickets] = {0, 1, 8};
 
 // XT rows from X in its own order: X[j + r ldx] goes to XT[sinv[j] W + r]
 // (0 for r >= nr). Reads of X are coalesced along j and every XT row is written
 // whole; the x-region rows that no source index maps to stay zero (every pass
-// width has its own XT, zeroed once). Also re-arms both ticket counters.
+// width has its own XT, zeroed once). Also re-arms the ticket counters.
 template <typename T, int W>
 __global__ void permute_multi_kernel(const T *__restrict__ X, int64_t ldx, int nr,
                                      const int32_t *__restrict__ sinv0, int64_t n_src,
                                      T *__restrict__ xt, int32_t *__restrict__ counter) {
   __shared__ T tile[64][W + 1];
-  if (blockIdx.x == 0 && threadIdx.x < 2) counter[threadIdx.x] = 0;  // both ticket slots
+  pdl_wait();
+  pdl_trigger();
+  if (blockIdx.x == 0 && threadIdx.x < kTickets) counter[kTicket[threadIdx.x]] = 0;
   for (int64_t j0 = blockIdx.x * 64ll; j0 < n_src; j0 += gridDim.x * 64ll) {
     for (int e = threadIdx.x; e < 64 * W; e += blockDim.x) {
       const int r = e / 64, jj = e % 64;  // consecutive threads: consecutive j
@@ -102,128 +82,285 @@ __device__ __forceinline__ void cp16(void *dst, const void *src, bool valid) {
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void cp_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
 
-// One panel of m <= 128 rows (row-major, stride lda, rows padded with zeros to
-// a multiple of 4 columns) times the W-wide XT rows of its columns. A thread
-// keeps TR rows x TW right-hand sides of accumulators (4 x 8 for W = 8, 2 x 16
-// otherwise, so that fewer threads load the same A entries); the layout is
-// ceil(m / TR) row groups x W / TW right-hand-side groups x S column slices,
-// and a thread steps 4 columns at a time (TR 16-byte loads of A, 4 TW values
-// of XT rows from shared memory, 4 TR TW FMAs). `stage(c0, cn, xs)` issues the asynchronous
-// copies (cp16) of the XT rows of columns [c0, c0 + cn) into xs; the XT rows of
-// the next CC columns are copied into the other half of `buf` while the FMAs
-// of the current ones run. The slices meet in shared memory in slice order.
-template <typename T, int W, typename Stage, typename Emit>
-__device__ __forceinline__ void multi_panel(const T *A, int64_t lda, int m, int ncols_pad, T *buf,
-                                            Stage stage, Emit emit) {
-  constexpr int CC = Cols<T, W>::value;
-  constexpr int TW = W == 8 ? 8 : 16;  // right-hand sides per thread
-  constexpr int TR = 32 / TW;          // rows per thread
-  constexpr int G = W / TW;            // threads sharing a row group (each loads its A)
-  T *red = buf;
-  const int tid = threadIdx.x;
-  const int RQ = (m + TR - 1) / TR, per = RQ * G;
-  int S = kThreads / per;
-  if (S < 1) S = 1;
-  const int ks = tid / per, r = tid - ks * per, rq = r % RQ, rg = r / RQ;
-  const bool active = ks < S;
-  T acc[TR][TW];
-#pragma unroll
-  for (int i = 0; i < TR; i++)
-#pragma unroll
-    for (int j = 0; j < TW; j++) acc[i][j] = T(0);
-  bool ok[TR];
-#pragma unroll
-  for (int i = 0; i < TR; i++) ok[i] = rq * TR + i < m;
-  const int nst = (ncols_pad + CC - 1) / CC;
-  __syncthreads();  // buf free (the previous panel's slice sums are read)
-  if (nst > 0) stage(0, min(CC, ncols_pad), buf);
-  cp_commit();
-  for (int st = 0; st < nst; st++) {
-    const int c0 = st * CC, cn = min(CC, ncols_pad - c0);
-    const T *xs = buf + (st & 1) * CC * W;
-    cp_wait_all();
-    __syncthreads();  // stage st in place everywhere; stage st - 1's half is free
-    if (st + 1 < nst) stage(c0 + CC, min(CC, ncols_pad - c0 - CC), buf + ((st + 1) & 1) * CC * W);
-    cp_commit();
-    if (active) {
-      // the A entries of the next step are loaded before this step's FMAs
-      const int step = 4 * S;
-      auto load = [&](int c, T (&d)[TR][4]) {
-#pragma unroll
-        for (int i = 0; i < TR; i++) {
-          if (ok[i] && c < cn)
-            ld4(A + static_cast<int64_t>(rq * TR + i) * lda + c0 + c, d[i]);
-          else
-            d[i][0] = d[i][1] = d[i][2] = d[i][3] = T(0);
-        }
-      };
-      auto step_fma = [&](int c, const T (&a)[TR][4]) {
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-          T b[TW];
-          ldsn<T, TW>(xs + (c + k) * W + rg * TW, b);
-#pragma unroll
-          for (int i = 0; i < TR; i++)
-#pragma unroll
-            for (int j = 0; j < TW; j++) acc[i][j] = fma(a[i][k], b[j], acc[i][j]);
-        }
-      };
-      T a0[TR][4], a1[TR][4];
-      int c = 4 * ks;
-      load(c, a0);
-      while (c < cn) {
-        load(c + step, a1);
-        step_fma(c, a0);
-        c += step;
-        if (c >= cn) break;
-        load(c + step, a0);
-        step_fma(c, a1);
-        c += step;
-      }
-    }
-  }
-  __syncthreads();  // red aliases xs
-  if (active)
+template <typename T>
+struct Elem {
+  static constexpr int kVec = 16 / sizeof(T);   // elements of a 16-byte copy
+  static constexpr int kStep = 64 / sizeof(T);  // columns per stage: 64 bytes of a panel row
+};
+
+// Lane layout of a panel of MT rows x W right-hand sides: NG lanes along the
+// right-hand sides (TN each) times RG lanes along the rows (rows rg, rg + RG, ...:
+// TR each). 8 right-hand sides a lane where that leaves 48 or 64 accumulators:
+// 16 shared loads of 16 bytes per 256 FMAs; 4 otherwise.
+template <int W, int MT>
+struct LaneTile {
+  static constexpr int TN = W == 32 && MT >= 48 ? 8 : 4;
+  static constexpr int NG = W / TN, RG = 32 / NG, TR = MT / RG;
+  static_assert(TR * RG == MT, "whole rows");
+};
+
+// Stages of one warp: per stage 64 rows x 64 bytes of the panel, the 16-byte
+// pieces of row r swapped by (r / 2) mod 4 (eight consecutive rows then touch all
+// banks once), then kStep rows of XT.
+template <typename T, int W>
+constexpr int stage_bytes() {
+  return kPanelRows * 64 + Elem<T>::kStep * W * static_cast<int>(sizeof(T));
+}
+template <typename T, int W, int NW>
+constexpr size_t multi_smem() {
+  return static_cast<size_t>(NW) * 2 * stage_bytes<T, W>();
+}
+
+__device__ __forceinline__ void lds16(const unsigned char *p, float (&v)[4]) {
+  const float4 a = *reinterpret_cast<const float4 *>(p);
+  v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+}
+__device__ __forceinline__ void lds16(const unsigned char *p, double (&v)[2]) {
+  const double2 a = *reinterpret_cast<const double2 *>(p);
+  v[0] = a.x; v[1] = a.y;
+}
+
+// A lane's TR x TN sums. In FP32 two neighbouring right-hand sides share a register pair and
+// an fma.rn.f32x2, each half rounded as a single FMA is: the FMA rate is the same, but it takes
+// half the issue slots (8 x 8 tiles from shared memory: 28 -> 31 TFMA/s), which the copies need.
+template <typename T, int TR, int TN>
+struct Sums {
+  T v[TR][TN];
+  __device__ __forceinline__ void zero() {
 #pragma unroll
     for (int i = 0; i < TR; i++)
 #pragma unroll
-      for (int j = 0; j < TW; j++) red[((ks * RQ + rq) * TR + i) * W + rg * TW + j] = acc[i][j];
-  __syncthreads();
-  for (int o = tid; o < m * W; o += kThreads) {
-    const int row = o / W, q = o % W;
-    T s = T(0);
-    for (int sl = 0; sl < S; sl++) s += red[(sl * RQ * TR + row) * W + q];
-    emit(row, q, s);
+      for (int j = 0; j < TN; j++) v[i][j] = T(0);
+  }
+  struct B {
+    T v[TN];
+    __device__ __forceinline__ void load(const unsigned char *p) {
+      constexpr int VEC = 16 / sizeof(T);
+#pragma unroll
+      for (int j = 0; j < TN / VEC; j++) {
+        T q[VEC];
+        lds16(p + j * 16, q);
+#pragma unroll
+        for (int e = 0; e < VEC; e++) v[j * VEC + e] = q[e];
+      }
+    }
+  };
+  __device__ __forceinline__ void add(int i, T a, const B &b) {
+#pragma unroll
+    for (int j = 0; j < TN; j++) v[i][j] = fma(a, b.v[j], v[i][j]);
+  }
+  __device__ __forceinline__ T get(int i, int j) const { return v[i][j]; }
+};
+template <int TR, int TN>
+struct Sums<float, TR, TN> {
+  unsigned long long v[TR][TN / 2];
+  __device__ __forceinline__ void zero() {
+#pragma unroll
+    for (int i = 0; i < TR; i++)
+#pragma unroll
+      for (int j = 0; j < TN / 2; j++) v[i][j] = 0ull;
+  }
+  struct B {
+    unsigned long long v[TN / 2];
+    __device__ __forceinline__ void load(const unsigned char *p) {
+#pragma unroll
+      for (int j = 0; j < TN / 4; j++) {
+        const ulonglong2 q = *reinterpret_cast<const ulonglong2 *>(p + j * 16);
+        v[2 * j] = q.x;
+        v[2 * j + 1] = q.y;
+      }
+    }
+  };
+  __device__ __forceinline__ void add(int i, float a, const B &b) {
+    unsigned long long aa;
+    asm("mov.b64 %0, {%1, %1};" : "=l"(aa) : "f"(a));
+#pragma unroll
+    for (int j = 0; j < TN / 2; j++) asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(v[i][j]) : "l"(aa), "l"(b.v[j]));
+  }
+  __device__ __forceinline__ float get(int i, int j) const {
+    return __uint_as_float(static_cast<unsigned>(j & 1 ? v[i][j / 2] >> 32 : v[i][j / 2]));
+  }
+};
+
+// acc += panel x XT over the column stages first, first + step, ... of a panel of m <=
+// MT rows (row-major, stride lda, ncols a multiple of 4), by one warp. row_of(c)
+// is the XT row of column c, -1 for a zero row; lane l asks for column l of a
+// stage, one stage ahead. `buf`: the warp's two stages.
+template <typename T, int W, int MT, typename RowOf>
+__device__ __forceinline__ void slice_product(const T *A, int64_t lda, int m, int ncols, int first, int step,
+                                              const T *__restrict__ xt, unsigned char *buf, RowOf row_of,
+                                              Sums<T, LaneTile<W, MT>::TR, LaneTile<W, MT>::TN> &acc) {
+  using L = LaneTile<W, MT>;
+  constexpr int VEC = Elem<T>::kVec, KS = Elem<T>::kStep;
+  constexpr int PB = W / VEC;  // 16-byte pieces of an XT row
+  constexpr int SB = stage_bytes<T, W>();
+  const int lane = threadIdx.x & 31, rg = lane / L::NG, ng = lane - rg * L::NG;
+  const int nst = (ncols + KS - 1) / KS;
+  const T *arow = A + (lane >> 2) * lda + (lane & 3) * VEC;  // the lane's first row and piece
+  int idx = -1;
+  auto look_up = [&](int st) {
+    const int c = st * KS + lane;
+    idx = lane < KS && st < nst ? row_of(c) : -1;
+  };
+  auto issue = [&](int st, unsigned char *b) {
+    const int c0 = st * KS, piece = lane & 3;
+    const bool in = c0 + piece * VEC < ncols;
+    const T *src = arow + (in ? c0 : 0);
+#pragma unroll
+    for (int j = 0; j < MT / 8; j++) {
+      const int r = (lane >> 2) + 8 * j;
+      if (r < m) cp16(b + r * 64 + ((piece ^ ((r >> 1) & 3)) << 4), src, in);
+      src += 8 * lda;
+    }
+    unsigned char *xb = b + kPanelRows * 64;
+#pragma unroll
+    for (int j = 0; j < (KS * PB + 31) / 32; j++) {
+      const int e = lane + 32 * j, k = e / PB, p = e - k * PB;
+      const int r = __shfl_sync(0xffffffffu, idx, k & 31);
+      if (KS * PB % 32 == 0 || e < KS * PB)
+        cp16(xb + e * 16, xt + static_cast<int64_t>(r < 0 ? 0 : r) * W + p * VEC, r >= 0);
+    }
+  };
+  if (first < nst) {
+    look_up(first);
+    issue(first, buf);
+    look_up(first + step);
+  }
+  cp_commit();
+  int h = 0;
+  for (int st = first; st < nst; st += step, h ^= 1) {
+    if (st + step < nst) {
+      issue(st + step, buf + (h ^ 1) * SB);
+      look_up(st + 2 * step);
+    }
+    cp_commit();
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    __syncwarp();  // every lane's copies of stage st are in place
+    const unsigned char *pa = buf + h * SB + rg * 64, *pb = buf + h * SB + kPanelRows * 64 + ng * L::TN * sizeof(T);
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      T a[L::TR][VEC];
+#pragma unroll
+      for (int i = 0; i < L::TR; i++) lds16(pa + i * L::RG * 64 + ((q ^ (((rg + i * L::RG) >> 1) & 3)) << 4), a[i]);
+#pragma unroll
+      for (int k = 0; k < VEC; k++) {
+        typename Sums<T, L::TR, L::TN>::B b;
+        b.load(pb + (q * VEC + k) * W * sizeof(T));
+#pragma unroll
+        for (int i = 0; i < L::TR; i++) acc.add(i, a[i][k], b);
+      }
+    }
+    __syncwarp();  // the stage may be filled again
+  }
+  cp_wait_all();
+}
+
+// The warps' sums of a panel of m <= MT rows, added in warp order: emit(row, q, sum) for
+// every row < m and q < W; consecutive threads get consecutive rows (ROWS) or
+// right-hand sides. By the whole CTA, after every warp's product.
+template <typename T, int W, int NW, int MT, bool ROWS, typename S, typename Emit>
+__device__ __forceinline__ void sum_warps(const S &acc, int m, unsigned char *smem, Emit emit) {
+  using L = LaneTile<W, MT>;
+  constexpr int LD = W + 1;  // row stride of the sums: no bank conflicts either way
+  // the sums of all rows at once where they fit the stages, else of half of them
+  constexpr int PARTS = static_cast<size_t>(NW) * MT * LD * sizeof(T) <= multi_smem<T, W, NW>() ? 1 : 2;
+  constexpr int TRP = L::TR / PARTS, MP = MT / PARTS;
+  static_assert(L::TR % PARTS == 0 && static_cast<size_t>(NW) * MP * LD * sizeof(T) <= multi_smem<T, W, NW>(), "sums");
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int rg = lane / L::NG, ng = lane - rg * L::NG;
+  T *red = reinterpret_cast<T *>(smem);
+#pragma unroll
+  for (int part = 0; part < PARTS; part++) {
+    __syncthreads();  // the stages (or the sums of the part before) are no longer read
+#pragma unroll
+    for (int i = 0; i < TRP; i++)
+#pragma unroll
+      for (int j = 0; j < L::TN; j++)
+        red[(warp * MP + rg + i * L::RG) * LD + ng * L::TN + j] = acc.get(part * TRP + i, j);
+    __syncthreads();
+    for (int o = tid; o < MP * W; o += NW * 32) {
+      const int row = ROWS ? o % MP : o / W, q = ROWS ? o / MP : o % W;
+      if (part * MP + row >= m) continue;
+      T s = red[row * LD + q];
+#pragma unroll
+      for (int w = 1; w < NW; w++) s += red[(w * MP + row) * LD + q];
+      emit(part * MP + row, q, s);
+    }
   }
 }
 
-// V pass: for every multi-RHS V item (ticket order)
+// Row count of the micro-kernel for a panel of m rows.
+template <typename F>
+__device__ __forceinline__ void with_rows(int m, F f) {
+  if (m > 48)
+    f(std::integral_constant<int, 64>());
+  else if (m > 32)
+    f(std::integral_constant<int, 48>());
+  else if (m > 16)
+    f(std::integral_constant<int, 32>());
+  else
+    f(std::integral_constant<int, 16>());
+}
+
+// V pass: for every multi-RHS V item
 //   out[(I.out + k) * W + r] = sum_j V[k, j] XT[(I.x_off + j) * W + r],
-// out = XT (t rows) or the partial rows P of a cut group.
+// out = XT (t rows) or the partial rows P of a cut group. Items [0, nbig) by
+// CTAs, the others, of few columns, by single warps; first items by number, the
+// next from ticket counters.
 template <typename T, int W>
-__global__ void __launch_bounds__(kThreads) v_multi_kernel(const T *__restrict__ V,
-                                                           const MVItem *__restrict__ items,
-                                                           int32_t nitems, T *__restrict__ xt,
-                                                           T *__restrict__ P, int32_t *counter) {
+__global__ void __launch_bounds__(kVWarps * 32, multi_ctas<T, kVWarps>()) v_multi_kernel(const T *__restrict__ V,
+                                                                            const MVItem *__restrict__ items,
+                                                                            int32_t nbig, int32_t nitems,
+                                                                            T *__restrict__ xt, T *__restrict__ P,
+                                                                            int32_t *counter) {
   extern __shared__ __align__(16) unsigned char dyn_smem[];
-  T *buf = reinterpret_cast<T *>(dyn_smem);  // XT rows while streaming, slice sums after
-  __shared__ int32_t s_ticket[2];
-  for (int it = 0;; it++) {
-    if (threadIdx.x == 0) s_ticket[it & 1] = atomicAdd(counter, 1);
-    __syncthreads();
-    const int32_t u = s_ticket[it & 1];
-    if (u >= nitems) break;
+  __shared__ int32_t s_ticket;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int32_t ctas = static_cast<int32_t>(gridDim.x);
+  unsigned char *buf = dyn_smem + warp * 2 * stage_bytes<T, W>();
+  pdl_wait();
+  pdl_trigger();
+  int32_t u = static_cast<int32_t>(blockIdx.x);
+  bool big = u < nbig;
+  if (!big) u = nbig + u * kVWarps + warp;
+  while (u < nitems) {  // one loop for both kinds, so that the micro-kernels' code is there once
+    int32_t next = 0;
+    if (big ? tid == 0 : lane == 0)
+      next = (big ? ctas : nbig + ctas * kVWarps) + atomicAdd(counter + kTicket[big ? 1 : 2], 1);
     const MVItem I = items[u];
-    const T *src = xt + static_cast<int64_t>(I.x_off) * W;
-    T *out = I.kind == 0 ? xt : P;
-    multi_panel<T, W>(
-        V + I.v_off, I.stride, I.nrows, I.ncols, buf,
-        [&](int c0, int cn, T *xs) {  // contiguous XT rows
-          constexpr int kV = 16 / sizeof(T);  // values per 16-byte copy
-          for (int e = threadIdx.x; e < cn * W / kV; e += kThreads)
-            cp16(xs + e * kV, src + static_cast<int64_t>(c0) * W + e * kV, true);
-        },
-        [&](int row, int q, T s) { out[static_cast<int64_t>(I.out + row) * W + q] = s; });
+    T *out = (I.kind == 0 ? xt : P) + static_cast<int64_t>(I.out) * W;
+    with_rows(I.nrows, [&](auto mt) {
+      using L = LaneTile<W, mt.value>;
+      Sums<T, L::TR, L::TN> acc;
+      acc.zero();
+      slice_product<T, W, mt.value>(V + I.v_off, I.stride, I.nrows, I.ncols, big ? warp : 0, big ? kVWarps : 1, xt, buf,
+                                    [&](int c) { return c < I.ncols ? I.x_off + c : -1; }, acc);
+      if (big) {
+        sum_warps<T, W, kVWarps, mt.value, false>(acc, I.nrows, dyn_smem,
+                                         [&](int row, int q, T s) { out[static_cast<int64_t>(row) * W + q] = s; });
+      } else {
+        const int rg = lane / L::NG, ng = lane - rg * L::NG;
+#pragma unroll
+        for (int i = 0; i < L::TR; i++) {
+          const int row = rg + i * L::RG;
+          T *o = out + static_cast<int64_t>(row) * W + ng * L::TN;
+          if (row < I.nrows)
+#pragma unroll
+            for (int j = 0; j < L::TN; j++) o[j] = acc.get(i, j);
+        }
+      }
+    });
+    if (big) {
+      if (tid == 0) s_ticket = next;
+      __syncthreads();  // the sums are read, the stages may be filled again
+      u = s_ticket;
+      if (u >= nbig) {
+        big = false;
+        u = nbig + static_cast<int32_t>(blockIdx.x) * kVWarps + warp;
+      }
+    } else {
+      u = __shfl_sync(0xffffffffu, next, 0);
+    }
   }
 }
 
@@ -232,6 +369,8 @@ template <typename T, int W>
 __global__ void reduce_multi_kernel(const MVReduce *__restrict__ red, int32_t nred, const T *__restrict__ P,
                                     T *__restrict__ xt) {
   const int lane = threadIdx.x & 31;
+  pdl_wait();
+  pdl_trigger();
   if (lane >= W) return;
   for (int32_t e = static_cast<int32_t>(blockIdx.x); e < nred; e += gridDim.x) {
     const MVReduce R = red[e];
@@ -244,14 +383,14 @@ __global__ void reduce_multi_kernel(const MVReduce *__restrict__ red, int32_t nr
   }
 }
 
-// Near/U pass: one whole row tile per CTA (tiles from a ticket counter).
+// Near/U pass: a run of at most 64 rows of one tile per CTA (first by number, then from a
+// ticket counter, tiles with the most columns first).
 template <typename T>
 struct DuMultiArgs {
   const T *panels;
-  const TileDesc *tiles;
-  const int32_t *order;  // tiles by decreasing work
-  int32_t ntiles;
-  const Seg *segs;
+  const MUnit *units;
+  int32_t nunits;
+  const int32_t *colmap;  // XT row of every tile column, tile after tile
   const T *xt;
   const int32_t *tmap0;
   T *y;
@@ -260,53 +399,69 @@ struct DuMultiArgs {
   int32_t *counter;
 };
 
-template <typename T, int W>
-__global__ void __launch_bounds__(kThreads) du_multi_kernel(DuMultiArgs<T> a) {
-  extern __shared__ __align__(16) unsigned char dyn_smem[];
-  T *buf = reinterpret_cast<T *>(dyn_smem);  // two halves of staged XT rows, slice sums after
-  __shared__ int32_t s_ticket[2];
-  const int tid = threadIdx.x;
-  for (int it = 0;; it++) {
-    if (tid == 0) s_ticket[it & 1] = atomicAdd(a.counter, 1);
-    __syncthreads();
-    const int32_t u = s_ticket[it & 1];
-    if (u >= a.ntiles) break;
-    const TileDesc d = a.tiles[a.order[u]];
-    const Seg *S = a.segs + d.seg0;
-    multi_panel<T, W>(
-        a.panels + d.data_off, d.ld, d.m, d.ld, buf,
-        [&](int c0, int cn, T *xs) {  // one thread per column: its XT row, then its copies
-          constexpr int kP = W * static_cast<int>(sizeof(T)) / 16;  // 16-byte pieces per XT row
-          for (int j = threadIdx.x; j < cn; j += kThreads) {
-            const int c = c0 + j;
-            int v = -1;
-            if (c < d.ncols) {
-              int lo = 0, hi = d.nseg - 1;
-              while (lo < hi) {
-                const int mid = (lo + hi + 1) >> 1;
-                if (S[mid].col0 <= c)
-                  lo = mid;
-                else
-                  hi = mid - 1;
-              }
-              v = S[lo].vec_off + (c - S[lo].col0);
-            }
-            const T *src = a.xt + static_cast<int64_t>(v >= 0 ? v : 0) * W;
-#pragma unroll
-            for (int q = 0; q < kP; q++) cp16(xs + j * W + q * (16 / sizeof(T)), src + q * (16 / sizeof(T)), v >= 0);
-          }
-        },
-        [&](int row, int q, T s) {
-          if (q < a.nr) a.y[a.tmap0[d.row0 + row] + q * a.ldy] = s;
-        });
+// The column map of every tile from its segments: a warp per segment would leave most lanes idle
+// on rank columns, so a warp takes a tile and each lane its columns, by binary search.
+__global__ void __launch_bounds__(kThreads) colmap_kernel(const TileDesc *__restrict__ tiles, int32_t ntiles,
+                                                          const Seg *__restrict__ segs,
+                                                          const int64_t *__restrict__ col0,
+                                                          int32_t *__restrict__ colmap) {
+  const int lane = threadIdx.x & 31;
+  for (int64_t t = blockIdx.x * static_cast<int64_t>((kThreads / 32)) + (threadIdx.x >> 5); t < ntiles;
+       t += static_cast<int64_t>(gridDim.x) * (kThreads / 32)) {
+    const TileDesc d = tiles[t];
+    const Seg *S = segs + d.seg0;
+    int lo0 = 0;
+    for (int c = lane; c < d.ncols; c += 32) {
+      int lo = lo0, hi = d.nseg - 1;  // last segment with col0 <= c
+      while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (S[mid].col0 <= c)
+          lo = mid;
+        else
+          hi = mid - 1;
+      }
+      lo0 = lo;
+      colmap[col0[t] + c] = S[lo].vec_off + (c - S[lo].col0);
+    }
   }
 }
 
-// Dynamic shared memory of the multi-RHS kernels: 32 accumulators per thread
-// for the slice reduction (also holds the staged XT rows).
-template <typename T>
-constexpr size_t multi_smem() {
-  return static_cast<size_t>(kThreads) * 32 * sizeof(T);
+cudaError_t launch_colmap(const TileDesc *tiles, int32_t ntiles, const Seg *segs, const int64_t *col0, int32_t *colmap,
+                          cudaStream_t s) {
+  colmap_kernel<<<ntiles < 8192 ? (ntiles + (kThreads / 32) - 1) / (kThreads / 32) : 1024, kThreads, 0, s>>>(tiles, ntiles, segs, col0,
+                                                                                          colmap);
+  return cudaGetLastError();
+}
+
+template <typename T, int W>
+__global__ void __launch_bounds__(kDuWarps * 32, multi_ctas<T, kDuWarps>()) du_multi_kernel(DuMultiArgs<T> a) {
+  extern __shared__ __align__(16) unsigned char dyn_smem[];
+  __shared__ int32_t s_ticket;
+  const int tid = threadIdx.x, warp = tid >> 5;
+  pdl_wait();
+  pdl_trigger();
+  for (int32_t u = static_cast<int32_t>(blockIdx.x); u < a.nunits;) {
+    const MUnit U = a.units[u];
+    int32_t next = 0;
+    if (tid == 0) next = static_cast<int32_t>(gridDim.x) + atomicAdd(a.counter + kTicket[0], 1);
+    const int32_t *map = a.colmap + U.map;
+    with_rows(U.m, [&](auto mt) {
+      using L = LaneTile<W, mt.value>;
+      Sums<T, L::TR, L::TN> acc;
+      acc.zero();
+      slice_product<T, W, mt.value>(a.panels + U.data_off, U.ld, U.m, U.ld, warp, kDuWarps, a.xt,
+                                    dyn_smem + warp * 2 * stage_bytes<T, W>(),
+                                    [&](int c) { return c < U.ncols ? __ldg(map + c) : -1; }, acc);
+      if (tid == 0) s_ticket = next;
+      sum_warps<T, W, kDuWarps, mt.value, true>(
+          acc, U.m, dyn_smem,
+          [&](int row, int q, T s) {
+            if (q < a.nr) a.y[a.tmap0[U.row0 + row] + q * a.ldy] = s;
+          });
+    });
+    __syncthreads();  // the sums are read, the stages may be filled again
+    u = s_ticket;
+  }
 }
 
 template <typename T, int W>
@@ -314,80 +469,73 @@ static void multi_attrs() {
   static bool done = false;  // once per process (the attribute is per function)
   if (done) return;
   cudaFuncSetAttribute(v_multi_kernel<T, W>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       static_cast<int>(multi_smem<T>()));
+                       static_cast<int>(multi_smem<T, W, kVWarps>()));
   cudaFuncSetAttribute(du_multi_kernel<T, W>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       static_cast<int>(multi_smem<T>()));
+                       static_cast<int>(multi_smem<T, W, kDuWarps>()));
   done = true;
 }
 
 template <typename T, int W>
 static cudaError_t run_multi(const DevPlan &p, const T *panels, const T *vdata, T *xt, T *P, const T *X,
-                             int64_t ldx, int nr, T *Y, int64_t ldy, int grid_du,
+                             int64_t ldx, int nr, T *Y, int64_t ldy, int num_sms,
                              cudaStream_t s, cudaEvent_t *ev, int *launches) {
   multi_attrs<T, W>();
   int gp = static_cast<int>((p.n_src + 63) / 64);
   if (gp > 2048) gp = 2048;
   int nl = 0;
   if (ev) cudaEventRecord(ev[0], s);
-  permute_multi_kernel<T, W><<<gp, kThreads, 0, s>>>(X, ldx, nr, p.sinv0, p.n_src, xt, p.counter);
+  cudaError_t e = launch_pdl(permute_multi_kernel<T, W>, gp, kThreads, 0, s, X, ldx, nr, p.sinv0, p.n_src, xt, p.counter);
   nl++;
   if (ev) cudaEventRecord(ev[1], s);
-  if (p.nmv > 0) {
-    v_multi_kernel<T, W><<<grid_du, kThreads, multi_smem<T>(), s>>>(vdata, p.mv_items, p.nmv, xt, P, p.counter);
+  if (e == cudaSuccess && p.nmv > 0) {
+    const int32_t nbig = sizeof(T) == 4 ? p.nmv_big : p.nmv;
+    e = launch_pdl(v_multi_kernel<T, W>, num_sms * multi_ctas<T, kVWarps>(), kVWarps * 32,
+                   multi_smem<T, W, kVWarps>(), s, vdata, p.mv_items, nbig, p.nmv, xt, P, p.counter);
     nl++;
-    if (p.nmvr > 0) {
-      reduce_multi_kernel<T, W><<<p.nmvr < 4096 ? p.nmvr : 4096, kThreads, 0, s>>>(p.mv_reduce, p.nmvr, P, xt);
+    if (e == cudaSuccess && p.nmvr > 0) {
+      e = launch_pdl(reduce_multi_kernel<T, W>, p.nmvr < 4096 ? p.nmvr : 4096, kThreads, 0, s, p.mv_reduce, p.nmvr, P,
+                     xt);
       nl++;
     }
   }
   if (ev) cudaEventRecord(ev[2], s);
-  DuMultiArgs<T> a{panels, p.tiles, p.tile_order, p.ntiles, p.segs, xt, p.tmap0, Y, ldy, nr, p.counter + 1};
-  du_multi_kernel<T, W><<<grid_du, kThreads, multi_smem<T>(), s>>>(a);
+  DuMultiArgs<T> a{panels, p.munits, p.nmunits, p.mcolmap, xt, p.tmap0, Y, ldy, nr, p.counter};
+  if (e == cudaSuccess)
+    e = launch_pdl(du_multi_kernel<T, W>, num_sms * multi_ctas<T, kDuWarps>(), kDuWarps * 32,
+                   multi_smem<T, W, kDuWarps>(), s, a);
   nl++;
   if (ev) cudaEventRecord(ev[3], s);
   if (launches) *launches = nl;
-  return cudaGetLastError();
+  return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 int rhs_per_pass() { return kRhs; }
 
 int multi_width(int nr) { return nr <= 8 ? 8 : nr <= 16 ? 16 : kRhs; }
 
-int occupancy_du_multi(bool f64) {
-  int n = 0;
-  if (f64) {
-    multi_attrs<double, kRhs>();
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, du_multi_kernel<double, kRhs>, kThreads, multi_smem<double>());
-  } else {
-    multi_attrs<float, kRhs>();
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, du_multi_kernel<float, kRhs>, kThreads, multi_smem<float>());
-  }
-  return n > 0 ? n : 1;
-}
-
 template <typename T>
 static cudaError_t run_multi_w(const DevPlan &p, const T *panels, const T *vdata, T *xt, T *P, const T *X,
-                               int64_t ldx, int nr, T *Y, int64_t ldy, int grid_du, cudaStream_t s,
+                               int64_t ldx, int nr, T *Y, int64_t ldy, int num_sms, cudaStream_t s,
                                cudaEvent_t *ev, int *launches) {
   switch (multi_width(nr)) {
-    case 8: return run_multi<T, 8>(p, panels, vdata, xt, P, X, ldx, nr, Y, ldy, grid_du, s, ev, launches);
-    case 16: return run_multi<T, 16>(p, panels, vdata, xt, P, X, ldx, nr, Y, ldy, grid_du, s, ev, launches);
-    default: return run_multi<T, kRhs>(p, panels, vdata, xt, P, X, ldx, nr, Y, ldy, grid_du, s, ev, launches);
+    case 8: return run_multi<T, 8>(p, panels, vdata, xt, P, X, ldx, nr, Y, ldy, num_sms, s, ev, launches);
+    case 16: return run_multi<T, 16>(p, panels, vdata, xt, P, X, ldx, nr, Y, ldy, num_sms, s, ev, launches);
+    default: return run_multi<T, kRhs>(p, panels, vdata, xt, P, X, ldx, nr, Y, ldy, num_sms, s, ev, launches);
   }
 }
 
 cudaError_t launch_matvec_multi(bool f64, const DevPlan &p, const void *panels, const void *vdata,
                                 void *xt, void *P, const void *X, int64_t ldx, int nr, void *Y,
-                                int64_t ldy, int grid_du, cudaStream_t s, cudaEvent_t *ev,
+                                int64_t ldy, int num_sms, cudaStream_t s, cudaEvent_t *ev,
                                 int *launches) {
   if (f64)
     return run_multi_w<double>(p, static_cast<const double *>(panels), static_cast<const double *>(vdata),
                              static_cast<double *>(xt), static_cast<double *>(P),
                              static_cast<const double *>(X), ldx, nr, static_cast<double *>(Y), ldy,
-                             grid_du, s, ev, launches);
+                             num_sms, s, ev, launches);
   return run_multi_w<float>(p, static_cast<const float *>(panels), static_cast<const float *>(vdata),
                           static_cast<float *>(xt), static_cast<float *>(P), static_cast<const float *>(X),
-                          ldx, nr, static_cast<float *>(Y), ldy, grid_du, s, ev, launches);
+                          ldx, nr, static_cast<float *>(Y), ldy, num_sms, s, ev, launches);
 }
 
 }  // namespace hm
