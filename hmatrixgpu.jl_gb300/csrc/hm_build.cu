@@ -39,27 +39,29 @@ __device__ __forceinline__ void reflect_cols(const double *x, int len, double ta
   for (int i = 1 + t; i < len; i += NT) {
     const double xi = x[i];
 #pragma unroll
-    for (int q = 0; q < NC; q++) d[q] += xi * y0[i * si + q * scs];
+    for (int q = 0; q < NC; q++) d[q] = dadd(d[q], dmul(xi, y0[i * si + q * scs]));
   }
-  tsum<NT, NC>(d, sc);
+  constexpr int G = sum_lanes<NC>();  // lanes that hold one column's sum
+  const int lane = threadIdx.x & 31, own = min(lane / G, NC - 1);
+  const double sum = tsum_spread<NT, NC>(d, sc), y00 = y0[own * scs];
+  const double wown = dmul(dadd(sum, y00), tau);
   double wv[NC];
 #pragma unroll
-  for (int q = 0; q < NC; q++) wv[q] = (d[q] + y0[q * scs]) * tau;
+  for (int q = 0; q < NC; q++) wv[q] = __shfl_sync(0xffffffffu, wown, q * G);
   for (int i = 1 + t; i < len; i += NT) {
     const double xi = x[i];
 #pragma unroll
-    for (int q = 0; q < NC; q++) y0[i * si + q * scs] -= wv[q] * xi;
+    for (int q = 0; q < NC; q++) y0[i * si + q * scs] = dsub(y0[i * si + q * scs], dmul(wv[q], xi));
   }
   tsync<NT>();
-  if (t == 0)
-#pragma unroll
-    for (int q = 0; q < NC; q++) y0[q * scs] -= wv[q];
+  if (t < 32 && lane == own * G) y0[own * scs] = dsub(y00, wown);
   tsync<NT>();
 }
 
+// (not inlined: the QR kernel missed the instruction cache with a copy per call)
 template <int NT>
-__device__ void reflect_any(int nc, const double *x, int len, double tau, double *y0, int64_t si, int64_t scs,
-                            TeamScratch *sc) {
+__device__ __noinline__ void reflect_any(int nc, const double *x, int len, double tau, double *y0, int64_t si,
+                                         int64_t scs, TeamScratch *sc) {
   switch (nc) {
     case 1: reflect_cols<NT, 1>(x, len, tau, y0, si, scs, sc); break;
     case 2: reflect_cols<NT, 2>(x, len, tau, y0, si, scs, sc); break;
@@ -82,15 +84,15 @@ __device__ void team_qr(double *A, int64_t ld, int rows, int cols, double *tau, 
     double *x = A + j + j * ld;
     const int len = rows - j;
     double s = 0.0;
-    for (int i = 1 + t; i < len; i += NT) s += x[i] * x[i];
-    const double xn = sqrt(tsum1<NT>(s, sc));
+    for (int i = 1 + t; i < len; i += NT) s = dadd(s, dmul(x[i], x[i]));
+    const double xn = dsqrt(tsum1<NT>(s, sc));
     const double alpha = x[0];
     double tj = 0.0;
     if (xn != 0.0) {
-      const double beta = -copysign(sqrt(alpha * alpha + xn * xn), alpha);
-      tj = (beta - alpha) / beta;
-      const double scl = 1.0 / (alpha - beta);
-      for (int i = 1 + t; i < len; i += NT) x[i] *= scl;
+      const double beta = -copysign(dsqrt(dadd(dmul(alpha, alpha), dmul(xn, xn))), alpha);
+      tj = ddiv(dsub(beta, alpha), beta);
+      const double scl = ddiv(1.0, dsub(alpha, beta));
+      for (int i = 1 + t; i < len; i += NT) x[i] = dmul(x[i], scl);
       tsync<NT>();
       if (t == 0) x[0] = beta;
     }
@@ -114,7 +116,7 @@ __device__ void qr_team(const AcaJob &jb, const AcaRes &rs, int svd, double *ws,
   for (int e = t; e < k * k; e += NT) {   // M = RU * RV' (:129)
     const int r = e % k, c = e / k;
     double s = 0.0;
-    for (int q = max(r, c); q < k; q++) s += w.U[r + static_cast<int64_t>(q) * m] * w.V[c + static_cast<int64_t>(q) * n];
+    for (int q = max(r, c); q < k; q++) s = dadd(s, dmul(w.U[r + static_cast<int64_t>(q) * m], w.V[c + static_cast<int64_t>(q) * n]));
     w.M[r + c * k] = s;
     w.Z[r + c * k] = r == c ? 1.0 : 0.0;
   }
@@ -173,11 +175,11 @@ __device__ __forceinline__ bool jac_pair(int c, int k, int l, int &p, int &q, bo
 // Cosine and sine of the rotation that makes two columns orthogonal (squared
 // norms a and b, product g); false where they are already.
 __device__ __forceinline__ bool jac_rotation(double a, double b, double g, double &c, double &s) {
-  if (g == 0.0 || fabs(g) <= 1e-15 * sqrt(a * b)) return false;
-  const double zeta = (b - a) / (2.0 * g);
-  const double tt = copysign(1.0, zeta) / (fabs(zeta) + sqrt(1.0 + zeta * zeta));
-  c = 1.0 / sqrt(1.0 + tt * tt);
-  s = c * tt;
+  if (g == 0.0 || fabs(g) <= dmul(1e-15, dsqrt(dmul(a, b)))) return false;
+  const double zeta = ddiv(dsub(b, a), dadd(g, g));
+  const double tt = ddiv(copysign(1.0, zeta), dadd(fabs(zeta), dsqrt(dadd(1.0, dmul(zeta, zeta)))));
+  c = ddiv(1.0, dsqrt(dadd(1.0, dmul(tt, tt))));
+  s = dmul(c, tt);
   return true;
 }
 
@@ -185,7 +187,7 @@ __device__ __forceinline__ bool jac_rotation(double a, double b, double g, doubl
 // rank, by one thread.
 __device__ void jac_finish(const WS &w, int k, double eps, bool converged, AcaRes *res) {
   for (int j = 0; j < k; j++) {
-    w.sig[j] = sqrt(w.sig[j]);
+    w.sig[j] = dsqrt(w.sig[j]);
     w.ord[j] = j;
   }
   for (int i = 1; i < k; i++) {  // stable, decreasing sigma
@@ -203,8 +205,8 @@ __device__ void jac_finish(const WS &w, int k, double eps, bool converged, AcaRe
   int r = k;
   double acc = 0.0;
   for (int i = k - 1; i >= 0; i--) {
-    acc += w.sig[w.ord[i]] * w.sig[w.ord[i]];
-    if (sqrt(acc) < eps)
+    acc = dadd(acc, dmul(w.sig[w.ord[i]], w.sig[w.ord[i]]));
+    if (dsqrt(acc) < eps)
       r = i;
     else
       break;
@@ -294,7 +296,7 @@ __global__ void __launch_bounds__(32) jacobi_group_kernel(const AcaJob *__restri
     if (mine)
       for (int j = l; j < k; j += gw) {
         double s = 0.0;
-        for (int i = 0; i < k; i++) s += M[i + j * ld] * M[i + j * ld];
+        for (int i = 0; i < k; i++) s = dadd(s, dmul(M[i + j * ld], M[i + j * ld]));
         norm[j] = s;
       }
     __syncwarp();
@@ -310,7 +312,7 @@ __global__ void __launch_bounds__(32) jacobi_group_kernel(const AcaJob *__restri
           if (t >= 0 && t < kJacSweeps) {
             double *mp = M + p * ld, *mq = M + q * ld;
             double g = 0.0;
-            for (int i = 0; i < k; i++) g += mp[i] * mq[i];
+            for (int i = 0; i < k; i++) g = dadd(g, dmul(mp[i], mq[i]));
             double cs, sn;
             if (jac_rotation(norm[p], norm[q], g, cs, sn)) {
               rot = true;
@@ -319,13 +321,13 @@ __global__ void __launch_bounds__(32) jacobi_group_kernel(const AcaJob *__restri
               double a = 0.0, b = 0.0;
               for (int i = 0; i < k; i++) {
                 const double u = mp[i], v = mq[i], zu = zp[i], zv = zq[i];
-                const double u2 = cs * u - sn * v, v2 = sn * u + cs * v;
-                a += u2 * u2;
-                b += v2 * v2;
+                const double u2 = dsub(dmul(cs, u), dmul(sn, v)), v2 = dadd(dmul(sn, u), dmul(cs, v));
+                a = dadd(a, dmul(u2, u2));
+                b = dadd(b, dmul(v2, v2));
                 mp[i] = u2;
                 mq[i] = v2;
-                zp[i] = cs * zu - sn * zv;
-                zq[i] = sn * zu + cs * zv;
+                zp[i] = dsub(dmul(cs, zu), dmul(sn, zv));
+                zq[i] = dadd(dmul(sn, zu), dmul(cs, zv));
               }
               norm[p] = a;
               norm[q] = b;
@@ -391,7 +393,7 @@ __global__ void __launch_bounds__(kBuildThreads) jacobi_cta_kernel(const AcaJob 
     __syncthreads();
     auto dot = [&](const double *x, const double *y) {
       double s = 0.0;
-      for (int i = 0; i < k; i++) s += x[i] * y[i];
+      for (int i = 0; i < k; i++) s = dadd(s, dmul(x[i], y[i]));
       return s;
     };
     int quiet = 0, last_rot = 0;
@@ -440,8 +442,8 @@ __global__ void __launch_bounds__(kBuildThreads) jacobi_cta_kernel(const AcaJob 
             double *xp = i < k ? M + p * ldm + i : Z + p * ldz + (i - k);
             double *xq = i < k ? M + q * ldm + i : Z + q * ldz + (i - k);
             const double u = *xp, v = *xq;
-            *xp = cs * u - sn * v;
-            *xq = sn * u + cs * v;
+            *xp = dsub(dmul(cs, u), dmul(sn, v));
+            *xq = dadd(dmul(sn, u), dmul(cs, v));
           }
         }
         __syncthreads();

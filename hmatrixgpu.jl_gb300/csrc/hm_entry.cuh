@@ -19,6 +19,7 @@
 #include "../../include/hmgpu.h"
 #endif
 #include "hm_packjob.h"
+#include "hm_soft64.cuh"
 
 // FP64 quiet NaN (the bits of CUDA's CUDART_NAN)
 #define HM_NAN __longlong_as_double(0xfff8000000000000ULL)
@@ -37,39 +38,35 @@ struct KDev {
   int32_t dx, dy;       // user kernel: entries per target / source point (tree dims)
 };
 
-__device__ __forceinline__ double dmul(double a, double b) { return __dmul_rn(a, b); }
-__device__ __forceinline__ double dadd(double a, double b) { return __dadd_rn(a, b); }
-__device__ __forceinline__ double dsub(double a, double b) { return __dsub_rn(a, b); }
-__device__ __forceinline__ double ddiv(double a, double b) { return __ddiv_rn(a, b); }
-
 // LinearAlgebra.generic_norm2 of a 3-vector (see hm_tree.cpp).
-__device__ double norm3_dev(double a, double b, double c) {
+__device__ __noinline__ double norm3_dev(double a, double b, double c) {
   if (isnan(a) || isnan(b) || isnan(c)) return HM_NAN;
   double mx = fabs(a);
   if (fabs(b) > mx) mx = fabs(b);
   if (fabs(c) > mx) mx = fabs(c);
   if (mx == 0.0 || isinf(mx)) return mx;
   if (isfinite(dmul(dmul(3.0, mx), mx)) && dmul(mx, mx) != 0.0)
-    return __dsqrt_rn(dadd(dadd(dmul(a, a), dmul(b, b)), dmul(c, c)));
+    return dsqrt(dadd(dadd(dmul(a, a), dmul(b, b)), dmul(c, c)));
   double qa = ddiv(fabs(a), mx), qb = ddiv(fabs(b), mx), qc = ddiv(fabs(c), mx);
-  return dmul(mx, __dsqrt_rn(dadd(dadd(dmul(qa, qa), dmul(qb, qb)), dmul(qc, qc))));
+  return dmul(mx, dsqrt(dadd(dadd(dmul(qa, qa), dmul(qb, qb)), dmul(qc, qc))));
 }
 
 // examples/hmatrix_vector.jl:12-28
-__device__ double dip_xx(double x, double y, double z) {
+__device__ __noinline__ double dip_xx(double x, double y, double z) {
   double R = dadd(dadd(dmul(x, x), dmul(y, y)), dmul(z, z));
   if (R == 0.0) return 0.0;
   double num = dsub(dsub(dmul(dmul(2.0, x), x), dmul(y, y)), dmul(z, z));
-  return ddiv(ddiv(-num, dmul(dmul(R, R), __dsqrt_rn(R))), 4.0 * 3.141592653589793);
+  return ddiv(ddiv(-num, dmul(dmul(R, R), dsqrt(R))), 4.0 * 3.141592653589793);
 }
-__device__ double dip_xy(double x, double y, double z) {
+__device__ __noinline__ double dip_xy(double x, double y, double z) {
   double R = dadd(dadd(dmul(x, x), dmul(y, y)), dmul(z, z));
   if (R == 0.0) return 0.0;
-  return ddiv(ddiv(dmul(dmul(-3.0, x), y), dmul(dmul(R, R), __dsqrt_rn(R))), 4.0 * 3.141592653589793);
+  return ddiv(ddiv(dmul(dmul(-3.0, x), y), dmul(dmul(R, R), dsqrt(R))), 4.0 * 3.141592653589793);
 }
 
-// K[i, j] for 0-based original (unpermuted) indices.
-__device__ double kentry(const KDev &K, int64_t i, int64_t j) {
+// K[i, j] for 0-based original (unpermuted) indices. Not inlined: it is some hundred
+// instructions long, and the ACA would hold dozens of copies.
+__device__ __noinline__ double kentry(const KDev &K, int64_t i, int64_t j) {
 #ifdef HM_USER_ENTRY
   // a user's kernel (kind HMGPU_KERNEL_USER): its function of the two points
   // and the two components (row i is component i mod dx of point i / dx)
@@ -84,7 +81,7 @@ __device__ double kentry(const KDev &K, int64_t i, int64_t j) {
     case HMGPU_KERNEL_YUKAWA: {
       const double *p = K.X + 3 * i, *q = K.Y + 3 * j;
       double dx = dsub(p[0], q[0]), dy = dsub(p[1], q[1]), dz = dsub(p[2], q[2]);
-      double r = __dsqrt_rn(dadd(dadd(dmul(dx, dx), dmul(dy, dy)), dmul(dz, dz)));
+      double r = dsqrt(dadd(dadd(dmul(dx, dx), dmul(dy, dy)), dmul(dz, dz)));
       if (r == 0.0) return 0.0;
       if (K.kind == HMGPU_KERNEL_LAPLACE3D) return ddiv(0.07957747154594767, r);
       return ddiv(exp(-r), r);
@@ -150,7 +147,7 @@ __device__ __forceinline__ void tsync() {
 
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  for (int o = 16; o > 0; o >>= 1) v = dadd(v, __shfl_xor_sync(0xffffffffu, v, o));
   return v;
 }
 
@@ -170,9 +167,45 @@ __device__ __forceinline__ void tsum(double (&v)[NV], TeamScratch *sc) {
 #pragma unroll
   for (int q = 0; q < NV; q++) {
     double s = sc->v[q][0];
-    for (int u = 1; u < NT / 32; u++) s += sc->v[q][u];
+    for (int u = 1; u < NT / 32; u++) s = dadd(s, sc->v[q][u]);
     v[q] = s;
   }
+}
+// The same sums, one per lane: lane l returns the total of value l / sum_lanes<NV>(). The values are
+// spread over the lanes while they are added (the butterfly's first steps each add half of
+// the values that are left), so that 8 values take 9 additions instead of 40; every partial
+// sum is the butterfly's, whose steps add the same two numbers in either order.
+template <int NV>
+__host__ __device__ constexpr int sum_lanes() {
+  return NV > 4 ? 4 : NV > 2 ? 8 : NV > 1 ? 16 : 32;
+}
+template <int NT, int NV>
+__device__ __forceinline__ double tsum_spread(const double (&v)[NV], TeamScratch *sc) {
+  constexpr int P = 32 / sum_lanes<NV>();
+  const int lane = threadIdx.x & 31;
+  double s[P];
+#pragma unroll
+  for (int q = 0; q < P; q++) s[q] = q < NV ? v[q] : 0.0;
+  int o = 16;
+#pragma unroll
+  for (int h = P / 2; h > 0; h /= 2, o >>= 1) {
+    const bool up = lane & o;
+#pragma unroll
+    for (int q = 0; q < h; q++) {
+      const double mine = up ? s[q + h] : s[q], other = up ? s[q] : s[q + h];
+      s[q] = dadd(mine, __shfl_xor_sync(0xffffffffu, other, o));
+    }
+  }
+#pragma unroll
+  for (; o > 0; o >>= 1) s[0] = dadd(s[0], __shfl_xor_sync(0xffffffffu, s[0], o));
+  if (NT == 32) return s[0];
+  const int w = threadIdx.x >> 5, q = lane / sum_lanes<NV>();
+  __syncthreads();  // earlier readers of the scratch are done
+  if (lane % sum_lanes<NV>() == 0) sc->v[q][w] = s[0];
+  __syncthreads();
+  double t = sc->v[q][0];
+  for (int u = 1; u < NT / 32; u++) t = dadd(t, sc->v[q][u]);
+  return t;
 }
 template <int NT>
 __device__ __forceinline__ double tsum1(double x, TeamScratch *sc) {
@@ -435,7 +468,7 @@ __device__ void aca_team(const KDev &K, const int32_t *tmap0, const int32_t *sma
     k++;
     tsum<NT, 2>(s2, sc);
     tsync<NT>();
-    if (sqrt(s2[1] * s2[0]) < eps) break;  // :95-99
+    if (dsqrt(dmul(s2[1], s2[0])) < eps) break;  // :95-99
     if (k == kcap && it < jb.max_iter) {
       flags |= 2;
       break;
@@ -447,7 +480,7 @@ __device__ void aca_team(const KDev &K, const int32_t *tmap0, const int32_t *sma
   }
 }
 
-__global__ void __launch_bounds__(kBuildThreads, 3) aca_kernel(KDev K, const int32_t *__restrict__ tmap0,
+__global__ void __launch_bounds__(kBuildThreads, 3) aca_kernel(const __grid_constant__ KDev K, const int32_t *__restrict__ tmap0,
                                                             const int32_t *__restrict__ smap0,
                                                             const AcaJob *__restrict__ jobs, int32_t nbig,
                                                             int32_t njobs, double eps, double *ws, AcaRes *res,
@@ -461,7 +494,7 @@ __global__ void __launch_bounds__(kBuildThreads, 3) aca_kernel(KDev K, const int
 
 // Dense blocks generated straight into the product layout (kind-2 pack jobs).
 template <typename T>
-__global__ void gen_dense_kernel(KDev K, const int32_t *__restrict__ tmap0,
+__global__ void gen_dense_kernel(const __grid_constant__ KDev K, const int32_t *__restrict__ tmap0,
                                  const int32_t *__restrict__ smap0, const PackJob *__restrict__ jobs,
                                  int64_t njobs, T *__restrict__ panels) {
   const int lane = threadIdx.x & 31;
@@ -485,7 +518,7 @@ struct SpJob {
   int64_t off;
 };
 
-__global__ void sparsify_kernel(KDev K, const int32_t *__restrict__ tmap0, const int32_t *__restrict__ smap0,
+__global__ void sparsify_kernel(const __grid_constant__ KDev K, const int32_t *__restrict__ tmap0, const int32_t *__restrict__ smap0,
                                 const SpJob *__restrict__ jobs, int64_t njobs, double *__restrict__ out) {
   const int lane = threadIdx.x & 31;
   const int64_t w0 = (blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x) >> 5;

@@ -30,6 +30,7 @@
 // header it includes).
 extern const char hm_src_entry_cuh[];
 extern const char hm_src_packjob_h[];
+extern const char hm_src_soft64_cuh[];
 
 struct hmgpu_user_kernel {
   std::vector<char> cubin;
@@ -188,10 +189,10 @@ extern "C" int hmgpu_user_kernel_compile(const char *source, hmgpu_user_kernel *
   if (!nv.ok) return fail(HMGPU_ERR_UNSUPPORTED, "the NVRTC library (libnvrtc.so.13) cannot be loaded");
   // the user's lines keep their own numbers in the compiler's messages
   const std::string src = prelude() + "#line 1 \"user_kernel.cu\"\n" + source + "\n#include \"hm_entry.cuh\"\n";
-  const char *hdrs[2] = {hm_src_entry_cuh, hm_src_packjob_h};
-  const char *hnames[2] = {"hm_entry.cuh", "hm_packjob.h"};
+  const char *hdrs[3] = {hm_src_entry_cuh, hm_src_packjob_h, hm_src_soft64_cuh};
+  const char *hnames[3] = {"hm_entry.cuh", "hm_packjob.h", "hm_soft64.cuh"};
   nvrtcProgram prog = nullptr;
-  if (nv.create(&prog, src.c_str(), "user_kernel.cu", 2, hdrs, hnames) != NVRTC_SUCCESS)
+  if (nv.create(&prog, src.c_str(), "user_kernel.cu", 3, hdrs, hnames) != NVRTC_SUCCESS)
     return fail(HMGPU_ERR_INVALID, "NVRTC could not create the program");
   std::unique_ptr<nvrtcProgram, void (*)(nvrtcProgram *)> hold(&prog, [](nvrtcProgram *p) { nvrtc().destroy(p); });
   for (const char *n : kNames)

@@ -44,7 +44,8 @@ def _compile(src, extra):
 
 # Headers the library compiles again at run time, with a user's entry function
 # (NVRTC, hm_user.cpp): embedded in the library as strings.
-EMBEDDED = (("hm_src_entry_cuh", "hm_entry.cuh"), ("hm_src_packjob_h", "hm_packjob.h"))
+EMBEDDED = (("hm_src_entry_cuh", "hm_entry.cuh"), ("hm_src_packjob_h", "hm_packjob.h"),
+            ("hm_src_soft64_cuh", "hm_soft64.cuh"))
 
 
 def _embedded_sources():
