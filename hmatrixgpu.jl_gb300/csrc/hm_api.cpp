@@ -207,7 +207,9 @@ int finalize_layout(HMatrix &H, const double *d64, const std::vector<int64_t> &d
   PackJob *djobs = nullptr;
   if ((rc = upload(H, &djobs, p.pjobs))) return rc;
   if (src32 && (f64 || d64)) return fail(HMGPU_ERR_INVALID, "FP32 factors need FP32 storage and generated dense blocks");
-  e = launch_pack_panels(f64, src32, djobs, static_cast<int64_t>(p.pjobs.size()), d64, u64, H.panels, 0);
+  e = launch_zero_pads(f64, H.dp.tiles, H.dp.ntiles, H.panels, 0);
+  if (e == cudaSuccess)
+    e = launch_pack_panels(f64, src32, djobs, static_cast<int64_t>(p.pjobs.size()), d64, u64, H.panels, 0);
   if (e != cudaSuccess) return cuda_fail(e, "pack panels");
   if (gen) {
     rc = gen->generate(H, djobs, static_cast<int64_t>(p.pjobs.size()));

@@ -59,6 +59,8 @@ cudaError_t launch_matvec(bool f64, bool comp, const DevPlan &p, const void *pan
 // or FP32 sources (src32) for FP32 storage.
 cudaError_t launch_pack_panels(bool f64, bool src32, const PackJob *jobs, int64_t njobs, const void *dsrc,
                                const void *usrc, void *panels, cudaStream_t stream);
+// Zeros in the padding columns of every panel row.
+cudaError_t launch_zero_pads(bool f64, const TileDesc *tiles, int32_t ntiles, void *panels, cudaStream_t stream);
 struct VPackJob {
   int64_t src_off, dst_off;
   int32_t n, r, stride, phase;

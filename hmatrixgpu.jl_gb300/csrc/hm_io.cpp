@@ -310,6 +310,9 @@ extern "C" int hmgpu_hmatrix_load(const char *path, hmgpu_hmatrix **out) {
   if (!r.ok || sum != want) return hm::fail(HMGPU_ERR_INVALID, std::string(path) + ": checksum mismatch");
   H->dp.v_dynamic = v_dynamic != 0;
   if ((rc = hm::upload_plan(*H, tmap0, smap0, zero_row))) return rc;
+  // (files written before the padding columns were zeroed hold whatever was there)
+  if (cudaError_t e = hm::launch_zero_pads(H->opt.precision == HMGPU_F64, H->dp.tiles, H->dp.ntiles, H->panels, 0))
+    return hm::cuda_fail(e, "zeroing the padding columns");
   if (H->opt.precision == HMGPU_MIXED && (rc = hm::build_tc(*H))) return rc;
   cudaError_t e = cudaDeviceSynchronize();
   if (e != cudaSuccess) return hm::cuda_fail(e, "loading an H-matrix");

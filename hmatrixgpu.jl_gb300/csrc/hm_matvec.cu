@@ -430,6 +430,32 @@ cudaError_t launch_matvec(bool f64, bool comp, const DevPlan &p, const void *pan
 }
 
 // ---------------------------------------------------------------------------
+// The padding columns [ncols, ld) of every panel row, which no pack job writes and every
+// product multiplies by zero: zeros, not whatever the memory held (0 * NaN is NaN).
+// ---------------------------------------------------------------------------
+template <typename T>
+__global__ void zero_pads_kernel(const TileDesc *__restrict__ tiles, int32_t ntiles, T *__restrict__ panels) {
+  const int lane = threadIdx.x & 31;
+  const int64_t w0 = (blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x) >> 5;
+  const int64_t nw = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
+  for (int64_t t = w0; t < ntiles; t += nw) {
+    const TileDesc d = tiles[t];
+    for (int i = lane; i < d.m; i += 32)
+      for (int c = d.ncols; c < d.ld; c++) panels[d.data_off + static_cast<int64_t>(i) * d.ld + c] = T(0);
+  }
+}
+
+cudaError_t launch_zero_pads(bool f64, const TileDesc *tiles, int32_t ntiles, void *panels, cudaStream_t s) {
+  if (ntiles == 0) return cudaSuccess;
+  const int grid = ntiles < 8 * 4096 ? (ntiles + 7) / 8 : 4096;
+  if (f64)
+    zero_pads_kernel<double><<<grid, kThreads, 0, s>>>(tiles, ntiles, static_cast<double *>(panels));
+  else
+    zero_pads_kernel<float><<<grid, kThreads, 0, s>>>(tiles, ntiles, static_cast<float *>(panels));
+  return cudaGetLastError();
+}
+
+// ---------------------------------------------------------------------------
 // packing: row-major factors (FP64, or FP32 for FP32 storage) -> product
 // layout (one warp per job)
 // ---------------------------------------------------------------------------
