@@ -175,6 +175,7 @@ int upload_plan(HMatrix &H, const std::vector<int32_t> &tmap0, const std::vector
   H.dp.zero_row = zero_row;
   H.dp.x_len = p.x_len;
   H.dp.xt_len = p.xt_len;
+  H.dp.entries = p.panel_len + p.v_len;
   return HMGPU_OK;
 }
 
@@ -578,23 +579,25 @@ extern "C" int hmgpu_matvec(hmgpu_hmatrix *h, const void *x, void *y, int64_t nr
         return rc;
       cudaMemsetAsync(H.xt_multi, 0, H.plan.xt_len * per * es, s);
     }
-    for (int64_t k0 = 0; k0 < nrhs; k0 += per) {
+    for (int64_t k0 = 0, nr = 0; k0 < nrhs; k0 += nr) {
       cudaEvent_t *ev;
       if ((rc = next_events(&ev))) return rc;
-      const int nr = static_cast<int>(std::min<int64_t>(per, nrhs - k0));
+      nr = tc ? std::min<int64_t>(per, nrhs - k0)
+              : hm::multi_pass_columns(f64, nrhs - k0, H.dp.entries, H.num_sms);
       int nl = 0;
       cudaError_t e;
       if (tc)  // scaled FP16 (hi, lo) splits on the tensor cores
         e = hm::launch_matvec_tc(H.dp, H.tc, reinterpret_cast<const float *>(static_cast<const char *>(x) + k0 * ldx * es),
-                                 ldx, nr, reinterpret_cast<float *>(static_cast<char *>(y) + k0 * ldy * es), ldy,
+                                 ldx, static_cast<int>(nr),
+                                 reinterpret_cast<float *>(static_cast<char *>(y) + k0 * ldy * es), ldy,
                                  s, ev, &nl);
       else {
         // each pass width has its own XT (zeroed once): rows that no pass
         // writes (padding, the zero row) must read as zero in that width's layout
-        const int w = hm::multi_width(nr);
+        const int w = hm::multi_width(f64, static_cast<int>(nr));
         void *xt = H.xt_multi;
         if (w < per) {
-          void *&xw = H.xt_multi_w[w == 8 ? 0 : 1];
+          void *&xw = H.xt_multi_w[w == 4 ? 0 : w == 8 ? 1 : 2];
           if (!xw) {
             if ((rc = H.dalloc(&xw, H.plan.xt_len * w * es))) return rc;
             cudaMemsetAsync(xw, 0, H.plan.xt_len * w * es, s);
@@ -602,7 +605,7 @@ extern "C" int hmgpu_matvec(hmgpu_hmatrix *h, const void *x, void *y, int64_t nr
           xt = xw;
         }
         e = hm::launch_matvec_multi(f64, H.dp, H.panels, H.vdata, xt, H.p_multi,
-                                    static_cast<const char *>(x) + k0 * ldx * es, ldx, nr,
+                                    static_cast<const char *>(x) + k0 * ldx * es, ldx, static_cast<int>(nr),
                                     static_cast<char *>(y) + k0 * ldy * es, ldy, H.num_sms, s, ev, &nl);
       }
       if (e != cudaSuccess) return hm::cuda_fail(e, "multi-RHS matvec launch");

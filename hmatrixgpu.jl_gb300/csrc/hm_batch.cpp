@@ -318,20 +318,20 @@ extern "C" int hmgpu_hmatrix_autotune(hmgpu_hmatrix *h, const char *cache_path, 
           best[3] = vd;
         }
       }
-  // crossover: one multi-RHS pass (8, 16 or rhs_per_pass() wide) against
-  // repeated single-RHS products; the threshold is the first k from which
-  // every k' up to a full pass is faster as one pass of its width
+  // crossover: the multi-RHS passes against repeated single-RHS products; the threshold is
+  // the first k from which every k' up to a full pass is faster in passes (a k' between two
+  // measured ones counts as the next)
   if (rc == HMGPU_OK && (rc = apply(H, best[0], best[1], 2, best[3])) == HMGPU_OK) {
-    const int64_t widths[3] = {8, 16, per};
-    float tw[3] = {0.0f, 0.0f, 0.0f};
-    for (int i = 0; i < 3 && rc == HMGPU_OK; i++)
-      rc = time_products(h, x, y, widths[i], n, m, s, e0, e1, 1, 3, &tw[i]);
+    const int64_t cols[5] = {2, 4, 8, 16, per};
+    float tw[5] = {};
+    for (int i = 0; i < 5 && rc == HMGPU_OK; i++)
+      rc = time_products(h, x, y, cols[i], n, m, s, e0, e1, 1, 3, &tw[i]);
     if (rc == HMGPU_OK) {
       int32_t from = 1 << 30;
+      int i = 4;
       for (int64_t k = per; k >= 2; k--) {
-        const int w = hm::multi_width(static_cast<int>(k));
-        const float tm = tw[w == 8 ? 0 : w == 16 ? 1 : 2];
-        if (static_cast<float>(k) * t1 > tm)
+        while (i > 0 && cols[i - 1] >= k) i--;
+        if (static_cast<float>(k) * t1 > tw[i])
           from = static_cast<int32_t>(k);
         else
           break;

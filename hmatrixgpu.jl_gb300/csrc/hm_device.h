@@ -38,6 +38,7 @@ struct DevPlan {
   int32_t *counter = nullptr;  // ticket counters of the passes (16 slots)
   int32_t *status = nullptr;   // device error word (0 = ok), see hmgpu_hmatrix_status
   int64_t m = 0, n = 0, x_len = 0, xt_len = 0;
+  int64_t entries = 0;  // stored entries
 };
 
 constexpr int kThreads = 256;  // threads per CTA of the product kernels
@@ -74,8 +75,10 @@ namespace hm {
 // Multi-right-hand-side plain product (hm_multi.cu): up to rhs_per_pass()
 // right-hand sides per call; xt holds x_len + R rows of rhs_per_pass() values.
 int rhs_per_pass();
-// Width (8, 16 or rhs_per_pass()) of the XT rows of a pass over nr columns.
-int multi_width(int nr);
+// Width (8, 16 or rhs_per_pass(), in FP64 4 too) of the XT rows of a pass over nr columns.
+int multi_width(bool f64, int nr);
+// Columns of the next pass when `left` remain, of a matrix with that many stored entries.
+int multi_pass_columns(bool f64, int64_t left, int64_t entries, int num_sms);
 // Mixed-precision tensor-core product (hm_tc.cu), 32 or 64 right-hand sides
 // per pass.
 struct TcPack {  // one item's FP32 row-major source -> canonical FP16 chunks and row factors

@@ -5,13 +5,25 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <cstdint>
+
 namespace hm {
 
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// Whether the kernels of a pass of `columns` right-hand sides over `entries` stored entries may
+// overlap: always in FP32. The CTAs of a kernel that starts while another ends land where there is
+// room, several on one SM while others get none; that is made good where memory bounds the
+// kernel, but not the FP64 pipe of the SMs (product of a 5266-point cube with 6 right-hand sides 805
+// us with overlap, 452 without; 1000 points on a circle 15.2 and 18.8). So in FP64 only while the
+// pipe's time, 2 FMAs per clock and SM, is short beside the launches.
+inline bool may_overlap(bool f64, int64_t entries, int columns) { return !f64 || entries * columns < 6000000; }
+
+// A launch that may overlap the end of the kernel before it (`overlap`).
 template <typename... P, typename... A>
-static cudaError_t launch_pdl(void (*k)(P...), int grid, int block, size_t smem, cudaStream_t s, A... args) {
+static cudaError_t launch_pdl(bool overlap, void (*k)(P...), int grid, int block, size_t smem, cudaStream_t s,
+                              A... args) {
   cudaLaunchAttribute at{};
   at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at.val.programmaticStreamSerializationAllowed = 1;
@@ -21,7 +33,7 @@ static cudaError_t launch_pdl(void (*k)(P...), int grid, int block, size_t smem,
   c.dynamicSmemBytes = smem;
   c.stream = s;
   c.attrs = &at;
-  c.numAttrs = 1;
+  c.numAttrs = overlap ? 1 : 0;
   return cudaLaunchKernelEx(&c, k, static_cast<P>(args)...);
 }
 

@@ -388,23 +388,24 @@ static cudaError_t run(const DevPlan &p, const T *panels, const T *vdata, T *xt,
                        int grid_v, int grid_du, cudaStream_t s, cudaEvent_t *ev, int *launches) {
   int gp = static_cast<int>((p.x_len + kThreads - 1) / kThreads);
   if (gp > 4096) gp = 4096;
+  const bool overlap = may_overlap(sizeof(T) == 8, p.entries, 1);
   int nl = 0;
   if (ev) cudaEventRecord(ev[0], s);
-  cudaError_t e = launch_pdl(permute_x_kernel<T>, gp, kThreads, 0, s, x, p.smap0, p.n, p.x_len, xt, p.counter);
+  cudaError_t e = launch_pdl(overlap, permute_x_kernel<T>, gp, kThreads, 0, s, x, p.smap0, p.n, p.x_len, xt, p.counter);
   if (e != cudaSuccess) return e;
   nl++;
   if (ev) cudaEventRecord(ev[1], s);
   if (!p.warp_begin_empty) {
     if (p.v_dynamic)
-      e = launch_pdl(v_pass_dyn_kernel<T>, grid_v, kThreads, 0, s, vdata, p.vunits, p.nvunits, xt, p.counter + 8);
+      e = launch_pdl(overlap, v_pass_dyn_kernel<T>, grid_v, kThreads, 0, s, vdata, p.vunits, p.nvunits, xt, p.counter + 8);
     else
-      e = launch_pdl(v_pass_kernel<T>, grid_v, kThreads, 0, s, vdata, p.vunits, p.warp_begin, xt);
+      e = launch_pdl(overlap, v_pass_kernel<T>, grid_v, kThreads, 0, s, vdata, p.vunits, p.warp_begin, xt);
     if (e != cudaSuccess) return e;
     nl++;
   }
   if (ev) cudaEventRecord(ev[2], s);
   DuArgs<T> a{panels, p.tiles, p.units, p.nunits, p.segs, xt, p.tmap0, y, p.counter};
-  e = launch_pdl(du_rows_kernel<T, COMP>, grid_du, kThreads, 0, s, a);
+  e = launch_pdl(overlap, du_rows_kernel<T, COMP>, grid_du, kThreads, 0, s, a);
   if (e != cudaSuccess) return e;
   nl++;
   if (ev) cudaEventRecord(ev[3], s);

@@ -1,8 +1,8 @@
 // Multi-right-hand-side H-matrix product, plain form (FP32 or FP64 on the CUDA
 // cores): Y = H X for up to kRhs right-hand sides per pass.
 //
-// A pass is W right-hand sides wide (W = 8, 16 or 32: the narrowest that holds
-// the pass's columns). XT holds, for every permuted source index and every
+// A pass is W right-hand sides wide (W = 8, 16 or 32, in FP64 4 too: the narrowest
+// that holds the pass's columns). XT holds, for every permuted source index and every
 // rank row, the W values of that row contiguously (row-major, 4W bytes per row
 // in FP32). The matrix is read once per pass and every element feeds W FMAs,
 // so the 32-wide form is bound by the CUDA cores' FMA rate (FP64: by the FP64
@@ -90,11 +90,14 @@ struct Elem {
 
 // Lane layout of a panel of MT rows x W right-hand sides: NG lanes along the
 // right-hand sides (TN each) times RG lanes along the rows (rows rg, rg + RG, ...:
-// TR each). 8 right-hand sides a lane where that leaves 48 or 64 accumulators:
-// 16 shared loads of 16 bytes per 256 FMAs; 4 otherwise.
-template <int W, int MT>
+// TR each). FP32: 8 right-hand sides a lane where that leaves 48 or 64 accumulators (16 shared
+// loads of 16 bytes per 256 FMAs), 4 otherwise. FP64 is bound by the FP64 pipe, which takes
+// as long for an idle lane as for a busy one, and shared loads are cheap beside it: few lanes
+// along the rows (4; 8 of a 4-wide pass), so that a panel of any number of rows wastes little.
+template <typename T, int W, int MT>
 struct LaneTile {
-  static constexpr int TN = W == 32 && MT >= 48 ? 8 : 4;
+  static constexpr bool F64 = sizeof(T) == 8;
+  static constexpr int TN = F64 ? (W >= 8 ? W / 8 : 1) : W == 32 && MT >= 48 ? 8 : 4;
   static constexpr int NG = W / TN, RG = 32 / NG, TR = MT / RG;
   static_assert(TR * RG == MT, "whole rows");
 };
@@ -136,12 +139,16 @@ struct Sums {
     T v[TN];
     __device__ __forceinline__ void load(const unsigned char *p) {
       constexpr int VEC = 16 / sizeof(T);
+      if constexpr (TN < VEC) {
+        v[0] = *reinterpret_cast<const T *>(p);
+      } else {
 #pragma unroll
-      for (int j = 0; j < TN / VEC; j++) {
-        T q[VEC];
-        lds16(p + j * 16, q);
+        for (int j = 0; j < TN / VEC; j++) {
+          T q[VEC];
+          lds16(p + j * 16, q);
 #pragma unroll
-        for (int e = 0; e < VEC; e++) v[j * VEC + e] = q[e];
+          for (int e = 0; e < VEC; e++) v[j * VEC + e] = q[e];
+        }
       }
     }
   };
@@ -189,8 +196,8 @@ struct Sums<float, TR, TN> {
 template <typename T, int W, int MT, typename RowOf>
 __device__ __forceinline__ void slice_product(const T *A, int64_t lda, int m, int ncols, int first, int step,
                                               const T *__restrict__ xt, unsigned char *buf, RowOf row_of,
-                                              Sums<T, LaneTile<W, MT>::TR, LaneTile<W, MT>::TN> &acc) {
-  using L = LaneTile<W, MT>;
+                                              Sums<T, LaneTile<T, W, MT>::TR, LaneTile<T, W, MT>::TN> &acc) {
+  using L = LaneTile<T, W, MT>;
   constexpr int VEC = Elem<T>::kVec, KS = Elem<T>::kStep;
   constexpr int PB = W / VEC;  // 16-byte pieces of an XT row
   constexpr int SB = stage_bytes<T, W>();
@@ -207,7 +214,7 @@ __device__ __forceinline__ void slice_product(const T *A, int64_t lda, int m, in
     const bool in = c0 + piece * VEC < ncols;
     const T *src = arow + (in ? c0 : 0);
 #pragma unroll
-    for (int j = 0; j < MT / 8; j++) {
+    for (int j = 0; j < (MT + 7) / 8; j++) {
       const int r = (lane >> 2) + 8 * j;
       if (r < m) cp16(b + r * 64 + ((piece ^ ((r >> 1) & 3)) << 4), src, in);
       src += 8 * lda;
@@ -241,13 +248,15 @@ __device__ __forceinline__ void slice_product(const T *A, int64_t lda, int m, in
     for (int q = 0; q < 4; q++) {
       T a[L::TR][VEC];
 #pragma unroll
-      for (int i = 0; i < L::TR; i++) lds16(pa + i * L::RG * 64 + ((q ^ (((rg + i * L::RG) >> 1) & 3)) << 4), a[i]);
+      for (int i = 0; i < L::TR; i++)
+        lds16(pa + i * L::RG * 64 + ((q ^ (((rg + i * L::RG) >> 1) & 3)) << 4), a[i]);
 #pragma unroll
       for (int k = 0; k < VEC; k++) {
         typename Sums<T, L::TR, L::TN>::B b;
         b.load(pb + (q * VEC + k) * W * sizeof(T));
 #pragma unroll
-        for (int i = 0; i < L::TR; i++) acc.add(i, a[i][k], b);
+        for (int i = 0; i < L::TR; i++)
+          acc.add(i, a[i][k], b);
       }
     }
     __syncwarp();  // the stage may be filled again
@@ -260,7 +269,7 @@ __device__ __forceinline__ void slice_product(const T *A, int64_t lda, int m, in
 // right-hand sides. By the whole CTA, after every warp's product.
 template <typename T, int W, int NW, int MT, bool ROWS, typename S, typename Emit>
 __device__ __forceinline__ void sum_warps(const S &acc, int m, unsigned char *smem, Emit emit) {
-  using L = LaneTile<W, MT>;
+  using L = LaneTile<T, W, MT>;
   constexpr int LD = W + 1;  // row stride of the sums: no bank conflicts either way
   // the sums of all rows at once where they fit the stages, else of half of them
   constexpr int PARTS = static_cast<size_t>(NW) * MT * LD * sizeof(T) <= multi_smem<T, W, NW>() ? 1 : 2;
@@ -289,17 +298,29 @@ __device__ __forceinline__ void sum_warps(const S &acc, int m, unsigned char *sm
   }
 }
 
-// Row count of the micro-kernel for a panel of m rows.
-template <typename F>
+// Row count of the micro-kernel for a panel of m rows: the smallest form that holds them, in
+// smaller steps in FP64, where every row counts (a row test inside one 64-row form does
+// not help: the FP64 pipe is as busy with instructions that are predicated off).
+template <typename T, typename F>
 __device__ __forceinline__ void with_rows(int m, F f) {
   if (m > 48)
     f(std::integral_constant<int, 64>());
   else if (m > 32)
     f(std::integral_constant<int, 48>());
-  else if (m > 16)
+  else if (sizeof(T) == 4 && m > 16)
     f(std::integral_constant<int, 32>());
-  else
+  else if (sizeof(T) == 4)
     f(std::integral_constant<int, 16>());
+  else if constexpr (sizeof(T) == 8) {
+    if (m > 24)
+      f(std::integral_constant<int, 32>());
+    else if (m > 16)
+      f(std::integral_constant<int, 24>());
+    else if (m > 8)
+      f(std::integral_constant<int, 16>());
+    else
+      f(std::integral_constant<int, 8>());
+  }
 }
 
 // V pass: for every multi-RHS V item
@@ -329,8 +350,8 @@ __global__ void __launch_bounds__(kVWarps * 32, multi_ctas<T, kVWarps>()) v_mult
       next = (big ? ctas : nbig + ctas * kVWarps) + atomicAdd(counter + kTicket[big ? 1 : 2], 1);
     const MVItem I = items[u];
     T *out = (I.kind == 0 ? xt : P) + static_cast<int64_t>(I.out) * W;
-    with_rows(I.nrows, [&](auto mt) {
-      using L = LaneTile<W, mt.value>;
+    with_rows<T>(I.nrows, [&](auto mt) {
+      using L = LaneTile<T, W, mt.value>;
       Sums<T, L::TR, L::TN> acc;
       acc.zero();
       slice_product<T, W, mt.value>(V + I.v_off, I.stride, I.nrows, I.ncols, big ? warp : 0, big ? kVWarps : 1, xt, buf,
@@ -445,8 +466,8 @@ __global__ void __launch_bounds__(kDuWarps * 32, multi_ctas<T, kDuWarps>()) du_m
     int32_t next = 0;
     if (tid == 0) next = static_cast<int32_t>(gridDim.x) + atomicAdd(a.counter + kTicket[0], 1);
     const int32_t *map = a.colmap + U.map;
-    with_rows(U.m, [&](auto mt) {
-      using L = LaneTile<W, mt.value>;
+    with_rows<T>(U.m, [&](auto mt) {
+      using L = LaneTile<T, W, mt.value>;
       Sums<T, L::TR, L::TN> acc;
       acc.zero();
       slice_product<T, W, mt.value>(a.panels + U.data_off, U.ld, U.m, U.ld, warp, kDuWarps, a.xt,
@@ -482,18 +503,19 @@ static cudaError_t run_multi(const DevPlan &p, const T *panels, const T *vdata, 
   multi_attrs<T, W>();
   int gp = static_cast<int>((p.n_src + 63) / 64);
   if (gp > 2048) gp = 2048;
+  const bool overlap = may_overlap(sizeof(T) == 8, p.entries, W);
   int nl = 0;
   if (ev) cudaEventRecord(ev[0], s);
-  cudaError_t e = launch_pdl(permute_multi_kernel<T, W>, gp, kThreads, 0, s, X, ldx, nr, p.sinv0, p.n_src, xt, p.counter);
+  cudaError_t e = launch_pdl(overlap, permute_multi_kernel<T, W>, gp, kThreads, 0, s, X, ldx, nr, p.sinv0, p.n_src, xt, p.counter);
   nl++;
   if (ev) cudaEventRecord(ev[1], s);
   if (e == cudaSuccess && p.nmv > 0) {
     const int32_t nbig = sizeof(T) == 4 ? p.nmv_big : p.nmv;
-    e = launch_pdl(v_multi_kernel<T, W>, num_sms * multi_ctas<T, kVWarps>(), kVWarps * 32,
+    e = launch_pdl(overlap, v_multi_kernel<T, W>, num_sms * multi_ctas<T, kVWarps>(), kVWarps * 32,
                    multi_smem<T, W, kVWarps>(), s, vdata, p.mv_items, nbig, p.nmv, xt, P, p.counter);
     nl++;
     if (e == cudaSuccess && p.nmvr > 0) {
-      e = launch_pdl(reduce_multi_kernel<T, W>, p.nmvr < 4096 ? p.nmvr : 4096, kThreads, 0, s, p.mv_reduce, p.nmvr, P,
+      e = launch_pdl(overlap, reduce_multi_kernel<T, W>, p.nmvr < 4096 ? p.nmvr : 4096, kThreads, 0, s, p.mv_reduce, p.nmvr, P,
                      xt);
       nl++;
     }
@@ -501,7 +523,7 @@ static cudaError_t run_multi(const DevPlan &p, const T *panels, const T *vdata, 
   if (ev) cudaEventRecord(ev[2], s);
   DuMultiArgs<T> a{panels, p.munits, p.nmunits, p.mcolmap, xt, p.tmap0, Y, ldy, nr, p.counter};
   if (e == cudaSuccess)
-    e = launch_pdl(du_multi_kernel<T, W>, num_sms * multi_ctas<T, kDuWarps>(), kDuWarps * 32,
+    e = launch_pdl(overlap, du_multi_kernel<T, W>, num_sms * multi_ctas<T, kDuWarps>(), kDuWarps * 32,
                    multi_smem<T, W, kDuWarps>(), s, a);
   nl++;
   if (ev) cudaEventRecord(ev[3], s);
@@ -511,13 +533,40 @@ static cudaError_t run_multi(const DevPlan &p, const T *panels, const T *vdata, 
 
 int rhs_per_pass() { return kRhs; }
 
-int multi_width(int nr) { return nr <= 8 ? 8 : nr <= 16 ? 16 : kRhs; }
+int multi_width(bool f64, int nr) { return nr <= 4 && f64 ? 4 : nr <= 8 ? 8 : nr <= 16 ? 16 : kRhs; }
+
+// FP32 passes are as wide as they can be: they read the matrix once. In FP64 a pass's time is
+// that of the FP64 pipe, in proportion to its width, beside some 12 us of launches and latency, so the
+// columns are split into the widths with the least sum of both (18 columns of a million
+// entries or more: 16 and 4 wide, not 32). A row's sum does not depend on the width.
+int multi_pass_columns(bool f64, int64_t left, int64_t entries, int num_sms) {
+  if (!f64 || left >= kRhs) return static_cast<int>(left < kRhs ? left : kRhs);
+  const double column = static_cast<double>(entries) / (2.0 * num_sms * 1900.0);  // us of the FP64 pipe per column
+  double best[kRhs + 1] = {0.0};
+  int first[kRhs + 1] = {0};
+  for (int r = 1; r <= left; r++) {
+    best[r] = 1e300;
+    for (int w : {32, 16, 8, 4}) {
+      const int n = w < r ? w : r;
+      const double t = 12.0 + w * column + best[r - n];
+      if (t < best[r]) {
+        best[r] = t;
+        first[r] = n;
+      }
+    }
+  }
+  return first[left];
+}
 
 template <typename T>
 static cudaError_t run_multi_w(const DevPlan &p, const T *panels, const T *vdata, T *xt, T *P, const T *X,
                                int64_t ldx, int nr, T *Y, int64_t ldy, int num_sms, cudaStream_t s,
                                cudaEvent_t *ev, int *launches) {
-  switch (multi_width(nr)) {
+  switch (multi_width(sizeof(T) == 8, nr)) {
+    case 4:
+      if constexpr (sizeof(T) == 8)
+        return run_multi<T, 4>(p, panels, vdata, xt, P, X, ldx, nr, Y, ldy, num_sms, s, ev, launches);
+      return cudaErrorInvalidValue;
     case 8: return run_multi<T, 8>(p, panels, vdata, xt, P, X, ldx, nr, Y, ldy, num_sms, s, ev, launches);
     case 16: return run_multi<T, 16>(p, panels, vdata, xt, P, X, ldx, nr, Y, ldy, num_sms, s, ev, launches);
     default: return run_multi<T, kRhs>(p, panels, vdata, xt, P, X, ldx, nr, Y, ldy, num_sms, s, ev, launches);
