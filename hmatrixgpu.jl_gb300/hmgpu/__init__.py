@@ -557,6 +557,13 @@ def _is_torch(a):
     return type(a).__module__.startswith("torch")
 
 
+def _current_stream(device):
+    """The raw handle of torch's current stream on a CUDA device."""
+    import torch
+    raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)  # the public call takes 2 us, this one 0.1
+    return raw(device.index) if raw is not None else torch.cuda.current_stream(device).cuda_stream
+
+
 class Shard:
     """Rows [row_begin, row_end) of an H-matrix in the permuted target order
     (hmgpu_hmatrix_shard). Each owned row of its product is bitwise the row
@@ -646,9 +653,8 @@ class Graph:
         self._g = g
 
     def launch(self, stream=None):
-        import torch
         if stream is None:
-            stream = torch.cuda.current_stream(self.x.device).cuda_stream
+            stream = _current_stream(self.x.device)
         check(lib().hmgpu_graph_launch(self._g, C.c_void_p(stream)))
         return self.y
 
@@ -670,18 +676,22 @@ def mul_(y, H, x, stream=None):
         want = torch.float64 if H.dtype == np.float64 else torch.float32
         if x.dtype != want or y.dtype != want:
             raise TypeError(f"x and y must be {want} for this H-matrix")
-        nrhs = 1 if x.dim() == 1 else x.shape[1]
-        if x.shape[0] != n or y.shape[0] != m or (x.dim() == 2 and y.shape[1] != nrhs):
+        two = x.dim() == 2
+        nrhs = x.shape[1] if two else 1
+        if x.shape[0] != n or y.shape[0] != m or (two and y.shape[1] != nrhs):
             raise ValueError("dimension mismatch")
-        if x.dim() == 2 and (x.stride(0) != 1 or y.stride(0) != 1):
+        if two and (x.stride(0) != 1 or y.stride(0) != 1):
             raise ValueError("x and y must be column-major (use .t().contiguous().t())")
-        ldx = x.stride(1) if x.dim() == 2 else n
+        ldx = x.stride(1) if two else n
         ldy = y.stride(1) if y.dim() == 2 else m
+        device = x.device
         if stream is None:
-            stream = torch.cuda.current_stream(x.device).cuda_stream
-        with torch.cuda.device(x.device):
-            check(L.hmgpu_matvec(H._h, C.c_void_p(x.data_ptr()), C.c_void_p(y.data_ptr()), nrhs,
-                                 ldx, ldy, C.c_void_p(stream)))
+            stream = _current_stream(device)
+        if torch.cuda.current_device() == device.index:
+            check(L.hmgpu_matvec(H._h, x.data_ptr(), y.data_ptr(), nrhs, ldx, ldy, stream))
+        else:
+            with torch.cuda.device(device):
+                check(L.hmgpu_matvec(H._h, x.data_ptr(), y.data_ptr(), nrhs, ldx, ldy, stream))
         return y
     xa = np.asarray(x)
     if xa.dtype != H.dtype:
