@@ -114,7 +114,11 @@ int upload_plan(HMatrix &H, const std::vector<int32_t> &tmap0, const std::vector
   if ((rc = upload(H, &H.dp.segs, p.segs))) return rc;
   if ((rc = upload_units(H))) return rc;
   if ((rc = upload(H, &H.dp.tmap0, tmap0))) return rc;
-  if ((rc = upload(H, &H.dp.smap0, smap0))) return rc;
+  {
+    std::vector<int32_t> sm = smap0;  // to the end of XT's x region, which the kernels read as a whole
+    sm.resize(static_cast<size_t>(p.x_len), -1);
+    if ((rc = upload(H, &H.dp.smap0, sm))) return rc;
+  }
   {
     int64_t n_src = 0;
     for (int32_t v : smap0) n_src = std::max<int64_t>(n_src, static_cast<int64_t>(v) + 1);
@@ -200,6 +204,7 @@ int finalize_layout(HMatrix &H, const double *d64, const std::vector<int64_t> &d
   std::vector<int32_t> t0(H.bs.m), s0(H.bs.n);
   for (int64_t i = 0; i < H.bs.m; i++) t0[i] = static_cast<int32_t>(H.bs.tmap[i] - 1);
   for (int64_t j = 0; j < H.bs.n; j++) s0[j] = static_cast<int32_t>(H.bs.smap[j] - 1);
+  H.dp.v_dynamic = p.v_len * static_cast<int64_t>(es) > kDynamicVBytes;
   if ((rc = upload_plan(H, t0, s0, H.bs.n))) return rc;
   H.build_phase[4] = clk.lap();
   cudaError_t e;

@@ -87,6 +87,7 @@ extern "C" int hmgpu_hmatrix_batch(hmgpu_hmatrix *const *members, int32_t count,
                      cudaMemcpyDeviceToDevice);
     if (e != cudaSuccess) return hm::cuda_fail(e, "copying a batch member");
   }
+  B->dp.v_dynamic = P.v_len * static_cast<int64_t>(es) > hm::kDynamicVBytes;
   // the padding entry after member 0's x is always zero
   if ((rc = hm::upload_plan(*B, tmap0, smap0, M[0]->bs.n))) return rc;
   if (B->opt.precision == HMGPU_MIXED && (rc = hm::build_tc(*B))) return rc;

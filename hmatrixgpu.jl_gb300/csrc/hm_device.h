@@ -23,7 +23,7 @@ struct DevPlan {
   int32_t *warp_begin = nullptr;
   int32_t nwarps = 0;
   bool warp_begin_empty = true;  // no V units (no low-rank blocks)
-  bool v_dynamic = true;         // V units from a ticket counter instead of warp ranges
+  bool v_dynamic = false;        // V units from a ticket counter instead of warp ranges
   MVItem *mv_items = nullptr;  // multi-RHS V items: those of many columns first
   int32_t nmv = 0;
   int32_t nmv_big = 0;         // items of more than kMvWarpCols columns
@@ -31,7 +31,7 @@ struct DevPlan {
   int32_t nmvr = 0;
   int64_t p_rows = 0;
   int32_t *tmap0 = nullptr;  // 0-based target map, length m
-  int32_t *smap0 = nullptr;  // 0-based source map, length n (-1: a zero entry)
+  int32_t *smap0 = nullptr;  // 0-based source map, length x_len (-1: a zero entry)
   int64_t zero_row = 0;      // an XT row that is always zero
   int32_t *sinv0 = nullptr;  // XT row of each 0-based source index (inverse of smap0)
   int64_t n_src = 0;
@@ -42,6 +42,8 @@ struct DevPlan {
 };
 
 constexpr int kThreads = 256;  // threads per CTA of the product kernels
+// V rows of more bytes than this (about the L2 cache) are taken by ticket, see v_unit
+constexpr int64_t kDynamicVBytes = int64_t(128) << 20;
 constexpr int kMvWarpCols = 128;  // a multi-RHS V item of at most this many columns goes to one warp (FP32)
 
 // Resident CTAs per SM of the V pass and of the near/U pass for an element type.

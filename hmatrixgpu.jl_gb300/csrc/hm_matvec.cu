@@ -13,6 +13,8 @@
 // and stay in L2.
 #include <cuda_runtime.h>
 
+#include <type_traits>
+
 #include "hm_device.h"
 #include "hm_launch.cuh"
 
@@ -97,14 +99,36 @@ struct RowAcc {
   }
 };
 
+// The vector that the two passes read: XT = [x permuted | t], or, for a matrix whose V
+// and near/U units all fit the resident warps and CTAs (DIRECT), x itself through the source map
+// in place of its permuted copy: one launch less, where launches are most of the time (1000
+// points, FP64: 9.1 us, 11.6 with the permutation), and no tickets, since every unit has a warp or CTA of its own.
+template <typename T>
+struct XSrc {
+  const T *xt;
+  const T *x;
+  const int32_t *smap0;  // x_len entries, -1: zero
+  int32_t x_len;
+};
+
+// 16 bytes of the x region at entry e (a multiple of the vector), through the source map
+__device__ __forceinline__ float4 gather_x(const XSrc<float> &s, int32_t e) {
+  const int4 i = __ldg(reinterpret_cast<const int4 *>(s.smap0 + e));
+  return make_float4(i.x >= 0 ? __ldg(s.x + i.x) : 0.0f, i.y >= 0 ? __ldg(s.x + i.y) : 0.0f,
+                     i.z >= 0 ? __ldg(s.x + i.z) : 0.0f, i.w >= 0 ? __ldg(s.x + i.w) : 0.0f);
+}
+__device__ __forceinline__ double2 gather_x(const XSrc<double> &s, int32_t e) {
+  const int2 i = __ldg(reinterpret_cast<const int2 *>(s.smap0 + e));
+  return make_double2(i.x >= 0 ? __ldg(s.x + i.x) : 0.0, i.y >= 0 ? __ldg(s.x + i.y) : 0.0);
+}
+
 // ---------------------------------------------------------------------------
-// x permutation: XT[j] = x[smap[j]] for j < n (zero where smap[j] < 0), zero
-// padding up to x_len.
+// x permutation: XT[j] = x[smap[j]] for j < x_len (zero where smap[j] < 0).
 // Also re-arms the unit ticket of the near/U pass.
 // ---------------------------------------------------------------------------
 template <typename T>
 __global__ void permute_x_kernel(const T *__restrict__ x, const int32_t *__restrict__ smap0,
-                                 int64_t n, int64_t x_len, T *__restrict__ xt,
+                                 int64_t x_len, T *__restrict__ xt,
                                  int32_t *__restrict__ counter) {
   int64_t j = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
   pdl_wait();
@@ -114,19 +138,19 @@ __global__ void permute_x_kernel(const T *__restrict__ x, const int32_t *__restr
     counter[8] = 0;  // V units (dynamic schedule)
   }
   for (; j < x_len; j += static_cast<int64_t>(gridDim.x) * blockDim.x)
-    xt[j] = (j < n && smap0[j] >= 0) ? x[smap0[j]] : T(0);  // negative: padding between batch members
+    xt[j] = smap0[j] >= 0 ? x[smap0[j]] : T(0);  // negative: padding, between batch members too
 }
 
 // ---------------------------------------------------------------------------
 // V pass. A unit is a run of rank rows of one block; `lanes` lanes share a
 // row and 32/lanes rows run side by side. Row storage is phase-aligned with
-// XT, so element p of the row pairs with XT[x_off + p]. Warps take units one at
-// a time from a ticket counter, largest first (the first one is the warp's own
-// number, the next ticket is drawn before the current unit runs). The other
-// schedule, which a caller or the autotuner may set: each warp owns a
-// contiguous, byte-balanced range of units, planned on the host. Measured in us
-// with tickets / ranges: film 2^20 FP32 507 / 540, 40,960-point cube FP64
-// 372 / 427, batch of 12 spheres 77 / 96, one sphere of 20,011 points 31 / 29.
+// XT, so element p of the row pairs with XT[x_off + p]. Two schedules. Matrices whose V
+// rows exceed the L2 cache take tickets: warps take units one at a time from a counter,
+// largest first (the first one is the warp's own number, the next ticket is drawn before
+// the current unit runs). On smaller ones each warp owns a contiguous, byte-balanced range
+// of units, planned on the host. Measured in us with tickets / ranges, V pass: film 2^20
+// FP32 507 / 540, 40,960-point cube FP64 372 / 427, batch of 12 spheres 77 / 96, one sphere of
+// 20,011 points 31 / 29; whole product: film 40,000 72 / 65, 17,921 33 / 30.
 // ---------------------------------------------------------------------------
 // Six CTAs per SM (40 registers) and four loads in flight per lane: the pass
 // is bound by memory latency, like the near/U pass.
@@ -183,6 +207,44 @@ __device__ __forceinline__ void v_unit(const T *__restrict__ V, const VUnit U, T
   }
 }
 
+// The same unit with x read through the source map (the sums in the same order).
+template <typename T>
+__device__ __forceinline__ void v_unit_direct(const T *__restrict__ V, const VUnit U, const XSrc<T> &src,
+                                              T *__restrict__ xt, int lane) {
+  using VT = typename Vec16<T>::type;
+  constexpr int VEC = Vec16<T>::N;
+  const int g = U.lanes, slot = lane / g, sub = lane - slot * g, per = 32 / g;
+  const int nv = U.stride / VEC;
+  for (int k0 = 0; k0 < U.nrows; k0 += per) {
+    const int k = k0 + slot;
+    T acc = T(0);
+    if (k < U.nrows) {
+      const VT *row = reinterpret_cast<const VT *>(V + U.v_off + static_cast<int64_t>(k) * U.stride);
+      // n vectors in flight, and no FMA that is predicated off (the FP64 pipe would be as busy with it)
+      auto some = [&](auto n, int p) {
+        VT a[n.value], b[n.value];
+#pragma unroll
+        for (int z = 0; z < n.value; z++) {
+          a[z] = ld_stream(row + p + z * g);
+          b[z] = gather_x(src, U.x_off + (p + z * g) * VEC);
+        }
+#pragma unroll
+        for (int z = 0; z < n.value; z++) {
+          const T *ea = reinterpret_cast<const T *>(&a[z]), *eb = reinterpret_cast<const T *>(&b[z]);
+#pragma unroll
+          for (int q = 0; q < VEC; q++) acc = fma_(ea[q], eb[q], acc);
+        }
+      };
+      int p = sub;
+      for (; p + 3 * g < nv; p += 4 * g) some(std::integral_constant<int, 4>(), p);
+      for (; p + g < nv; p += 2 * g) some(std::integral_constant<int, 2>(), p);
+      if (p < nv) some(std::integral_constant<int, 1>(), p);
+    }
+    for (int o = g >> 1; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    if (sub == 0 && k < U.nrows) xt[U.t_off + k] = acc;
+  }
+}
+
 template <typename T>
 __global__ void __launch_bounds__(kThreads, 6) v_pass_kernel(const T *__restrict__ V,
                                                           const VUnit *__restrict__ units,
@@ -216,6 +278,19 @@ __global__ void __launch_bounds__(kThreads, 6) v_pass_dyn_kernel(const T *__rest
   }
 }
 
+// One unit per warp, straight from x.
+template <typename T>
+__global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 6 : 5) v_pass_direct_kernel(const T *__restrict__ V,
+                                                                const VUnit *__restrict__ units, int32_t nunits,
+                                                                const XSrc<T> src, T *__restrict__ xt) {
+  const int u = static_cast<int>((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+  if (u >= nunits) return;
+  const VUnit U = units[u];
+  pdl_wait();  // x is there, and t no longer read
+  pdl_trigger();
+  v_unit_direct(V, U, src, xt, threadIdx.x & 31);
+}
+
 // ---------------------------------------------------------------------------
 // Near/U pass. CTAs take row units (rows of one tile) from a ticket counter
 // (the first one is the CTA's own number, its tables are read while the V pass
@@ -236,7 +311,7 @@ struct DuArgs {
   const RowUnit *units;
   int32_t nunits;
   const Seg *segs;
-  const T *xt;
+  XSrc<T> src;
   const int32_t *tmap0;
   T *y;
   int32_t *counter;
@@ -251,7 +326,7 @@ constexpr int kDuSegs = 512;
 // Six CTAs per SM (40 registers, a few spilled to L1) keep more rows, and so
 // more 16-byte loads, in flight than five CTAs without spills: the pass is
 // bound by memory latency, not by the instructions the spills add.
-template <typename T, bool COMP>
+template <typename T, bool COMP, bool DIRECT>
 __global__ void __launch_bounds__(kThreads, 6) du_rows_kernel(DuArgs<T> a) {
   using VT = typename Vec16<T>::type;
   constexpr int VEC = Vec16<T>::N;
@@ -272,7 +347,7 @@ __global__ void __launch_bounds__(kThreads, 6) du_rows_kernel(DuArgs<T> a) {
       pdl_trigger();
     }
     int32_t next = 0;
-    if (tid == 0) next = static_cast<int32_t>(gridDim.x) + atomicAdd(a.counter, 1);
+    if (!DIRECT && tid == 0) next = static_cast<int32_t>(gridDim.x) + atomicAdd(a.counter, 1);
     // Rows 16 at a time (a warp per row pair); a unit has more than 16 rows
     // only when its tile fits one chunk of entries, which are then gathered
     // once for all its rows.
@@ -297,7 +372,13 @@ __global__ void __launch_bounds__(kThreads, 6) du_rows_kernel(DuArgs<T> a) {
                 else
                   hi = mid - 1;
               }
-              v = a.xt[S[lo].vec_off + (c - S[lo].col0)];
+              const int32_t e = S[lo].vec_off + (c - S[lo].col0);
+              if (DIRECT && e < a.src.x_len) {
+                const int32_t i = a.src.smap0[e];
+                if (i >= 0) v = a.src.x[i];
+              } else {
+                v = a.src.xt[e];
+              }
             }
             vals[j] = v;
           }
@@ -357,6 +438,7 @@ __global__ void __launch_bounds__(kThreads, 6) du_rows_kernel(DuArgs<T> a) {
         if (hb) a.y[a.tmap0[d.row0 + ib]] = yb;
       }
     }
+    if (DIRECT) break;  // a unit per CTA
     if (tid == 0) s_ticket = next;
     __syncthreads();  // the entries and segments are no longer read
     u = s_ticket;
@@ -375,37 +457,49 @@ int occupancy_v(bool f64) {
 int occupancy_du(bool f64, bool comp) {
   int n = 0;
   if (f64)
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, du_rows_kernel<double, false>, kThreads, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, du_rows_kernel<double, false, false>, kThreads, 0);
   else if (comp)
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, du_rows_kernel<float, true>, kThreads, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, du_rows_kernel<float, true, false>, kThreads, 0);
   else
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, du_rows_kernel<float, false>, kThreads, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, du_rows_kernel<float, false, false>, kThreads, 0);
   return n > 0 ? n : 1;
 }
 
 template <typename T, bool COMP>
 static cudaError_t run(const DevPlan &p, const T *panels, const T *vdata, T *xt, const T *x, T *y,
                        int grid_v, int grid_du, cudaStream_t s, cudaEvent_t *ev, int *launches) {
-  int gp = static_cast<int>((p.x_len + kThreads - 1) / kThreads);
-  if (gp > 4096) gp = 4096;
   const bool overlap = may_overlap(sizeof(T) == 8, p.entries, 1);
+  const bool direct = p.nvunits <= grid_v * (kThreads / 32) && p.nunits <= grid_du;
   int nl = 0;
+  cudaError_t e = cudaSuccess;
   if (ev) cudaEventRecord(ev[0], s);
-  cudaError_t e = launch_pdl(overlap, permute_x_kernel<T>, gp, kThreads, 0, s, x, p.smap0, p.n, p.x_len, xt, p.counter);
-  if (e != cudaSuccess) return e;
-  nl++;
+  if (!direct) {
+    int gp = static_cast<int>((p.x_len + kThreads - 1) / kThreads);
+    if (gp > 4096) gp = 4096;
+    e = launch_pdl(overlap, permute_x_kernel<T>, gp, kThreads, 0, s, x, p.smap0, p.x_len, xt, p.counter);
+    if (e != cudaSuccess) return e;
+    nl++;
+  }
+  const XSrc<T> src{xt, x, p.smap0, static_cast<int32_t>(p.x_len)};
   if (ev) cudaEventRecord(ev[1], s);
   if (!p.warp_begin_empty) {
-    if (p.v_dynamic)
-      e = launch_pdl(overlap, v_pass_dyn_kernel<T>, grid_v, kThreads, 0, s, vdata, p.vunits, p.nvunits, xt, p.counter + 8);
+    if (direct)
+      e = launch_pdl(overlap, v_pass_direct_kernel<T>, (p.nvunits + kThreads / 32 - 1) / (kThreads / 32), kThreads, 0, s,
+                     vdata, p.vunits, p.nvunits, src, xt);
+    else if (p.v_dynamic)
+      e = launch_pdl(overlap, v_pass_dyn_kernel<T>, grid_v, kThreads, 0, s, vdata, p.vunits, p.nvunits, xt,
+                     p.counter + 8);
     else
       e = launch_pdl(overlap, v_pass_kernel<T>, grid_v, kThreads, 0, s, vdata, p.vunits, p.warp_begin, xt);
     if (e != cudaSuccess) return e;
     nl++;
   }
   if (ev) cudaEventRecord(ev[2], s);
-  DuArgs<T> a{panels, p.tiles, p.units, p.nunits, p.segs, xt, p.tmap0, y, p.counter};
-  e = launch_pdl(overlap, du_rows_kernel<T, COMP>, grid_du, kThreads, 0, s, a);
+  DuArgs<T> a{panels, p.tiles, p.units, p.nunits, p.segs, src, p.tmap0, y, p.counter};
+  if (direct)
+    e = launch_pdl(overlap, du_rows_kernel<T, COMP, true>, p.nunits, kThreads, 0, s, a);
+  else
+    e = launch_pdl(overlap, du_rows_kernel<T, COMP, false>, grid_du, kThreads, 0, s, a);
   if (e != cudaSuccess) return e;
   nl++;
   if (ev) cudaEventRecord(ev[3], s);

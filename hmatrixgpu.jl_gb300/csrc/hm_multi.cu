@@ -102,6 +102,14 @@ struct LaneTile {
   static_assert(TR * RG == MT, "whole rows");
 };
 
+// Sets of sums a lane keeps, the four quarters of a stage in turn: narrow FP32 passes have the
+// registers, and the shorter chains of additions are closer to the exact sum. By the width alone, so
+// that a row's sum does not depend on how its tile's rows are cut.
+template <typename T, int W>
+constexpr int sum_sets() {
+  return sizeof(T) == 8 || W == 32 ? 1 : 32 / W;
+}
+
 // Stages of one warp: per stage 64 rows x 64 bytes of the panel, the 16-byte
 // pieces of row r swapped by (r / 2) mod 4 (eight consecutive rows then touch all
 // banks once), then kStep rows of XT.
@@ -156,6 +164,12 @@ struct Sums {
 #pragma unroll
     for (int j = 0; j < TN; j++) v[i][j] = fma(a, b.v[j], v[i][j]);
   }
+  __device__ __forceinline__ void add(const Sums &o) {
+#pragma unroll
+    for (int i = 0; i < TR; i++)
+#pragma unroll
+      for (int j = 0; j < TN; j++) v[i][j] += o.v[i][j];
+  }
   __device__ __forceinline__ T get(int i, int j) const { return v[i][j]; }
 };
 template <int TR, int TN>
@@ -184,12 +198,18 @@ struct Sums<float, TR, TN> {
 #pragma unroll
     for (int j = 0; j < TN / 2; j++) asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(v[i][j]) : "l"(aa), "l"(b.v[j]));
   }
+  __device__ __forceinline__ void add(const Sums &o) {
+#pragma unroll
+    for (int i = 0; i < TR; i++)
+#pragma unroll
+      for (int j = 0; j < TN / 2; j++) asm("add.rn.f32x2 %0, %0, %1;" : "+l"(v[i][j]) : "l"(o.v[i][j]));
+  }
   __device__ __forceinline__ float get(int i, int j) const {
     return __uint_as_float(static_cast<unsigned>(j & 1 ? v[i][j / 2] >> 32 : v[i][j / 2]));
   }
 };
 
-// acc += panel x XT over the column stages first, first + step, ... of a panel of m <=
+// acc = panel x XT over the column stages first, first + step, ... of a panel of m <=
 // MT rows (row-major, stride lda, ncols a multiple of 4), by one warp. row_of(c)
 // is the XT row of column c, -1 for a zero row; lane l asks for column l of a
 // stage, one stage ahead. `buf`: the warp's two stages.
@@ -197,6 +217,10 @@ template <typename T, int W, int MT, typename RowOf>
 __device__ __forceinline__ void slice_product(const T *A, int64_t lda, int m, int ncols, int first, int step,
                                               const T *__restrict__ xt, unsigned char *buf, RowOf row_of,
                                               Sums<T, LaneTile<T, W, MT>::TR, LaneTile<T, W, MT>::TN> &acc) {
+  constexpr int SETS = sum_sets<T, W>();
+  Sums<T, LaneTile<T, W, MT>::TR, LaneTile<T, W, MT>::TN> set[SETS];
+#pragma unroll
+  for (int z = 0; z < SETS; z++) set[z].zero();
   using L = LaneTile<T, W, MT>;
   constexpr int VEC = Elem<T>::kVec, KS = Elem<T>::kStep;
   constexpr int PB = W / VEC;  // 16-byte pieces of an XT row
@@ -256,12 +280,15 @@ __device__ __forceinline__ void slice_product(const T *A, int64_t lda, int m, in
         b.load(pb + (q * VEC + k) * W * sizeof(T));
 #pragma unroll
         for (int i = 0; i < L::TR; i++)
-          acc.add(i, a[i][k], b);
+          set[q % SETS].add(i, a[i][k], b);
       }
     }
     __syncwarp();  // the stage may be filled again
   }
   cp_wait_all();
+  acc = set[0];
+#pragma unroll
+  for (int z = 1; z < SETS; z++) acc.add(set[z]);
 }
 
 // The warps' sums of a panel of m <= MT rows, added in warp order: emit(row, q, sum) for
@@ -353,7 +380,6 @@ __global__ void __launch_bounds__(kVWarps * 32, multi_ctas<T, kVWarps>()) v_mult
     with_rows<T>(I.nrows, [&](auto mt) {
       using L = LaneTile<T, W, mt.value>;
       Sums<T, L::TR, L::TN> acc;
-      acc.zero();
       slice_product<T, W, mt.value>(V + I.v_off, I.stride, I.nrows, I.ncols, big ? warp : 0, big ? kVWarps : 1, xt, buf,
                                     [&](int c) { return c < I.ncols ? I.x_off + c : -1; }, acc);
       if (big) {
@@ -469,7 +495,6 @@ __global__ void __launch_bounds__(kDuWarps * 32, multi_ctas<T, kDuWarps>()) du_m
     with_rows<T>(U.m, [&](auto mt) {
       using L = LaneTile<T, W, mt.value>;
       Sums<T, L::TR, L::TN> acc;
-      acc.zero();
       slice_product<T, W, mt.value>(a.panels + U.data_off, U.ld, U.m, U.ld, warp, kDuWarps, a.xt,
                                     dyn_smem + warp * 2 * stage_bytes<T, W>(),
                                     [&](int c) { return c < U.ncols ? __ldg(map + c) : -1; }, acc);

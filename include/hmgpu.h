@@ -388,8 +388,8 @@ int hmgpu_hmatrix_autotune(hmgpu_hmatrix *H, const char *cache_path, int32_t *re
 /* The product parameters in force (no counterpart in the reference): rows per
  * near/U unit, V unit KiB at most (small matrices take smaller units), multi-RHS
  * threshold, V schedule (0: each warp owns a byte-balanced range of V units, 1:
- * warps take V units from a ticket counter, the default; the autotuner times
- * both). Writes min(n, 4) values. */
+ * warps take V units from a ticket counter, the default for large matrices; the
+ * autotuner times both). Writes min(n, 4) values. */
 int hmgpu_hmatrix_tuning(const hmgpu_hmatrix *H, int32_t *values, int32_t n);
 /* Sets those four parameters directly (for instance from an earlier autotune
  * on the same structure); n must be 4. Results do not depend on them. */
