@@ -22,13 +22,13 @@ inline bool may_overlap(bool f64, int64_t entries, int columns) { return !f64 ||
 
 // A launch that may overlap the end of the kernel before it (`overlap`).
 template <typename... P, typename... A>
-static cudaError_t launch_pdl(bool overlap, void (*k)(P...), int grid, int block, size_t smem, cudaStream_t s,
-                              A... args) {
+static cudaError_t launch_pdl(bool overlap, void (*k)(P...), dim3 grid, int block, size_t smem, cudaStream_t s,
+                              const A &...args) {
   cudaLaunchAttribute at{};
   at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at.val.programmaticStreamSerializationAllowed = 1;
   cudaLaunchConfig_t c{};
-  c.gridDim = dim3(static_cast<unsigned>(grid));
+  c.gridDim = grid;
   c.blockDim = dim3(static_cast<unsigned>(block));
   c.dynamicSmemBytes = smem;
   c.stream = s;

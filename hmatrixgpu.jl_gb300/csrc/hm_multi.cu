@@ -58,8 +58,9 @@ __global__ void permute_multi_kernel(const T *__restrict__ X, int64_t ldx, int n
   pdl_trigger();
   if (blockIdx.x == 0 && threadIdx.x < kTickets) counter[kTicket[threadIdx.x]] = 0;
   for (int64_t j0 = blockIdx.x * 64ll; j0 < n_src; j0 += gridDim.x * 64ll) {
-    for (int e = threadIdx.x; e < 64 * W; e += blockDim.x) {
-      const int r = e / 64, jj = e % 64;  // consecutive threads: consecutive j
+#pragma unroll
+    for (int i = 0; i < W / 4; i++) {  // all of a thread's loads in flight
+      const int e = threadIdx.x + i * kThreads, r = e / 64, jj = e % 64;  // consecutive threads: consecutive j
       const int64_t j = j0 + jj;
       tile[jj][r] = (j < n_src && r < nr) ? X[j + r * ldx] : T(0);
     }
@@ -423,8 +424,17 @@ __global__ void reduce_multi_kernel(const MVReduce *__restrict__ red, int32_t nr
     const MVReduce R = red[e];
     for (int row = threadIdx.x >> 5; row < R.nrows; row += blockDim.x >> 5) {
       T s = T(0);
-      for (int j = 0; j < R.npieces; j++)
-        s += P[(static_cast<int64_t>(R.p_row) + static_cast<int64_t>(j) * R.nrows + row) * W + lane];
+      const T *p = P + (static_cast<int64_t>(R.p_row) + row) * W + lane;
+      const int64_t step = static_cast<int64_t>(R.nrows) * W;
+      int j = 0;
+      for (; j + 8 <= R.npieces; j += 8) {  // eight loads in flight, added in order
+        T v[8];
+#pragma unroll
+        for (int i = 0; i < 8; i++) v[i] = p[(j + i) * step];
+#pragma unroll
+        for (int i = 0; i < 8; i++) s += v[i];
+      }
+      for (; j < R.npieces; j++) s += p[j * step];
       xt[static_cast<int64_t>(R.t_row + row) * W + lane] = s;
     }
   }

@@ -69,6 +69,7 @@
 #include <cuda_runtime.h>
 
 #include "hm_device.h"
+#include "hm_launch.cuh"
 
 namespace hm {
 
@@ -352,6 +353,8 @@ struct TcArgs {
   int32_t nr;
   int32_t zero_row;
   int32_t *status;
+  unsigned *xmax;              // near/U launch: the maxima of x, cleared for the next product (else NULL)
+  int32_t nxmax;
 };
 
 template <int R>
@@ -392,6 +395,10 @@ __global__ void __launch_bounds__(TcShape<R>::kThreads, 1) tc_kernel(const __gri
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  pdl_wait();  // XTS and the ticket are as the kernels before left them
+  pdl_trigger();
+  if (a.xmax && blockIdx.x == 0)
+    for (int e = threadIdx.x; e < a.nxmax; e += Sh::kThreads) a.xmax[e] = 0u;
 
   if (warp == 0) {
     // ---- item tickets, queued with the items for the other roles -------------
@@ -791,6 +798,8 @@ __global__ void xmax_kernel(const float *__restrict__ X, int64_t ldx, int nr, in
                             const int64_t *__restrict__ col0, int nmem, unsigned *__restrict__ xmax) {
   const int lane = threadIdx.x & 31;
   const int r = blockIdx.y * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  pdl_wait();  // x is there, the maxima are cleared
+  pdl_trigger();
   if (r >= nr) return;
   const int64_t j0 = blockIdx.x * static_cast<int64_t>(kXmaxSpan), j1 = min(n_src, j0 + kXmaxSpan);
   const float *xr = X + r * ldx;
@@ -812,49 +821,55 @@ __global__ void xmax_kernel(const float *__restrict__ X, int64_t ldx, int nr, in
   }
 }
 
-// sigma per member and right-hand side (sig) and its inverse (xs_inv), from
-// the maxima; right-hand sides past nr get 1.
-__global__ void sigma_kernel(const unsigned *__restrict__ xmax, int nmem, int nr, float *__restrict__ sig,
-                             float *__restrict__ xs_inv) {
-  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < nmem * kTcMaxRhs; e += gridDim.x * blockDim.x) {
-    const int r = e % kTcMaxRhs;
-    const float s = r < nr ? pow2_scale(__uint_as_float(xmax[e])) : 1.0f;
-    sig[e] = s;
-    xs_inv[e] = 1.0f / s;
-  }
-}
-
 // XTS x rows from X in its own order: the R right-hand sides X[j + r ldx]
-// (0 for r >= nr) of source index j, times sigma of (j's batch member, r),
-// split into FP16 hi (first 2R bytes) and lo (last 2R bytes), go to row
-// sinv[j]. Reads of X are coalesced along j and every row is written whole;
-// x-region rows that no source index maps to stay zero from the allocation.
-// Also re-arms the two item tickets.
+// (0 for r >= nr) of source index j, times sigma = pow2_scale(max |x_r|) of (j's batch
+// member, r), split into FP16 hi (first 2R bytes) and lo (last 2R bytes), go to row
+// sinv[j]. Reads of X are coalesced along j, all of a thread's at once, and every row is
+// written whole; x-region rows that no source index maps to stay zero from the allocation.
+// Also writes 1 / sigma per member and right-hand side, and re-arms the two item tickets.
 template <int R>
-__global__ void permute_split_kernel(const float *__restrict__ X, int64_t ldx, int nr,
-                                     const int32_t *__restrict__ sinv0, int64_t n_src,
-                                     uint16_t *__restrict__ xts, int32_t *__restrict__ tickets,
-                                     const int64_t *__restrict__ col0, int nmem, const float *__restrict__ sig) {
+__global__ void __launch_bounds__(256) permute_split_kernel(const float *__restrict__ X, int64_t ldx, int nr,
+                                                            const int32_t *__restrict__ sinv0, int64_t n_src,
+                                                            uint16_t *__restrict__ xts, int32_t *__restrict__ tickets,
+                                                            const int64_t *__restrict__ col0, int nmem,
+                                                            const unsigned *__restrict__ xmax,
+                                                            float *__restrict__ xs_inv) {
   __shared__ float tile[64][R + 1];
+  __shared__ float s0[R];  // sigma of the block's first member
   __shared__ int mem[64];
-  if (blockIdx.x == 0 && threadIdx.x < 2) tickets[threadIdx.x] = 0;  // V and near/U item tickets
+  const int tid = threadIdx.x;
+  pdl_wait();
+  pdl_trigger();
+  auto sigma = [&](int m, int r) { return r < nr ? pow2_scale(__uint_as_float(xmax[m * kTcMaxRhs + r])) : 1.0f; };
+  if (blockIdx.x == 0 && tid < 2) tickets[tid] = 0;  // V and near/U item tickets
+  for (int64_t e = blockIdx.x * 256ll + tid; e < static_cast<int64_t>(nmem) * kTcMaxRhs; e += gridDim.x * 256ll)
+    xs_inv[e] = 1.0f / sigma(static_cast<int>(e / kTcMaxRhs), static_cast<int>(e % kTcMaxRhs));
   for (int64_t j0 = blockIdx.x * 64ll; j0 < n_src; j0 += gridDim.x * 64ll) {
-    if (threadIdx.x < 64) mem[threadIdx.x] = member_of(col0, nmem, min(j0 + threadIdx.x, n_src - 1));
+    float v[R / 4];
+#pragma unroll
+    for (int i = 0; i < R / 4; i++) {  // consecutive threads: consecutive j
+      const int e = tid + i * 256, r = e / 64;
+      const int64_t j = j0 + e % 64;
+      v[i] = j < n_src && r < nr ? X[j + r * ldx] : 0.0f;
+    }
+    if (tid < 64) mem[tid] = member_of(col0, nmem, min(j0 + tid, n_src - 1));
+    if (tid >= 64 && tid - 64 < R) s0[tid - 64] = sigma(member_of(col0, nmem, j0), tid - 64);
     __syncthreads();
-    for (int e = threadIdx.x; e < 64 * R; e += blockDim.x) {
-      const int r = e / 64, jj = e % 64;  // consecutive threads: consecutive j
-      const int64_t j = j0 + jj;
-      tile[jj][r] = (j < n_src && r < nr) ? X[j + r * ldx] * __ldg(sig + mem[jj] * kTcMaxRhs + r) : 0.0f;
+#pragma unroll
+    for (int i = 0; i < R / 4; i++) {
+      const int e = tid + i * 256, r = e / 64, jj = e % 64;
+      tile[jj][r] = v[i] * (mem[jj] == mem[0] ? s0[r] : sigma(mem[jj], r));
     }
     __syncthreads();
-    for (int e = threadIdx.x; e < 64 * (R / 8); e += blockDim.x) {
-      const int jj = e / (R / 8), q = e % (R / 8);
-      if (j0 + jj < n_src) {
-        float v[8];
 #pragma unroll
-        for (int i = 0; i < 8; i++) v[i] = tile[jj][8 * q + i];
+    for (int i = 0; i < R / 32; i++) {
+      const int e = tid + i * 256, jj = e / (R / 8), q = e % (R / 8);
+      if (j0 + jj < n_src) {
+        float w[8];
+#pragma unroll
+        for (int z = 0; z < 8; z++) w[z] = tile[jj][8 * q + z];
         uint4 hi, lo;
-        split8(v, hi, lo);
+        split8(w, hi, lo);
         uint4 *dst = reinterpret_cast<uint4 *>(xts + static_cast<int64_t>(sinv0[j0 + jj]) * (2 * R));
         dst[q] = hi;
         dst[R / 8 + q] = lo;
@@ -871,6 +886,8 @@ template <int R>
 __global__ void reduce_split_kernel(const MVReduce *__restrict__ red, int32_t nred, const float *__restrict__ P,
                                     uint16_t *__restrict__ xts) {
   const int lane = threadIdx.x & 31;
+  pdl_wait();
+  pdl_trigger();
   for (int32_t e = static_cast<int32_t>(blockIdx.x); e < nred; e += gridDim.x) {
     const MVReduce D = red[e];
     for (int row = threadIdx.x >> 5; row < D.nrows; row += blockDim.x >> 5) {
@@ -878,8 +895,17 @@ __global__ void reduce_split_kernel(const MVReduce *__restrict__ red, int32_t nr
 #pragma unroll
       for (int c = lane; c < R; c += 32) {
         float s = 0.0f;
-        for (int j = 0; j < D.npieces; j++)
-          s += P[(static_cast<int64_t>(D.p_row) + static_cast<int64_t>(j) * D.nrows + row) * R + c];
+        const float *p = P + (static_cast<int64_t>(D.p_row) + row) * R + c;
+        const int64_t step = static_cast<int64_t>(D.nrows) * R;
+        int j = 0;
+        for (; j + 8 <= D.npieces; j += 8) {  // eight loads in flight, added in order
+          float v[8];
+#pragma unroll
+          for (int i = 0; i < 8; i++) v[i] = p[(j + i) * step];
+#pragma unroll
+          for (int i = 0; i < 8; i++) s += v[i];
+        }
+        for (; j < D.npieces; j++) s += p[j * step];
         const __half hb = __float2half_rn(s);
         const __half lb = __float2half_rn(s - __half2float(hb));
         dst[c] = *reinterpret_cast<const uint16_t *>(&hb);
@@ -1040,25 +1066,23 @@ cudaError_t encode_xts_map(DevTc &t, int R) {
 }
 
 template <int R>
-static int run_tc(const DevPlan &p, const DevTc &t, const float *X, int64_t ldx, int nr, float *Y, int64_t ldy,
-                  cudaStream_t s, cudaEvent_t *ev) {
+static cudaError_t run_tc(const DevPlan &p, const DevTc &t, const float *X, int64_t ldx, int nr, float *Y, int64_t ldy,
+                          cudaStream_t s, cudaEvent_t *ev, int *nl) {
   using Sh = TcShape<R>;
   uint16_t *xts = R == 64 ? t.xts64 : t.xts;
-  int nl = 0;
   int gp = static_cast<int>((p.n_src + 63) / 64);
   if (gp > 8192) gp = 8192;
   if (ev) cudaEventRecord(ev[0], s);
-  // per member and right-hand side: max |x| bits, sigma, 1 / sigma
+  // per member and right-hand side: max |x| bits (zero between products), 1 / sigma
   const int64_t nm64 = static_cast<int64_t>(t.nmem) * kTcMaxRhs;
   unsigned *xmax = reinterpret_cast<unsigned *>(t.xscale);
-  float *sig = t.xscale + nm64, *xs_inv = t.xscale + 2 * nm64;
-  cudaMemsetAsync(xmax, 0, nm64 * sizeof(unsigned), s);
+  float *xs_inv = t.xscale + nm64;
   const dim3 gx(static_cast<unsigned>((p.n_src + kXmaxSpan - 1) / kXmaxSpan), static_cast<unsigned>((nr + 7) / 8));
-  xmax_kernel<<<gx, 256, 0, s>>>(X, ldx, nr, p.n_src, t.mcol0, t.nmem, xmax);
-  sigma_kernel<<<static_cast<unsigned>((nm64 + 255) / 256), 256, 0, s>>>(xmax, t.nmem, nr, sig, xs_inv);
-  permute_split_kernel<R><<<gp, 256, 0, s>>>(X, ldx, nr, p.sinv0, p.n_src, xts, p.counter + 2, t.mcol0, t.nmem,
-                                              sig);
-  nl += 3;
+  cudaError_t e = launch_pdl(true, xmax_kernel, gx, 256, 0, s, X, ldx, nr, p.n_src, t.mcol0, t.nmem, xmax);
+  if (e == cudaSuccess)
+    e = launch_pdl(true, permute_split_kernel<R>, gp, 256, 0, s, X, ldx, nr, p.sinv0, p.n_src, xts, p.counter + 2,
+                   t.mcol0, t.nmem, xmax, xs_inv);
+  *nl = 2;
   if (ev) cudaEventRecord(ev[1], s);
   TcArgs a{};
   a.xmap = t.xmap[R / 64];
@@ -1077,16 +1101,17 @@ static int run_tc(const DevPlan &p, const DevTc &t, const float *X, int64_t ldx,
   a.zero_row = static_cast<int32_t>(p.zero_row);
   a.status = p.status;
   const size_t smem = smem_bytes<R>();
-  if (t.n_v > 0) {
+  if (e == cudaSuccess && t.n_v > 0) {
     a.items = t.v_items;
     a.nitems = t.n_v;
     a.grab = 8;  // V pieces are short: a few chunks each
     a.ticket = p.counter + 2;
-    tc_kernel<R><<<t.ctas, Sh::kThreads, smem, s>>>(a);
-    nl++;
-    if (t.n_reduce > 0) {
-      reduce_split_kernel<R><<<t.n_reduce < 4096 ? t.n_reduce : 4096, 256, 0, s>>>(t.reduce, t.n_reduce, t.prow, xts);
-      nl++;
+    e = launch_pdl(true, tc_kernel<R>, t.ctas, Sh::kThreads, smem, s, a);
+    ++*nl;
+    if (e == cudaSuccess && t.n_reduce > 0) {
+      e = launch_pdl(true, reduce_split_kernel<R>, t.n_reduce < 4096 ? t.n_reduce : 4096, 256, 0, s, t.reduce, t.n_reduce,
+                     t.prow, xts);
+      ++*nl;
     }
   }
   if (ev) cudaEventRecord(ev[2], s);
@@ -1094,10 +1119,13 @@ static int run_tc(const DevPlan &p, const DevTc &t, const float *X, int64_t ldx,
   a.nitems = t.n_du;
   a.grab = 1;  // row tiles are long; single tickets keep neighbouring tiles together
   a.ticket = p.counter + 3;
-  tc_kernel<R><<<t.ctas, Sh::kThreads, smem, s>>>(a);
-  nl++;
+  a.xmax = xmax;
+  a.nxmax = static_cast<int32_t>(nm64);
+  if (e == cudaSuccess) e = launch_pdl(true, tc_kernel<R>, t.ctas, Sh::kThreads, smem, s, a);
+  ++*nl;
   if (ev) cudaEventRecord(ev[3], s);
-  return nl;
+  if (e != cudaSuccess) cudaMemsetAsync(xmax, 0, nm64 * sizeof(unsigned), s);  // what the near/U launch would do
+  return e;
 }
 
 cudaError_t launch_tc_scales(const VGroup *groups, int64_t ngroups, const float *vdata, int64_t xt_rows,
@@ -1124,9 +1152,11 @@ cudaError_t launch_matvec_tc(const DevPlan &p, const DevTc &t, const float *X, i
   if (nr < 1 || nr > 64 || (nr > 32 && !t.xts64) || !t.xts || !t.xscale || !t.mcol0 || t.nmem < 1)
     return cudaErrorInvalidValue;
   tc_attrs();
-  const int nl = nr > 32 ? run_tc<64>(p, t, X, ldx, nr, Y, ldy, s, ev) : run_tc<32>(p, t, X, ldx, nr, Y, ldy, s, ev);
+  int nl = 0;
+  const cudaError_t e = nr > 32 ? run_tc<64>(p, t, X, ldx, nr, Y, ldy, s, ev, &nl)
+                                : run_tc<32>(p, t, X, ldx, nr, Y, ldy, s, ev, &nl);
   if (launches) *launches = nl;
-  return cudaGetLastError();
+  return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 }  // namespace hm
