@@ -135,8 +135,10 @@ int upload_plan(HMatrix &H, const std::vector<int32_t> &tmap0, const std::vector
   H.dp.status = H.dp.counter + 4;  // its own 16-byte slot of the same allocation
   H.dp.ntiles = static_cast<int32_t>(p.tiles.size());
   {  // rows of a tile in near-equal parts of at most 64, or 32 or 16 where that is
-    // what gives each SM four (the smallest parts re-read the XT rows most often)
-    const int64_t want = 4 * static_cast<int64_t>(H.num_sms);
+    // what gives each SM four (the smallest parts re-read the XT rows most often); in FP64,
+    // where a CTA fills an SM's FP64 pipe and reading is cheap beside it, eight, and down to 8 rows
+    const bool fp64 = H.opt.precision == HMGPU_F64;
+    const int64_t want = (fp64 ? 8 : 4) * static_cast<int64_t>(H.num_sms);
     std::vector<int64_t> map0(p.tiles.size());
     int64_t ncm = 0;
     for (size_t t = 0; t < map0.size(); t++) {
@@ -144,7 +146,7 @@ int upload_plan(HMatrix &H, const std::vector<int32_t> &tmap0, const std::vector
       ncm += p.tiles[t].ncols;
     }
     std::vector<MUnit> mu;
-    for (int32_t rows = 64; rows >= 16; rows /= 2) {
+    for (int32_t rows = 64; rows >= (fp64 ? 8 : 16); rows /= 2) {
       mu.clear();
       for (int32_t ti : p.tile_order) {
         const TileDesc &d = p.tiles[ti];

@@ -301,8 +301,8 @@ __device__ __forceinline__ void sum_warps(const S &acc, int m, unsigned char *sm
   constexpr int LD = W + 1;  // row stride of the sums: no bank conflicts either way
   // the sums of all rows at once where they fit the stages, else of half of them
   constexpr int PARTS = static_cast<size_t>(NW) * MT * LD * sizeof(T) <= multi_smem<T, W, NW>() ? 1 : 2;
-  constexpr int TRP = L::TR / PARTS, MP = MT / PARTS;
-  static_assert(L::TR % PARTS == 0 && static_cast<size_t>(NW) * MP * LD * sizeof(T) <= multi_smem<T, W, NW>(), "sums");
+  constexpr int TRP = (L::TR + PARTS - 1) / PARTS, MP = TRP * L::RG;
+  static_assert(static_cast<size_t>(NW) * MP * LD * sizeof(T) <= multi_smem<T, W, NW>(), "sums");
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int rg = lane / L::NG, ng = lane - rg * L::NG;
   T *red = reinterpret_cast<T *>(smem);
@@ -311,9 +311,10 @@ __device__ __forceinline__ void sum_warps(const S &acc, int m, unsigned char *sm
     __syncthreads();  // the stages (or the sums of the part before) are no longer read
 #pragma unroll
     for (int i = 0; i < TRP; i++)
+      if (part * TRP + i < L::TR)
 #pragma unroll
-      for (int j = 0; j < L::TN; j++)
-        red[(warp * MP + rg + i * L::RG) * LD + ng * L::TN + j] = acc.get(part * TRP + i, j);
+        for (int j = 0; j < L::TN; j++)
+          red[(warp * MP + rg + i * L::RG) * LD + ng * L::TN + j] = acc.get(part * TRP + i, j);
     __syncthreads();
     for (int o = tid; o < MP * W; o += NW * 32) {
       const int row = ROWS ? o % MP : o / W, q = ROWS ? o / MP : o % W;
@@ -326,29 +327,20 @@ __device__ __forceinline__ void sum_warps(const S &acc, int m, unsigned char *sm
   }
 }
 
-// Row count of the micro-kernel for a panel of m rows: the smallest form that holds them, in
-// smaller steps in FP64, where every row counts (a row test inside one 64-row form does
-// not help: the FP64 pipe is as busy with instructions that are predicated off).
-template <typename T, typename F>
+// Row count of the micro-kernel for a panel of m rows: the smallest form that holds them. In
+// FP64, where every row counts, there is one for each number of rows per lane (a row test
+// inside one 64-row form does not help: the FP64 pipe is as busy with instructions that
+// are predicated off); in FP32 four.
+template <typename T, int W, int MT = 64, typename F>
 __device__ __forceinline__ void with_rows(int m, F f) {
-  if (m > 48)
-    f(std::integral_constant<int, 64>());
-  else if (m > 32)
-    f(std::integral_constant<int, 48>());
-  else if (sizeof(T) == 4 && m > 16)
-    f(std::integral_constant<int, 32>());
-  else if (sizeof(T) == 4)
-    f(std::integral_constant<int, 16>());
-  else if constexpr (sizeof(T) == 8) {
-    if (m > 24)
-      f(std::integral_constant<int, 32>());
-    else if (m > 16)
-      f(std::integral_constant<int, 24>());
-    else if (m > 8)
-      f(std::integral_constant<int, 16>());
-    else
-      f(std::integral_constant<int, 8>());
+  constexpr int STEP = sizeof(T) == 8 ? LaneTile<T, W, 64>::RG : 16;
+  if constexpr (MT > STEP) {
+    if (m <= MT - STEP) {
+      with_rows<T, W, MT - STEP>(m, f);
+      return;
+    }
   }
+  f(std::integral_constant<int, MT>());
 }
 
 // V pass: for every multi-RHS V item
@@ -378,7 +370,7 @@ __global__ void __launch_bounds__(kVWarps * 32, multi_ctas<T, kVWarps>()) v_mult
       next = (big ? ctas : nbig + ctas * kVWarps) + atomicAdd(counter + kTicket[big ? 1 : 2], 1);
     const MVItem I = items[u];
     T *out = (I.kind == 0 ? xt : P) + static_cast<int64_t>(I.out) * W;
-    with_rows<T>(I.nrows, [&](auto mt) {
+    with_rows<T, W>(I.nrows, [&](auto mt) {
       using L = LaneTile<T, W, mt.value>;
       Sums<T, L::TR, L::TN> acc;
       slice_product<T, W, mt.value>(V + I.v_off, I.stride, I.nrows, I.ncols, big ? warp : 0, big ? kVWarps : 1, xt, buf,
@@ -502,7 +494,7 @@ __global__ void __launch_bounds__(kDuWarps * 32, multi_ctas<T, kDuWarps>()) du_m
     int32_t next = 0;
     if (tid == 0) next = static_cast<int32_t>(gridDim.x) + atomicAdd(a.counter + kTicket[0], 1);
     const int32_t *map = a.colmap + U.map;
-    with_rows<T>(U.m, [&](auto mt) {
+    with_rows<T, W>(U.m, [&](auto mt) {
       using L = LaneTile<T, W, mt.value>;
       Sums<T, L::TR, L::TN> acc;
       slice_product<T, W, mt.value>(a.panels + U.data_off, U.ld, U.m, U.ld, warp, kDuWarps, a.xt,
