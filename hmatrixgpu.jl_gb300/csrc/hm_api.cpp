@@ -547,28 +547,28 @@ extern "C" int hmgpu_matvec(hmgpu_hmatrix *h, const void *x, void *y, int64_t nr
   if (nrhs >= H.multi_from) {
     // several right-hand sides: one pass per rhs_per_pass() columns, the
     // matrix read once per pass (hm_multi.cu); for mixed precision one pass
-    // per 64 columns on the tensor cores (hm_tc.cu), 32 wide when at most 32
+    // per 64 columns on the tensor cores (hm_tc.cu), 16 or 32 wide when no more
     // columns remain
     const bool tc = H.opt.precision == HMGPU_MIXED;
     const int per = tc ? hm::kTcMaxRhs : hm::rhs_per_pass();
     int rc;
-    if (tc && !H.tc.xts) {
-      const int64_t xb = H.plan.xt_len * 2 * 32 * 2;
-      if ((rc = H.dalloc(reinterpret_cast<void **>(&H.tc.xts), xb)) ||
+    if (tc && !H.tc.prow) {
+      const size_t sb = 2 * static_cast<size_t>(H.tc.nmem) * hm::kTcMaxRhs * sizeof(float);
+      if ((rc = H.dalloc(reinterpret_cast<void **>(&H.tc.xscale), sb)) ||
           (rc = H.dalloc(reinterpret_cast<void **>(&H.tc.prow),
-                         std::max<int64_t>(H.plan.p_rows, 1) * hm::kTcMaxRhs * 4)) ||
-          (rc = H.dalloc(reinterpret_cast<void **>(&H.tc.xscale),
-                         2 * static_cast<size_t>(H.tc.nmem) * hm::kTcMaxRhs * sizeof(float))))
+                         std::max<int64_t>(H.plan.p_rows, 1) * hm::kTcMaxRhs * 4)))
         return rc;
-      cudaMemsetAsync(H.tc.xts, 0, xb, s);
-      cudaMemsetAsync(H.tc.xscale, 0, 2 * static_cast<size_t>(H.tc.nmem) * hm::kTcMaxRhs * sizeof(float), s);
-      if (cudaError_t e = hm::encode_xts_map(H.tc, 32)) return hm::cuda_fail(e, "tensor map of XTS");
+      cudaMemsetAsync(H.tc.xscale, 0, sb, s);
     }
-    if (tc && nrhs > 32 && !H.tc.xts64) {
-      const int64_t xb = H.plan.xt_len * 2 * 64 * 2;
-      if ((rc = H.dalloc(reinterpret_cast<void **>(&H.tc.xts64), xb))) return rc;
-      cudaMemsetAsync(H.tc.xts64, 0, xb, s);
-      if (cudaError_t e = hm::encode_xts_map(H.tc, 64)) return hm::cuda_fail(e, "tensor map of XTS");
+    // the XTS of every width that this call's passes have
+    for (int64_t left = nrhs; tc && left > 0; left -= std::min<int64_t>(left, per)) {
+      const int w = hm::tc_width(static_cast<int>(std::min<int64_t>(left, per)));
+      uint16_t *&xts = H.tc.xts[w / 32];
+      if (xts) continue;
+      const int64_t xb = H.plan.xt_len * 2 * w * 2;
+      if ((rc = H.dalloc(reinterpret_cast<void **>(&xts), xb))) return rc;
+      cudaMemsetAsync(xts, 0, xb, s);
+      if (cudaError_t e = hm::encode_xts_map(H.tc, w)) return hm::cuda_fail(e, "tensor map of XTS");
     }
     if (!tc && !H.xt_multi) {
       std::vector<int64_t> col0(H.plan.tiles.size());

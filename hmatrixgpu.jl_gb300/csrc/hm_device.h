@@ -81,7 +81,7 @@ int rhs_per_pass();
 int multi_width(bool f64, int nr);
 // Columns of the next pass when `left` remain, of a matrix with that many stored entries.
 int multi_pass_columns(bool f64, int64_t left, int64_t entries, int num_sms);
-// Mixed-precision tensor-core product (hm_tc.cu), 32 or 64 right-hand sides
+// Mixed-precision tensor-core product (hm_tc.cu), 16, 32 or 64 right-hand sides
 // per pass.
 struct TcPack {  // one item's FP32 row-major source -> canonical FP16 chunks and row factors
   int64_t src_off, a_off;
@@ -97,20 +97,20 @@ struct DevTc {
   TcItem *v_items = nullptr, *du_items = nullptr;
   int32_t *colmap = nullptr;
   MVReduce *reduce = nullptr;
-  uint16_t *xts = nullptr;    // xt_len rows of 32 FP16 hi + 32 FP16 lo (passes of <= 32 columns)
-  uint16_t *xts64 = nullptr;  // xt_len rows of 64 FP16 hi + 64 FP16 lo (passes of 33..64 columns)
+  // xt_len rows of R FP16 hi + R FP16 lo at [R / 32]: passes R = 16, 32 and 64 wide
+  uint16_t *xts[3] = {nullptr, nullptr, nullptr};
   float *prow = nullptr;      // partial rows of split V items, 64 values per row
   float *xscale = nullptr;    // per member: max |x_r| bits (zero between products), 1 / sigma_r (64 words each)
   int64_t *mcol0 = nullptr;   // first source index of each batch member, nmem + 1 entries
   int32_t nmem = 1;           // batch members (1 outside batches)
   int32_t n_v = 0, n_du = 0, n_reduce = 0, ctas = 0;
-  int64_t xt_rows = 0;  // rows of either XTS
-  CUtensorMap xmap[4];  // tile-load maps of xts and xts64: 64-row boxes, then 8-row boxes (encode_xts_map)
+  int64_t xt_rows = 0;  // rows of each XTS
+  CUtensorMap xmap[6];  // tile-load maps of the three XTS: 64-row boxes, then 8-row boxes (encode_xts_map)
 };
 constexpr int kTcMaxRhs = 64;  // right-hand sides of the widest pass
-size_t tc_smem_bytes(int nr);
-// The tile-load map of the XTS of width R (32: xts, 64: xts64), after the
-// buffer exists.
+// Width (16, 32 or 64) of a pass over nr columns.
+int tc_width(int nr);
+// The tile-load maps of the XTS of width R, after the buffer exists.
 cudaError_t encode_xts_map(DevTc &t, int R);
 // Scales of the rank rows from the FP32 V rows of every source group: nu
 // (max magnitude into [2^14, 2^15)), gam (2^-ceil(log2 of the row's 1-norm))
@@ -120,7 +120,7 @@ cudaError_t launch_tc_scales(const VGroup *groups, int64_t ngroups, const float 
 cudaError_t launch_pack_tc(const TcPack *jobs, int64_t njobs, const float *src, void *adata, const int32_t *colmap,
                            const float *colsc, const float *nu, const float *gam, cudaStream_t s);
 // permutation + split of X, V pass, reduction of pieces, near/U pass over
-// nr <= 64 columns (xts64 must exist for nr > 32); ev (optional) gets 4
+// nr <= 64 columns (the XTS of their width must exist); ev (optional) gets 4
 // events as launch_matvec_multi.
 cudaError_t launch_matvec_tc(const DevPlan &p, const DevTc &t, const float *X, int64_t ldx, int nr,
                              float *Y, int64_t ldy, cudaStream_t s, cudaEvent_t *ev, int *launches);

@@ -23,7 +23,7 @@
 //
 // Pipelines (one persistent CTA per SM; items from a ticket counter, in list
 // order, so concurrent CTAs work on neighbouring panels and share XTS rows in
-// L2; warp 0 takes the tickets and queues them for the other roles). A 32-wide
+// L2; warp 0 takes the tickets and queues them for the other roles). A 16- or 32-wide
 // pass runs two pipelines, item n in pipeline n & 1; they share the tensor
 // cores but have their own stages, producers, MMA warp and epilogue set,
 // because one MMA warp's own instructions per chunk bound a pipeline. A
@@ -43,7 +43,7 @@
 //               source clusters and rank ranges), 16-byte cp.async gathers
 //               for the other groups (padding columns read the zero row),
 //               then a wait, a proxy fence and an mbarrier arrive;
-//   MMA         warp 2 (pipeline 0) and, in a 32-wide pass, the last warp
+//   MMA         warp 2 (pipeline 0) and, with two pipelines, the last warp
 //               (pipeline 1); one elected lane each: per 16 columns one UMMA,
 //               [A_hi; A_lo] x [B_hi B_lo] with M = 128, N = 2R (hi and lo
 //               stacked along both M and N; items have at most 64 rows), into
@@ -97,19 +97,22 @@ constexpr int kSegChunksV = HM_TC_SEG_CHUNKS_V;
 // columns TcShape<R>::kBGroupK bytes apart.
 constexpr uint32_t kBGroupN = 128;
 
-// The shape of a pass over R = 32 or 64 right-hand sides. A 64-wide pass reads
+// The shape of a pass over R = 16, 32 or 64 right-hand sides. A 64-wide pass reads
 // every tile once for twice the columns; its B tiles are twice as large, so
-// the ring has 6 stages instead of 8.
+// the ring has 6 stages instead of 8. A 16-wide pass gathers half the XTS bytes of a
+// 32-wide one, and its smaller B tiles leave room for 10 stages: 32,768-point cube at 1e-6,
+// up to 16 columns, 482 us per product against 578 of the 32-wide pass; film 500,500 1108
+// against 1309.
 template <int R>
 struct TcShape {
-  static_assert(R == 32 || R == 64, "32 or 64 right-hand sides per pass");
+  static_assert(R == 16 || R == 32 || R == 64, "16, 32 or 64 right-hand sides per pass");
   static constexpr int kBN = 2 * R;                   // B rows: R hi, then R lo
   static constexpr int kBBytes = kBN * kKc * 2;       // one FP16 B tile: 8 or 16 KB
-  static constexpr int kStages = R == 32 ? 8 : 6;
-  // Two pipelines for 32 right-hand sides. A 64-wide pass keeps one: a 17th
+  static constexpr int kStages = R == 16 ? 10 : R == 32 ? 8 : 6;
+  // Two pipelines for 16 and 32 right-hand sides. A 64-wide pass keeps one: a 17th
   // warp would cap every thread at 96 registers (warps per scheduler x
   // threads x registers), and its epilogue needs more for 64 sums a row.
-  static constexpr int kPipes = R == 32 ? 2 : 1;
+  static constexpr int kPipes = R <= 32 ? 2 : 1;
   static constexpr int kPipeStages = kStages / kPipes;  // stages of each pipeline
   static constexpr int kBProducers = kStages;           // warps 1, 3, 8 .. 5 + kStages
   static constexpr int kEpi1 = 6 + kBProducers;         // first warp of the second epilogue set
@@ -224,7 +227,7 @@ struct TcSmem {
 // operand layouts need 128-byte alignment at most); 232448 bytes is the
 // per-block limit
 constexpr size_t kSmemAlign = 128;
-static_assert(sizeof(TcSmem<32>) + kSmemAlign <= 232448 && sizeof(TcSmem<64>) + kSmemAlign <= 232448,
+static_assert(sizeof(TcSmem<16>) + kSmemAlign <= 232448 && sizeof(TcSmem<32>) + kSmemAlign <= 232448 && sizeof(TcSmem<64>) + kSmemAlign <= 232448,
               "tensor-core pass shared memory");
 
 // Waits for the phase of `bar` with parity `parity`; false when the abort flag
@@ -862,9 +865,9 @@ __global__ void __launch_bounds__(256) permute_split_kernel(const float *__restr
     }
     __syncthreads();
 #pragma unroll
-    for (int i = 0; i < R / 32; i++) {
+    for (int i = 0; i < (R + 31) / 32; i++) {
       const int e = tid + i * 256, jj = e / (R / 8), q = e % (R / 8);
-      if (j0 + jj < n_src) {
+      if (jj < 64 && j0 + jj < n_src) {
         float w[8];
 #pragma unroll
         for (int z = 0; z < 8; z++) w[z] = tile[jj][8 * q + z];
@@ -1027,11 +1030,12 @@ template <int R>
 static size_t smem_bytes() {
   return sizeof(TcSmem<R>) + kSmemAlign;
 }
-size_t tc_smem_bytes(int nr) { return nr > 32 ? smem_bytes<64>() : smem_bytes<32>(); }
+int tc_width(int nr) { return nr <= 16 ? 16 : nr <= 32 ? 32 : 64; }
 
 static void tc_attrs() {
   static bool done = false;
   if (done) return;
+  cudaFuncSetAttribute(tc_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem_bytes<16>()));
   cudaFuncSetAttribute(tc_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem_bytes<32>()));
   cudaFuncSetAttribute(tc_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem_bytes<64>()));
   done = true;
@@ -1048,8 +1052,9 @@ cudaError_t encode_xts_map(DevTc &t, int R) {
       f = nullptr;
     return reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(f);
   }();
-  uint16_t *xts = R == 64 ? t.xts64 : t.xts;
-  if (!enc || !xts || t.xt_rows < 8 || (R != 32 && R != 64)) return cudaErrorInvalidValue;
+  if (R != 16 && R != 32 && R != 64) return cudaErrorInvalidValue;
+  uint16_t *xts = t.xts[R / 32];
+  if (!enc || !xts || t.xt_rows < 8) return cudaErrorInvalidValue;
   // element (e, row, g) = XTS[row][8 g + e]: a box of 8 x 64 x 2R/8 lands as
   // 2R/8 N groups of 64 rows x 16 bytes
   cuuint64_t dims[3] = {8, static_cast<cuuint64_t>(t.xt_rows), static_cast<cuuint64_t>(2 * R / 8)};
@@ -1057,7 +1062,7 @@ cudaError_t encode_xts_map(DevTc &t, int R) {
   for (int b = 0; b < 2; b++) {  // boxes of 64 rows (V pieces) and of 8 rows (K groups of near/U tiles)
     cuuint32_t box[3] = {8, b == 0 ? 64u : 8u, static_cast<cuuint32_t>(2 * R / 8)};
     cuuint32_t es[3] = {1, 1, 1};
-    const CUresult r = enc(&t.xmap[2 * b + R / 64], CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, xts, dims, strides, box, es,
+    const CUresult r = enc(&t.xmap[3 * b + R / 32], CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, xts, dims, strides, box, es,
                            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE,
                            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return cudaErrorInvalidValue;
@@ -1069,7 +1074,7 @@ template <int R>
 static cudaError_t run_tc(const DevPlan &p, const DevTc &t, const float *X, int64_t ldx, int nr, float *Y, int64_t ldy,
                           cudaStream_t s, cudaEvent_t *ev, int *nl) {
   using Sh = TcShape<R>;
-  uint16_t *xts = R == 64 ? t.xts64 : t.xts;
+  uint16_t *xts = t.xts[R / 32];
   int gp = static_cast<int>((p.n_src + 63) / 64);
   if (gp > 8192) gp = 8192;
   if (ev) cudaEventRecord(ev[0], s);
@@ -1085,8 +1090,8 @@ static cudaError_t run_tc(const DevPlan &p, const DevTc &t, const float *X, int6
   *nl = 2;
   if (ev) cudaEventRecord(ev[1], s);
   TcArgs a{};
-  a.xmap = t.xmap[R / 64];
-  a.xmap8 = t.xmap[2 + R / 64];
+  a.xmap = t.xmap[R / 32];
+  a.xmap8 = t.xmap[3 + R / 32];
   a.adata = static_cast<const unsigned char *>(t.adata);
   a.colmap = t.colmap;
   a.xts = xts;
@@ -1149,12 +1154,14 @@ cudaError_t launch_pack_tc(const TcPack *jobs, int64_t njobs, const float *src, 
 
 cudaError_t launch_matvec_tc(const DevPlan &p, const DevTc &t, const float *X, int64_t ldx, int nr,
                              float *Y, int64_t ldy, cudaStream_t s, cudaEvent_t *ev, int *launches) {
-  if (nr < 1 || nr > 64 || (nr > 32 && !t.xts64) || !t.xts || !t.xscale || !t.mcol0 || t.nmem < 1)
+  if (nr < 1 || nr > 64 || !t.xts[tc_width(nr) / 32] || !t.xscale || !t.mcol0 || t.nmem < 1)
     return cudaErrorInvalidValue;
   tc_attrs();
   int nl = 0;
-  const cudaError_t e = nr > 32 ? run_tc<64>(p, t, X, ldx, nr, Y, ldy, s, ev, &nl)
-                                : run_tc<32>(p, t, X, ldx, nr, Y, ldy, s, ev, &nl);
+  const int w = tc_width(nr);
+  const cudaError_t e = w == 64   ? run_tc<64>(p, t, X, ldx, nr, Y, ldy, s, ev, &nl)
+                        : w == 32 ? run_tc<32>(p, t, X, ldx, nr, Y, ldy, s, ev, &nl)
+                                  : run_tc<16>(p, t, X, ldx, nr, Y, ldy, s, ev, &nl);
   if (launches) *launches = nl;
   return e != cudaSuccess ? e : cudaGetLastError();
 }
