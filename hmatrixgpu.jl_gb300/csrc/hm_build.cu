@@ -19,6 +19,7 @@
 
 #include "hm_api.h"
 #include "hm_entry.cuh"
+#include "hm_launch.cuh"
 #include "hm_user.h"
 
 namespace hm {
@@ -144,24 +145,36 @@ __global__ void __launch_bounds__(kBuildThreads) qr_kernel(const AcaJob *__restr
 // are one sweep, in which every column sees the rotations it would see one by
 // one, bit for bit. k rounds in a row without a rotation have looked at every
 // pair of the same M (the first and the last k rounds look at part of them),
-// which is the sweep without a rotation that ends the sequential loop. The columns' squared norms are kept from one rotation to the
-// next (the same sums of the same values).
+// which is the sweep without a rotation that ends the sequential loop. The columns'
+// squared norms are kept from one rotation to the next (the same sums of the same values).
 //
 // Bound by the FP64 pipe, whose rate does not depend on how many lanes of a warp
 // are active: a group of k / 2 lanes takes a block, as many groups of the same
-// k as fit share a warp, M and Z lie in shared memory (columns an odd number of
-// doubles apart: no bank conflicts between lanes). Blocks of more than
+// k as fit share a CTA of three warps, M and Z lie in shared memory (columns an odd
+// number of doubles apart: no bank conflicts between lanes). Blocks of more than
 // kJacGroupMax terms get a CTA. Measured against one thread per block on M and Z in
 // global memory, whole assemblies: 32,768-point cube at tol 1e-6 722 -> 507 ms,
 // film 262,144 at 1e-4 266 -> 250 ms, 216 cells with the demagnetising tensor
-// (cores of over 100 terms) 1062 -> 57 ms.
+// (cores of over 100 terms) 1062 -> 57 ms. Three warps share the lanes that a block of odd
+// size leaves over, and nine overlapping launches by size fit more of them on an SM: of the
+// cube's assembly, then at 400 ms, one warp 392, two 378, three 369; two warps in three
+// launches that follow one another 394 (demagnetising tensor 52 -> 40). The pipe is at 80 % of
+// its rate in the large launches, 21 of 32 lanes active (pairs that need no rotation idle).
 // ---------------------------------------------------------------------------
 constexpr int kJacGroupMax = 64;   // terms of the largest block that a group of lanes takes
+constexpr int kJacThreads = 96;    // threads per CTA of the group form
 constexpr int kJacSweeps = 80;
 constexpr int kJacBins = kJacGroupMax + 2;  // bin k: blocks of k terms; the last: larger ones
 constexpr int kJacPairs = 512;     // pairs per step of the CTA form
-// words of the bin table: per bin its first id and its first warp, then four tickets
-constexpr int kJacTable = 2 * kJacBins + 4;
+// Largest k of each launch of the group form. A launch's CTAs ask for the shared memory of its
+// largest blocks, and the warps that fit an SM are few (6 at k = 32, 10 at 22).
+constexpr int kJacClasses = 9;
+__host__ __device__ constexpr int jac_class_max(int c) {
+  constexpr int hi[kJacClasses + 1] = {kJacGroupMax, 48, 40, 32, 28, 24, 20, 16, 8, 0};
+  return hi[c];
+}
+// words of the bin table: per bin its first id and its first CTA, then a ticket per launch
+constexpr int kJacTable = 2 * kJacBins + 1 + kJacClasses;
 
 // Pair l of round c (c = p + q mod k, l < k / 2); head: p + q = c, else p + q = c + k.
 __device__ __forceinline__ bool jac_pair(int c, int k, int l, int &p, int &q, bool &head) {
@@ -216,7 +229,7 @@ __device__ void jac_finish(const WS &w, int k, double eps, bool converged, AcaRe
 }
 
 // Sorts the blocks by their number of terms (largest first; one CTA) and counts
-// the warps that each bin's groups fill. Blocks that need no SVD get r = k here.
+// the CTAs that each bin's groups fill. Blocks that need no SVD get r = k here.
 __global__ void __launch_bounds__(1024) jacobi_bins_kernel(int32_t njobs, int svd, AcaRes *res, int32_t *table,
                                                            int32_t *ids) {
   __shared__ int32_t count[kJacBins], at[kJacBins];
@@ -237,49 +250,54 @@ __global__ void __launch_bounds__(1024) jacobi_bins_kernel(int32_t njobs, int sv
       at[b] = table[b] = first;
       first += count[b];
     }
-    // first warp of each bin, counted from the largest bin of its launch
-    int32_t *warp0 = table + kJacBins;
+    // first CTA of each bin, counted from the largest bin of its launch
+    int32_t *cta0 = table + kJacBins;
     int w = 0;
-    for (int b = kJacGroupMax; b >= 1; b--) {
-      if (b == 32 || b == 16) w = 0;  // the launches take bins 33-64, 17-32 and 1-16
-      warp0[b] = w;
-      const int groups = 32 / max(1, b / 2);
+    for (int b = kJacGroupMax, c = 0; b >= 1; b--) {
+      if (b == jac_class_max(c)) w = 0, c++;
+      cta0[b] = w;
+      const int groups = kJacThreads / max(1, b / 2);
       w += (count[b] + groups - 1) / groups;
     }
-    for (int q = 0; q < 4; q++) table[2 * kJacBins + q] = 0;
+    for (int q = 2 * kJacBins; q < kJacTable; q++) table[q] = 0;
   }
   __syncthreads();
   for (int j = threadIdx.x; j < njobs; j += blockDim.x) ids[atomicAdd(&at[bin_of(res[j])], 1)] = j;
 }
 
-// Blocks of klo <= k <= khi terms, a group of k / 2 lanes each. CTAs of one warp.
-__global__ void __launch_bounds__(32) jacobi_group_kernel(const AcaJob *__restrict__ jobs, int klo, int khi,
-                                                          double eps, double *ws, AcaRes *res, int32_t *table,
-                                                          const int32_t *__restrict__ ids, int32_t *ticket) {
+// Blocks of klo <= k <= khi terms, a group of k / 2 lanes each; the groups of a CTA have
+// the same k.
+__global__ void __launch_bounds__(kJacThreads) jacobi_group_kernel(const AcaJob *__restrict__ jobs, int klo, int khi,
+                                                                   double eps, double *ws, AcaRes *res,
+                                                                   int32_t *table, const int32_t *__restrict__ ids,
+                                                                   int32_t *ticket) {
   extern __shared__ __align__(16) double jac_smem[];
-  const int lane = threadIdx.x;
-  const int32_t *first = table, *warp0 = table + kJacBins;
+  __shared__ int s_ticket;
+  __shared__ int s_rot[2][kJacThreads];  // rounds by parity: bit 0 a rotation in the group, bit 1 in the last sweep
+  pdl_trigger();
+  const int tid = threadIdx.x;
+  const int32_t *first = table, *cta0 = table + kJacBins;
   for (;;) {
-    int wi = 0;
-    if (lane == 0) wi = atomicAdd(ticket, 1);
-    wi = __shfl_sync(0xffffffffu, wi, 0);
-    int k = klo;  // the bin of warp wi: the smallest k with warp0[k] <= wi
+    if (tid == 0) s_ticket = atomicAdd(ticket, 1);
+    s_rot[0][tid] = s_rot[1][tid] = 0;
+    __syncthreads();
+    const int wi = s_ticket;
+    int k = klo;  // the bin of CTA wi: the smallest k with cta0[k] <= wi
     {
       int hi = khi;
       while (k < hi) {
         const int mid = (k + hi) / 2;
-        if (warp0[mid] <= wi)
+        if (cta0[mid] <= wi)
           hi = mid;
         else
           k = mid + 1;
       }
     }
-    const int gw = max(1, k / 2), groups = 32 / gw;
-    const int at0 = first[k] + (wi - warp0[k]) * groups, end = first[k - 1];
-    if (at0 >= end) return;  // past the last warp of the smallest bin
-    const int grp = lane / gw, l = lane - grp * gw;
+    const int gw = max(1, k / 2), groups = kJacThreads / gw;
+    const int at0 = first[k] + (wi - cta0[k]) * groups, end = first[k - 1];
+    if (at0 >= end) break;  // past the last CTA of the smallest bin
+    const int grp = tid / gw, l = tid - grp * gw;
     const bool mine = grp < groups && at0 + grp < end;
-    const unsigned gmask = (gw == 32 ? 0xffffffffu : ((1u << gw) - 1u)) << (mine ? grp * gw : 0);
     const int ld = k | 1;
     const int job = mine ? ids[at0 + grp] : 0;
     double *M = jac_smem + static_cast<int64_t>(grp) * (2 * k * ld + k), *Z = M + k * ld, *norm = Z + k * ld;
@@ -292,18 +310,18 @@ __global__ void __launch_bounds__(32) jacobi_group_kernel(const AcaJob *__restri
         Z[e % k + (e / k) * ld] = w.Z[e];
       }
     }
-    __syncwarp();
+    __syncthreads();
     if (mine)
       for (int j = l; j < k; j += gw) {
         double s = 0.0;
         for (int i = 0; i < k; i++) s = dadd(s, dmul(M[i + j * ld], M[i + j * ld]));
         norm[j] = s;
       }
-    __syncwarp();
+    __syncthreads();
     int quiet = 0, last_rot = 0;  // rounds without a rotation; a rotation in the last sweep
     bool done = !mine;
-    for (int c = 0, sweep = 0;;) {
-      bool rot = false, last = false;
+    for (int c = 0, sweep = 0, par = 0;; par ^= 1) {
+      int rot = 0;
       if (!done) {
         int p, q;
         bool head;
@@ -315,8 +333,7 @@ __global__ void __launch_bounds__(32) jacobi_group_kernel(const AcaJob *__restri
             for (int i = 0; i < k; i++) g = dadd(g, dmul(mp[i], mq[i]));
             double cs, sn;
             if (jac_rotation(norm[p], norm[q], g, cs, sn)) {
-              rot = true;
-              last = t == kJacSweeps - 1;
+              rot = t == kJacSweeps - 1 ? 3 : 1;
               double *zp = Z + p * ld, *zq = Z + q * ld;
               double a = 0.0, b = 0.0;
               for (int i = 0; i < k; i++) {
@@ -335,16 +352,18 @@ __global__ void __launch_bounds__(32) jacobi_group_kernel(const AcaJob *__restri
           }
         }
       }
-      const unsigned rb = __ballot_sync(0xffffffffu, rot), lb = __ballot_sync(0xffffffffu, last);
-      __syncwarp();  // this round's columns are read by others in the next
-      quiet = (rb & gmask) || sweep == 0 || sweep == kJacSweeps ? 0 : quiet + 1;
-      last_rot |= (lb & gmask) != 0;
+      if (rot) atomicOr(&s_rot[par][grp], rot);
+      __syncthreads();  // the round's flags are set; its columns are read by others in the next
+      const int flags = mine ? s_rot[par][grp] : 0;
+      s_rot[par ^ 1][tid] = 0;  // (the next round's: read by all before the barrier above)
+      quiet = (flags & 1) || sweep == 0 || sweep == kJacSweeps ? 0 : quiet + 1;
+      last_rot |= flags & 2;
       if (++c == k) {
         c = 0;
         sweep++;
       }
       done = done || quiet >= k || sweep > kJacSweeps;
-      if (__all_sync(0xffffffffu, done)) break;
+      if (__syncthreads_and(done)) break;
     }
     if (mine) {
       for (int e = l; e < k * k; e += gw) {
@@ -356,8 +375,9 @@ __global__ void __launch_bounds__(32) jacobi_group_kernel(const AcaJob *__restri
         jac_finish(w, k, eps, quiet >= k || !last_rot, res + job);
       }
     }
-    __syncwarp();  // the shared memory goes to the next blocks
+    __syncthreads();  // the shared memory goes to the next blocks
   }
+  if (blockIdx.x == 0) pdl_wait();  // the grid ends after the one before it
 }
 
 // Blocks of more than kJacGroupMax terms, a CTA each: the products and norms of a
@@ -371,6 +391,7 @@ __global__ void __launch_bounds__(kBuildThreads) jacobi_cta_kernel(const AcaJob 
   __shared__ double pg[kJacPairs], pc[kJacPairs], ps[kJacPairs];
   __shared__ int s_ticket;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  pdl_trigger();
   const int n = table[kJacBins - 2];  // bin kJacBins - 1 comes first
   for (;;) {
     if (tid == 0) s_ticket = atomicAdd(ticket, 1);
@@ -656,23 +677,29 @@ static cudaError_t launch_jacobi(const AcaJob *jobs, int32_t njobs, double eps, 
   e = cudaFuncSetAttribute(jacobi_cta_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(cap * 8));
   if (e != cudaSuccess) return e;
   jacobi_cta_kernel<<<sms, kBuildThreads, cap * 8>>>(jobs, eps, cap, ws, res, table, ids, ticket);
-  // group launches by size, so that small blocks do not pay for the shared
-  // memory of large ones (a warp's groups of k terms hold 2 k (k | 1) + k doubles each)
-  const int hi[3] = {kJacGroupMax, 32, 16}, lo[3] = {33, 17, 1};
-  int64_t words[3] = {0, 0, 0};
-  for (int c = 0; c < 3; c++)
-    for (int k = lo[c]; k <= hi[c]; k++)
-      words[c] = std::max<int64_t>(words[c], static_cast<int64_t>(32 / std::max(1, k / 2)) * (2 * k * (k | 1) + k));
+  // The group launches read nothing of one another, nor of the kernel above: each may start as
+  // soon as the CTAs of the one before have started, and takes the SMs as they fall idle.
+  auto words = [](int c) {  // a CTA's groups of k terms hold 2 k (k | 1) + k doubles each
+    int64_t w = 0;
+    for (int k = jac_class_max(c + 1) + 1; k <= jac_class_max(c); k++)
+      w = std::max<int64_t>(w, static_cast<int64_t>(kJacThreads / std::max(1, k / 2)) * (2 * k * (k | 1) + k));
+    return w;
+  };
+  int64_t most_words = 0;
+  for (int c = 0; c < kJacClasses; c++) most_words = std::max(most_words, words(c));
   e = cudaFuncSetAttribute(jacobi_group_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           static_cast<int>(words[0] * 8));
-  if (e != cudaSuccess) return e;
-  for (int c = 0; c < 3; c++) {
+                           static_cast<int>(most_words * 8));
+  if (e == cudaSuccess)  // one split of the SM's memory for all of them
+    e = cudaFuncSetAttribute(jacobi_group_kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
+                             cudaSharedmemCarveoutMaxShared);
+  for (int c = 0; c < kJacClasses && e == cudaSuccess; c++) {
     int occ = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, jacobi_group_kernel, 32, words[c] * 8);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, jacobi_group_kernel, kJacThreads, words(c) * 8);
     const int64_t grid = std::min<int64_t>(static_cast<int64_t>(sms) * std::max(1, occ), njobs);
-    jacobi_group_kernel<<<static_cast<unsigned>(grid), 32, words[c] * 8>>>(jobs, lo[c], hi[c], eps, ws, res, table,
-                                                                        ids, ticket + 1 + c);
+    e = launch_pdl(true, jacobi_group_kernel, dim3(static_cast<unsigned>(grid)), kJacThreads, words(c) * 8, nullptr,
+                   jobs, jac_class_max(c + 1) + 1, jac_class_max(c), eps, ws, res, table, ids, ticket + 1 + c);
   }
+  if (e != cudaSuccess) return e;
   return cudaGetLastError();
 }
 

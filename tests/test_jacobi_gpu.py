@@ -9,7 +9,7 @@ from oracle import oracle as O
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("k", [1, 2, 3, 16, 17, 32, 33, 63, 64, 65, 100, 131, 170])
+@pytest.mark.parametrize("k", [1, 2, 3, 8, 9, 16, 17, 20, 21, 24, 25, 28, 29, 32, 33, 40, 41, 48, 49, 63, 64, 65, 100, 131, 170])
 @pytest.mark.parametrize("decay", [0.0, 8.0])
 def test_svd_recompress_core_sizes(gpu, k, decay):
     """Every factor bitwise the oracle's, whose sweep visits the pairs one by one."""
