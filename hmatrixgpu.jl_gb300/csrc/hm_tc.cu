@@ -26,7 +26,8 @@
 // L2; warp 0 takes the tickets and queues them for the other roles). A 16- or 32-wide
 // pass runs two pipelines, item n in pipeline n & 1; they share the tensor
 // cores but have their own stages, producers, MMA warp and epilogue set,
-// because one MMA warp's own instructions per chunk bound a pipeline. A
+// because one MMA warp's own instructions per chunk bound a pipeline; each item is queued
+// for the warps of its pipeline alone. A
 // 64-wide pass runs one (every item in pipeline 0), whose epilogue sets still
 // take every other item:
 //   warp 0      item tickets (lane 0), queued in shared memory for the others;
@@ -47,8 +48,8 @@
 //               (pipeline 1); one elected lane each: per 16 columns one UMMA,
 //               [A_hi; A_lo] x [B_hi B_lo] with M = 128, N = 2R (hi and lo
 //               stacked along both M and N; items have at most 64 rows), into
-//               a fresh TMEM accumulator buffer (FP32) every kSegChunks
-//               chunks; commits free the stage and hand each buffer to the
+//               a fresh TMEM accumulator buffer (FP32) every
+//               chunk; commits free the stage and hand each buffer to the
 //               item's epilogue set. In a V piece's last chunk it first
 //               zeroes the B rows of padding columns (other blocks' XTS rows,
 //               which the 64-row tile load brought in: 0 * Inf must not reach
@@ -78,24 +79,12 @@ namespace {
 constexpr int kKc = 64;                // columns per chunk
 constexpr int kABytes = 128 * kKc * 2;  // A tile: 64 hi rows, then 64 lo rows: 16 KB
 constexpr int kQ = 16;                  // item queue slots
-#ifndef HM_TC_SEG_CHUNKS
-#define HM_TC_SEG_CHUNKS 1
-#endif
-#ifndef HM_TC_SEG_CHUNKS_V
-#define HM_TC_SEG_CHUNKS_V HM_TC_SEG_CHUNKS
-#endif
-// chunks per accumulator buffer, for near/U tiles and for V pieces: the
-// tensor cores' own accumulation spans at most this many chunks (4 UMMAs
-// each) before the epilogue takes the partial sums into FP32 registers
-constexpr int kSegChunksDU = HM_TC_SEG_CHUNKS;
-
-constexpr int kSegChunksV = HM_TC_SEG_CHUNKS_V;
-
 // MN-major B: the hi and lo halves of the R right-hand sides are stacked along
-// N, so one XTS row (4R bytes) is one K row of B. Core matrices of 8 N values
-// (16 B) x 8 columns; the N groups are kBGroupN bytes apart, the K groups of 8
-// columns TcShape<R>::kBGroupK bytes apart.
-constexpr uint32_t kBGroupN = 128;
+// N, so one XTS row (4R bytes) is one K row of B. Swizzled atoms of 8 columns (K) x
+// TcShape<R>::kRowB bytes of their rows: 64 bytes with 16 right-hand sides, else 128. A tile load
+// moves a row's part of an atom as one request; with unswizzled core matrices (16 bytes of 8
+// rows) the loads' 16-byte requests bound the near/U passes: film 500,500, 32 columns, 847 us
+// against 739; 32,768-point cube, 64 columns, 609 against 534.
 
 // The shape of a pass over R = 16, 32 or 64 right-hand sides. A 64-wide pass reads
 // every tile once for twice the columns; its B tiles are twice as large, so
@@ -124,8 +113,20 @@ struct TcShape {
   static constexpr uint32_t kTmemCols = 512;
   static constexpr int kBufs = static_cast<int>(kTmemCols) / kBN;  // 8 or 4
   static constexpr int kSetBufs = kBufs / 2;
-  static constexpr int kConsumers = kBProducers + kPipes + 8;  // warps that read each queued item
-  static constexpr uint32_t kBGroupK = (kBN / 8) * kBGroupN;
+  static constexpr int kConsumers = kPipeStages + 1 + 4;  // warps that read each queued item: pipeline and epilogue set
+  static constexpr uint32_t kRowB = R == 16 ? 64 : 128;     // bytes of a row in an atom: the swizzle's span
+  static constexpr uint32_t kAtoms = 4 * R / kRowB;         // atoms along N
+  static constexpr uint32_t kAtomB = 8 * kRowB;
+  // near/U tiles: K groups of 8 columns, the atoms of each behind one another; V pieces (a 64-row
+  // tile load): the K groups of the first atom, then those of the second
+  static constexpr uint32_t kBGroupK = kAtoms * kAtomB, kVAtom = kKc * kRowB;
+  static constexpr uint64_t kBSwizzle = static_cast<uint64_t>(R == 16 ? 4 : 2) << 61;  // descriptor: 64- or 128-byte
+  // place of 16-byte piece p of column k's row in a near/U tile
+  static __device__ __forceinline__ uint32_t b_piece(uint32_t k, uint32_t p) {
+    constexpr uint32_t per = kRowB / 16;
+    const uint32_t x = R == 16 ? (k >> 1) & 3u : k & 7u;
+    return (k >> 3) * kBGroupK + (p / per) * kAtomB + (k & 7u) * kRowB + (((p % per) ^ x) << 4);
+  }
   static constexpr int kPieces = R / 4;               // 16-byte pieces of an XTS row
   static constexpr int kRowsPerCopy = 32 / kPieces;   // XTS rows per warp-wide copy
   // kind::f16 instruction descriptor: FP32 D, FP16 A (K-major) and B
@@ -136,8 +137,6 @@ struct TcShape {
   // one release ahead, which a parity wait on the stage's barrier could not
   // tell apart from the release before.
   static_assert(kBProducers == kStages, "one producer warp per stage");
-  // the MMA warp waits for a whole segment's chunks before it releases any
-  static_assert(kSegChunksDU <= kPipeStages && kSegChunksV <= kPipeStages, "a segment fits a pipeline's stages");
 };
 constexpr unsigned long long kWaitNs = 2000000000ull;  // 2 s per wait
 constexpr unsigned long long kWaitIters = 1ull << 26;   // backstop if the timer stood still
@@ -153,7 +152,7 @@ __device__ __forceinline__ uint64_t sdesc(uint32_t saddr, uint32_t lbo, uint32_t
   d |= static_cast<uint64_t>((saddr >> 4) & 0x3FFF);
   d |= static_cast<uint64_t>((lbo >> 4) & 0x3FFF) << 16;
   d |= static_cast<uint64_t>((sbo >> 4) & 0x3FFF) << 32;
-  d |= static_cast<uint64_t>(1) << 46;  // descriptor version for tcgen05; no swizzle
+  d |= static_cast<uint64_t>(1) << 46;  // descriptor version for tcgen05; no swizzle unless added
   return d;
 }
 
@@ -223,10 +222,9 @@ struct TcSmem {
   uint32_t tmem;
   volatile int32_t abort;
 };
-// 128 bytes of alignment slack on top (the tile loads and the no-swizzle
-// operand layouts need 128-byte alignment at most); 232448 bytes is the
-// per-block limit
-constexpr size_t kSmemAlign = 128;
+// 1024 bytes of alignment slack on top (a 128-byte swizzle's pattern; the stages' A and B tiles
+// are multiples of it); 232448 bytes is the per-block limit
+constexpr size_t kSmemAlign = 1024;
 static_assert(sizeof(TcSmem<16>) + kSmemAlign <= 232448 && sizeof(TcSmem<32>) + kSmemAlign <= 232448 && sizeof(TcSmem<64>) + kSmemAlign <= 232448,
               "tensor-core pass shared memory");
 
@@ -273,7 +271,7 @@ __device__ __forceinline__ bool wait_bar_warp(SM &S, uint64_t *bar, uint32_t par
 }
 
 // Item n of this CTA from the queue (false: no more items, or an abort); every
-// consumer warp calls it once per n and releases the slot. The item itself
+// warp of the item's pipeline and epilogue set calls it once per n and releases the slot. The item itself
 // travels in the queue, so no consumer waits on a global load per item.
 template <class SM>
 __device__ __forceinline__ bool next_item(SM &S, int n, int32_t *status, TcItem &I) {
@@ -337,7 +335,7 @@ __global__ void wait_selftest_kernel(unsigned long long limit_ns, int32_t *statu
 }
 
 struct TcArgs {
-  CUtensorMap xmap;            // XTS as 8 FP16 x rows x N groups, 64-row boxes: the B tiles of V pieces
+  CUtensorMap xmap;            // XTS as swizzle spans x rows, 64-row boxes: the B tiles of V pieces
   CUtensorMap xmap8;           // the same view, 8-row boxes: K groups of near/U B tiles
   const unsigned char *adata;  // tensor-core panels
   const TcItem *items;
@@ -419,7 +417,7 @@ __global__ void __launch_bounds__(TcShape<R>::kThreads, 1) tc_kernel(const __gri
       TcItem mine{};
       mine.kind = -1;
       if (lane < want && b + lane < a.nitems) mine = a.items[b + lane];
-      for (int j = 0; j < want; j++, n++) {
+      for (int j = 0, ends = 0; j < want; n++) {
         TcItem t;
         t.a_off = __shfl_sync(0xffffffffu, mine.a_off, j);
         t.m = __shfl_sync(0xffffffffu, mine.m, j);
@@ -437,7 +435,9 @@ __global__ void __launch_bounds__(TcShape<R>::kThreads, 1) tc_kernel(const __gri
           S.qdata[q] = t;
           arrive(&S.qfull[q]);
         }
-        if (t.kind < 0) {
+        if (t.kind >= 0)
+          j++;
+        else if (++ends == 2) {  // one for the readers of even items, one for those of odd ones
           more = false;
           break;
         }
@@ -446,23 +446,23 @@ __global__ void __launch_bounds__(TcShape<R>::kThreads, 1) tc_kernel(const __gri
   } else if (warp == 1 || warp == 3 || (warp >= 8 && warp < Sh::kEpi1)) {
     // ---- producers: pipeline p = bw & 1 (items n with n & 1 == p); its chunk
     // g (stage p kPipeStages + g % kPipeStages) goes to its producer
-    // q = g % kPipeStages. Column rows are looked up before the stage is
+    // q = g % kPipeStages, so that a producer keeps to one stage. Column rows are looked up before the stage is
     // free; then each warp-wide copy moves kRowsPerCopy whole XTS rows
     // (kPieces lanes x 16 bytes per row), the warp waits for its copies,
     // fences them for the tensor cores' proxy and publishes the stage.
     const int bw = warp == 1 ? 0 : warp == 3 ? 1 : warp - 6;  // 0..kStages-1
     const int pipe = bw % Sh::kPipes, q = bw / Sh::kPipes;
-    int64_t g = 0, last_g = -1;  // last_g: the chunk whose bulk copies this warp issued last
+    const int s = pipe * Sh::kPipeStages + q;  // this warp's stage
+    uint32_t used = 0;                         // its chunks so far
+    int ch = q;                                // its next chunk, counted from the item's first
     bool stop = false;
     const int piece = lane % Sh::kPieces, sub = lane / Sh::kPieces;
-    for (int n = 0; !stop; n++) {
+    for (int n = pipe; !stop; n += Sh::kPipes) {
       TcItem I;
       if (!next_item(S, n, a.status, I)) break;
-      if ((n & 1) % Sh::kPipes != pipe) continue;
-      const int npad = I.ncols > 0 ? (I.ncols + 15) & ~15 : 16;
-      for (int c0 = 0; c0 < npad; c0 += kKc, g++) {
-        if (g % Sh::kPipeStages != q) continue;
-        const int kc = min(kKc, npad - c0), s = pipe * Sh::kPipeStages + static_cast<int>(g % Sh::kPipeStages);
+      const int npad = I.ncols > 0 ? (I.ncols + 15) & ~15 : 16, nch = (npad + kKc - 1) / kKc;
+      for (; ch < nch; ch += Sh::kPipeStages) {
+        const int c0 = ch * kKc, kc = min(kKc, npad - c0);
         // B of a V piece by one tile load of 64 XTS rows (in a last chunk the
         // MMA warp zeroes the rows of padding columns before it multiplies)
         const bool tma_b = I.kind != 0;
@@ -493,7 +493,7 @@ __global__ void __launch_bounds__(TcShape<R>::kThreads, 1) tc_kernel(const __gri
           }
           gmask &= (1u << (kc / 8)) - 1u;
         }
-        if (!wait_bar_warp(S, &S.empty[s], static_cast<uint32_t>((g / Sh::kPipeStages) & 1) ^ 1u, a.status, 22)) {
+        if (!wait_bar_warp(S, &S.empty[s], (used & 1u) ^ 1u, a.status, 22)) {
           stop = true;
           break;
         }
@@ -522,8 +522,7 @@ __global__ void __launch_bounds__(TcShape<R>::kThreads, 1) tc_kernel(const __gri
               : "memory");
           if (tma_b) {
             // B of a V piece: its columns are the consecutive XTS rows map + c0
-            // .., so one tile load of 64 rows lands them in the canonical
-            // MN-major layout (K groups 128 B apart, N groups 1024 B apart)
+            // .., so one tile load of 64 rows lands them
             asm volatile(
                 "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, "
                 "%4}], [%5];" ::"r"(su32(S.b[s])),
@@ -532,7 +531,7 @@ __global__ void __launch_bounds__(TcShape<R>::kThreads, 1) tc_kernel(const __gri
             arrive(&S.full[s]);
           }
         }
-        last_g = g;
+        used++;
         if (tma_b) {  // the copies complete on the stage's barrier
           __syncwarp();
           continue;
@@ -546,14 +545,14 @@ __global__ void __launch_bounds__(TcShape<R>::kThreads, 1) tc_kernel(const __gri
                 "%4}], [%5];" ::"r"(su32(S.b[s]) + static_cast<uint32_t>(q) * Sh::kBGroupK),
                 "l"(reinterpret_cast<uint64_t>(&a.xmap8)), "r"(0), "r"(grow[q]), "r"(0), "r"(su32(&S.full[s]))
                 : "memory");
-        const uint32_t dst0 = su32(S.b[s]) + piece * kBGroupN;
+        const uint32_t dst0 = su32(S.b[s]);
 #pragma unroll
         for (int i = 0; i < kKc / Sh::kRowsPerCopy; i++) {
           const int k = Sh::kRowsPerCopy * i + sub;
           const int r = __shfl_sync(0xffffffffu, rows[(i * Sh::kRowsPerCopy) >> 5], k & 31);
           if (k < kc && !((gmask >> (k >> 3)) & 1u)) {
             const uint16_t *src = a.xts + static_cast<int64_t>(r) * (2 * R) + piece * 8;
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst0 + (k >> 3) * Sh::kBGroupK + (k & 7) * 16),
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst0 + Sh::b_piece(k, piece)),
                          "l"(src)
                          : "memory");
           }
@@ -564,13 +563,13 @@ __global__ void __launch_bounds__(TcShape<R>::kThreads, 1) tc_kernel(const __gri
         __syncwarp();
         if (lane == 0) arrive(&S.full[s]);
       }
+      ch -= nch;
     }
     // The bulk copies of this warp's last chunk land before the CTA can exit,
     // aborted or not (one stage per producer: earlier chunks have landed).
-    if (last_g >= 0 && lane == 0) {
+    if (used > 0 && lane == 0) {
       volatile int32_t none = 0;
-      wait_bar_bounded(&S.full[pipe * Sh::kPipeStages + last_g % Sh::kPipeStages],
-                       static_cast<uint32_t>((last_g / Sh::kPipeStages) & 1), &none, a.status, 31, kWaitNs);
+      wait_bar_bounded(&S.full[s], (used - 1u) & 1u, &none, a.status, 31, kWaitNs);
     }
     __syncwarp();
   } else if (warp == 2 || (Sh::kPipes == 2 && warp == Sh::kMma1)) {
@@ -582,91 +581,86 @@ __global__ void __launch_bounds__(TcShape<R>::kThreads, 1) tc_kernel(const __gri
     // into the item's accumulator; the epilogue adds its four quadrants.
     const int pipe = warp == 2 ? 0 : 1;
     const int s0 = pipe * Sh::kPipeStages;  // the pipeline's first stage
-    int64_t g = 0;                          // the pipeline's chunks so far
-    int n = 0;
-    bool stop = false;
-    // Every kSegChunks chunks of an item go to a fresh accumulator buffer of
-    // the item's epilogue set (set n & 1, buffers used in turn), whose warps
-    // add the buffers' sums in FP32 registers: the tensor cores' own
-    // accumulation then spans at most 4 kSegChunks UMMAs, whatever the item's
-    // length.
-    uint32_t kseg[2] = {0u, 0u};  // buffers handed to each epilogue set so far
-    for (; !stop; n++) {
+    const bool leader = elect_one();        // issues every UMMA and commit
+    // Every chunk of an item goes to a fresh accumulator buffer of the item's
+    // epilogue set (set n & 1, buffers used in turn), whose warps add the
+    // buffers' sums in FP32 registers: the tensor cores' own accumulation
+    // spans 4 UMMAs, whatever the item's length. The warp's own instructions per
+    // chunk bound the passes (without any copies they took as long), so stage, phase and
+    // buffer are counted up, not divided out of a 64-bit chunk number, a warp reads the
+    // items of its own pipeline only, and the votes are one per chunk: 32,768-point cube, 64
+    // columns, V pass 319 -> 283 us, near/U 534 -> 415; film 500,500, 32 columns, V 380 -> 338.
+    uint32_t st = 0, phase = 0;             // stage of the next chunk, parity of its phase
+    uint32_t seg0 = 0, seg1 = 0;            // buffers handed to each epilogue set so far
+    bool stop = false, any = false;
+    for (int n = pipe; !stop; n += Sh::kPipes) {
       TcItem I;
       if (!next_item(S, n, a.status, I)) break;
-      if ((n & 1) % Sh::kPipes != pipe) continue;
       const int e = n & 1;
       const int npad = I.ncols > 0 ? (I.ncols + 15) & ~15 : 16;
-      // V pieces' B tiles come from the tile load (K groups 128 B apart, N
-      // groups 1024 B), near/U tiles' from the gather (kBGroupK, 128 B)
       const bool tma_b = I.kind != 0;
-      const int kSegChunks = tma_b ? kSegChunksV : kSegChunksDU;
-      // One pass of this loop per accumulator buffer: the segment's chunks
-      // c0 / kKc .. + nseg - 1 (stages g .. g + nseg - 1) are waited for
-      // first, then all their UMMAs go out under one fence and one election.
-      // The warp's own per-chunk instructions are what bound the pass, so
-      // they are paid once per segment. nseg <= kPipeStages: the producers of
-      // the segment's chunks never wait for the segment itself.
-      for (int c0 = 0; c0 < npad;) {
-        const int nseg = min(kSegChunks, (npad - c0 + kKc - 1) / kKc);
-        const int buf = e * Sh::kSetBufs + static_cast<int>(kseg[e] % Sh::kSetBufs);
-        bool ok = wait_bar_warp(S, &S.seg_empty[buf], ((kseg[e] / Sh::kSetBufs) & 1u) ^ 1u, a.status, 23);
-        for (int j = 0; ok && j < nseg; j++)
-          ok = wait_bar_warp(S, &S.full[s0 + static_cast<int>((g + j) % Sh::kPipeStages)],
-                             static_cast<uint32_t>(((g + j) / Sh::kPipeStages) & 1), a.status, 24);
-        if (!ok) {
+      // B, swizzled: offsets from atom to atom along N, and from K group to K group; the two
+      // K groups of a UMMA follow one another
+      const uint32_t lbo = tma_b ? Sh::kVAtom : Sh::kAtomB, sbo = tma_b ? Sh::kAtomB : Sh::kBGroupK;
+      uint32_t seg = e ? seg1 : seg0;
+      for (int c0 = 0; c0 < npad; c0 += kKc, seg++) {
+        const int kc = min(kKc, npad - c0);
+        const int buf = e * Sh::kSetBufs + static_cast<int>(seg % Sh::kSetBufs);
+        const int at = s0 + static_cast<int>(st);
+        const bool ok = wait_bar(S, &S.seg_empty[buf], ((seg / Sh::kSetBufs) & 1u) ^ 1u, a.status, 23) &&
+                        wait_bar(S, &S.full[at], phase, a.status, 24);
+        if (!__all_sync(0xffffffffu, ok)) {
           stop = true;
           break;
         }
-        const int cl = c0 + (nseg - 1) * kKc, kcl = min(kKc, npad - cl);  // the segment's last chunk
-        if (tma_b && I.ncols - cl < kcl) {
+        if (tma_b && I.ncols - c0 < kc) {
           // the last chunk of a V piece: the tile load brought 64 consecutive
           // XTS rows, and those of the padding columns [ncols, kc) belong to
           // other blocks (or are t rows being rewritten). The A tile is zero
           // there, but 0 * Inf and 0 * NaN are not, so the rows are zeroed
-          // (16 bytes per row and N group) before the UMMAs read them.
-          const uint32_t bl = su32(S.b[s0 + static_cast<int>((g + nseg - 1) % Sh::kPipeStages)]);
-          const int valid = I.ncols - cl, nz = kcl - valid;
+          // before the UMMAs read them (whole rows, so their pieces' order does not matter).
+          const uint32_t bl = su32(S.b[at]);
+          const int valid = I.ncols - c0, nz = kc - valid;
           for (int z = lane; z < nz * (Sh::kBN / 8); z += 32) {
             const int k = valid + z % nz, gq = z / nz;
-            asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(bl + gq * 1024u + k * 16u), "r"(0u)
+            asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(bl + gq / (Sh::kRowB / 16) * Sh::kVAtom +
+                                                                         k * Sh::kRowB + gq % (Sh::kRowB / 16) * 16u),
+                         "r"(0u)
                          : "memory");
           }
           asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
           __syncwarp();
         }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        if (elect_one()) {
+        if (leader) {
           const uint32_t acc = S.tmem + static_cast<uint32_t>(buf * Sh::kBN);
-          for (int j = 0; j < nseg; j++) {
-            const int st = s0 + static_cast<int>((g + j) % Sh::kPipeStages), kc = min(kKc, npad - c0 - j * kKc);
-            // leading byte offset: K direction; stride byte offset: N direction
-            const uint64_t da = sdesc(su32(S.a[st]), 128, static_cast<uint32_t>(kc) * 16);
-            const uint64_t db =
-                tma_b ? sdesc(su32(S.b[st]), 128, 1024) : sdesc(su32(S.b[st]), Sh::kBGroupK, kBGroupN);
+          // A: leading byte offset in the K direction, stride byte offset in the M direction
+          const uint64_t da = sdesc(su32(S.a[at]), 128, static_cast<uint32_t>(kc) * 16);
+          const uint64_t db = Sh::kBSwizzle | sdesc(su32(S.b[at]), lbo, sbo);
 #pragma unroll
-            for (int ks = 0; ks < kKc / 16; ks++) {
-              if (ks < kc / 16) {
-                // the start address field counts 16-byte units
-                const uint64_t oa = static_cast<uint64_t>(ks * 256) >> 4,
-                               ob = static_cast<uint64_t>(tma_b ? ks * 256 : ks * 2 * Sh::kBGroupK) >> 4;
-                mma(acc, da + oa, db + ob, Sh::kIdesc, (j == 0 && ks == 0) ? 0u : 1u);
-              }
-            }
-            commit(&S.empty[st]);
-          }
+          for (int ks = 0; ks < kKc / 16; ks++)
+            if (ks < kc / 16)  // the start address field counts 16-byte units
+              mma(acc, da + ((ks * 256) >> 4), db + ((ks * 2 * sbo) >> 4), Sh::kIdesc, ks == 0 ? 0u : 1u);
+          commit(&S.empty[at]);
           commit(&S.seg_full[buf]);
         }
-        __syncwarp();
-        kseg[e]++;
-        g += nseg;
-        c0 += nseg * kKc;
+        any = true;
+        if (++st == Sh::kPipeStages) {
+          st = 0;
+          phase ^= 1u;
+        }
       }
+      if (e)
+        seg1 = seg;
+      else
+        seg0 = seg;
     }
     // the last stage release must land before the CTA's shared memory goes away
-    if (!stop && g > 0)
-      wait_bar_warp(S, &S.empty[s0 + static_cast<int>((g - 1) % Sh::kPipeStages)],
-                    static_cast<uint32_t>(((g - 1) / Sh::kPipeStages) & 1), a.status, 26);
+    if (!stop && any) {
+      const bool first = st == 0;
+      wait_bar_warp(S, &S.empty[s0 + (first ? Sh::kPipeStages - 1 : static_cast<int>(st) - 1)],
+                    first ? phase ^ 1u : phase, a.status, 26);
+    }
   } else if ((warp >= 4 && warp < 8) || (warp >= Sh::kEpi1 && warp < Sh::kEpi1 + 4)) {
     // ---- epilogue -----------------------------------------------------------
     // Set e (warps 4-7 or the last four) takes accumulator e, that is items
@@ -688,14 +682,11 @@ __global__ void __launch_bounds__(TcShape<R>::kThreads, 1) tc_kernel(const __gri
     uint64_t *i_ready = lo_part ? &S.xb_ready[e] : &S.xa_ready[e];
     uint64_t *i_free = lo_part ? &S.xb_free[e] : &S.xa_free[e];
     uint32_t kseg = 0;  // accumulator buffers of this set consumed so far
-    for (int n = 0;; n++) {
+    for (int n = e;; n += 2) {
       TcItem I;
       if (!next_item(S, n, a.status, I)) break;
-      if ((n & 1) != e) continue;
       const uint32_t k = static_cast<uint32_t>(n >> 1);  // this set's item count
-      const int nch = ((I.ncols > 0 ? (I.ncols + 15) & ~15 : 16) + kKc - 1) / kKc;
-      const int span = I.kind != 0 ? kSegChunksV : kSegChunksDU;
-      const int nbuf = (nch + span - 1) / span;  // accumulator buffers of the item
+      const int nbuf = ((I.ncols > 0 ? (I.ncols + 15) & ~15 : 16) + kKc - 1) / kKc;  // one per chunk
       // the row's factor (1 / rho_i, or gamma_k / nu_k for V rows) and, for y
       // rows, the output row and the member, loaded now: they do not depend on
       // the MMA, so their latency hides behind its wait
@@ -1055,15 +1046,17 @@ cudaError_t encode_xts_map(DevTc &t, int R) {
   if (R != 16 && R != 32 && R != 64) return cudaErrorInvalidValue;
   uint16_t *xts = t.xts[R / 32];
   if (!enc || !xts || t.xt_rows < 8) return cudaErrorInvalidValue;
-  // element (e, row, g) = XTS[row][8 g + e]: a box of 8 x 64 x 2R/8 lands as
-  // 2R/8 N groups of 64 rows x 16 bytes
-  cuuint64_t dims[3] = {8, static_cast<cuuint64_t>(t.xt_rows), static_cast<cuuint64_t>(2 * R / 8)};
-  cuuint64_t strides[2] = {static_cast<cuuint64_t>(4 * R), 16};
+  // element (e, row, g) = XTS[row][w g + e], w = 32 or 64: a box lands as 2R / w atoms' rows of
+  // 2 w bytes, swizzled
+  const int w = R == 16 ? 32 : 64;
+  cuuint64_t dims[3] = {static_cast<cuuint64_t>(w), static_cast<cuuint64_t>(t.xt_rows), static_cast<cuuint64_t>(2 * R / w)};
+  cuuint64_t strides[2] = {static_cast<cuuint64_t>(4 * R), static_cast<cuuint64_t>(2 * w)};
   for (int b = 0; b < 2; b++) {  // boxes of 64 rows (V pieces) and of 8 rows (K groups of near/U tiles)
-    cuuint32_t box[3] = {8, b == 0 ? 64u : 8u, static_cast<cuuint32_t>(2 * R / 8)};
+    cuuint32_t box[3] = {static_cast<cuuint32_t>(w), b == 0 ? 64u : 8u, static_cast<cuuint32_t>(2 * R / w)};
     cuuint32_t es[3] = {1, 1, 1};
     const CUresult r = enc(&t.xmap[3 * b + R / 32], CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, xts, dims, strides, box, es,
-                           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE,
+                           CU_TENSOR_MAP_INTERLEAVE_NONE, R == 16 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B,
+                           CU_TENSOR_MAP_L2_PROMOTION_NONE,
                            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return cudaErrorInvalidValue;
   }
