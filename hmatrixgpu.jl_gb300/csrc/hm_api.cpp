@@ -570,23 +570,24 @@ extern "C" int hmgpu_matvec(hmgpu_hmatrix *h, const void *x, void *y, int64_t nr
       cudaMemsetAsync(xts, 0, xb, s);
       if (cudaError_t e = hm::encode_xts_map(H.tc, w)) return hm::cuda_fail(e, "tensor map of XTS");
     }
-    if (!tc && !H.xt_multi) {
+    if (!tc && !H.dp.mcolmap) {  // one allocation: an allocation costs more than the kernel
       std::vector<int64_t> col0(H.plan.tiles.size());
       int64_t ncm = 0;
       for (size_t t = 0; t < col0.size(); t++) {
         col0[t] = ncm;
         ncm += H.plan.tiles[t].ncols;
       }
-      if ((rc = hm::upload(H, &H.dp.mcol0, col0)) ||
-          (rc = H.dalloc(reinterpret_cast<void **>(&H.dp.mcolmap), ncm * sizeof(int32_t))))
-        return rc;
-      if (cudaError_t e = hm::launch_colmap(H.dp.tiles, H.dp.ntiles, H.dp.segs, H.dp.mcol0, H.dp.mcolmap, s))
-        return hm::cuda_fail(e, "column map");
-      if ((rc = H.dalloc(&H.xt_multi, H.plan.xt_len * per * es)) ||
-          (rc = H.dalloc(&H.p_multi, std::max<int64_t>(H.plan.p_rows, 1) * per * es)))
-        return rc;
-      cudaMemsetAsync(H.xt_multi, 0, H.plan.xt_len * per * es, s);
+      const int64_t mb = (ncm * static_cast<int64_t>(sizeof(int32_t)) + 7) & ~int64_t(7);
+      char *map = nullptr;
+      if ((rc = H.dalloc(reinterpret_cast<void **>(&map), mb + col0.size() * sizeof(int64_t)))) return rc;
+      int64_t *first = reinterpret_cast<int64_t *>(map + mb);
+      cudaError_t e = cudaMemcpyAsync(first, col0.data(), col0.size() * sizeof(int64_t), cudaMemcpyHostToDevice, s);
+      if (e == cudaSuccess)
+        e = hm::launch_colmap(H.dp.tiles, H.dp.ntiles, H.dp.segs, first, reinterpret_cast<int32_t *>(map), s);
+      if (e != cudaSuccess) return hm::cuda_fail(e, "column map");
+      H.dp.mcolmap = reinterpret_cast<int32_t *>(map);
     }
+    if (!tc && !H.p_multi && H.plan.p_rows > 0 && (rc = H.dalloc(&H.p_multi, H.plan.p_rows * per * es))) return rc;
     for (int64_t k0 = 0, nr = 0; k0 < nrhs; k0 += nr) {
       cudaEvent_t *ev;
       if ((rc = next_events(&ev))) return rc;
@@ -603,14 +604,10 @@ extern "C" int hmgpu_matvec(hmgpu_hmatrix *h, const void *x, void *y, int64_t nr
         // each pass width has its own XT (zeroed once): rows that no pass
         // writes (padding, the zero row) must read as zero in that width's layout
         const int w = hm::multi_width(f64, static_cast<int>(nr));
-        void *xt = H.xt_multi;
-        if (w < per) {
-          void *&xw = H.xt_multi_w[w == 4 ? 0 : w == 8 ? 1 : 2];
-          if (!xw) {
-            if ((rc = H.dalloc(&xw, H.plan.xt_len * w * es))) return rc;
-            cudaMemsetAsync(xw, 0, H.plan.xt_len * w * es, s);
-          }
-          xt = xw;
+        void *&xt = w == per ? H.xt_multi : H.xt_multi_w[w == 4 ? 0 : w == 8 ? 1 : 2];
+        if (!xt) {
+          if ((rc = H.dalloc(&xt, H.plan.xt_len * w * es))) return rc;
+          cudaMemsetAsync(xt, 0, H.plan.xt_len * w * es, s);
         }
         e = hm::launch_matvec_multi(f64, H.dp, H.panels, H.vdata, xt, H.p_multi,
                                     static_cast<const char *>(x) + k0 * ldx * es, ldx, static_cast<int>(nr),

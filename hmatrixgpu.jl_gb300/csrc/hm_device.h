@@ -17,7 +17,6 @@ struct DevPlan {
   MUnit *munits = nullptr;       // multi-RHS near/U work: at most 64 rows of a tile, widest tiles first
   int32_t nmunits = 0;
   int32_t *mcolmap = nullptr;    // XT row of every tile column, tile after tile (first multi-RHS product)
-  int64_t *mcol0 = nullptr;      // first entry of each tile
   VUnit *vunits = nullptr;
   int32_t nvunits = 0;
   int32_t *warp_begin = nullptr;

@@ -115,7 +115,7 @@ struct VUnit {
 };
 static_assert(sizeof(VUnit) == 32, "VUnit layout");
 
-// A work item of the multi-right-hand-side V pass: at most 128 rows of one
+// A work item of the multi-right-hand-side V pass: at most 64 rows of one
 // source group times one column piece [c, c + ncols) of the group's stored
 // columns. Wide groups are cut into pieces of bounded size whose partial
 // products go to rows of a scratch array P and are summed in piece order
@@ -198,7 +198,7 @@ struct Plan {
 void make_plan(const BlockSet &bs, int vec, int nwarps, const std::vector<int64_t> &dense_src_off,
                const std::vector<int64_t> &u_src_off, Plan &p);
 
-// Near/U row units of `unit_rows` (<= 16) rows over p.tile_order, and the V
+// Near/U row units of `unit_rows` (8, 16, 32 or 64) rows over p.tile_order, and the V
 // units of about `unit_bytes` with their static split over `nwarps` warps: both
 // only partition the stored layout, so they can be rebuilt at any time.
 void make_units(Plan &p, int32_t unit_rows);

@@ -303,7 +303,7 @@ void make_plan(const BlockSet &bs, int vec, int nwarps, const std::vector<int64_
     if (rows == 0) continue;
     const int64_t t0 = p.t_off[a0];  // the group's t entries are contiguous
     p.vgroups.push_back(VGroup{gbase, stride, rows, bs.a_cs[a0] - ph, static_cast<int32_t>(t0)});
-    // multi-RHS items: 128-row blocks, wide ones cut into column pieces
+    // multi-RHS items: 64-row blocks, wide ones cut into column pieces
     for (int32_t k0 = 0; k0 < rows; k0 += kMVRows) {
       const int32_t nr = std::min(kMVRows, rows - k0);
       const int64_t pieces0 = std::max<int64_t>(1, (static_cast<int64_t>(nr) * stride + kMVEntries - 1) / kMVEntries);

@@ -90,8 +90,8 @@ constexpr int kQ = 16;                  // item queue slots
 // every tile once for twice the columns; its B tiles are twice as large, so
 // the ring has 6 stages instead of 8. A 16-wide pass gathers half the XTS bytes of a
 // 32-wide one, and its smaller B tiles leave room for 10 stages: 32,768-point cube at 1e-6,
-// up to 16 columns, 482 us per product against 578 of the 32-wide pass; film 500,500 1108
-// against 1309.
+// up to 16 columns, 412 us per product against 500 of the 32-wide pass; film 500,500 1018
+// against 1109.
 template <int R>
 struct TcShape {
   static_assert(R == 16 || R == 32 || R == 64, "16, 32 or 64 right-hand sides per pass");
@@ -100,7 +100,9 @@ struct TcShape {
   static constexpr int kStages = R == 16 ? 10 : R == 32 ? 8 : 6;
   // Two pipelines for 16 and 32 right-hand sides. A 64-wide pass keeps one: a 17th
   // warp would cap every thread at 96 registers (warps per scheduler x
-  // threads x registers), and its epilogue needs more for 64 sums a row.
+  // threads x registers), and its epilogue needs more for 64 sums a row (two pipelines of
+  // three stages, TMEM read 8 columns at a time: near/U of the 32,768-point cube 467 us
+  // against 415).
   static constexpr int kPipes = R <= 32 ? 2 : 1;
   static constexpr int kPipeStages = kStages / kPipes;  // stages of each pipeline
   static constexpr int kBProducers = kStages;           // warps 1, 3, 8 .. 5 + kStages
