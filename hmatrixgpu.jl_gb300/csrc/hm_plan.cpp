@@ -83,8 +83,12 @@ void make_vunits(Plan &p, int64_t unit_bytes, int nwarps) {
   // more, since the FP64 pipe takes as long for one active lane as for 32. V pass
   // in us with 4 / 8 / 16 vectors a lane: film 2^20 FP32 580 / 507 / 512, batch of
   // 12 spheres 113 / 77 / 81; 40,960-point cube FP64 673 / 497 / 372.
-  const int32_t lane_vecs = p.vec == 2 ? 16 : 8;
+  // FP32 groups of many rank rows (volumes) take 4: their matrices are large, and longer
+  // runs of each row per load count more (cube 2^18 at 1e-6 2245 us with 8, 1894 with 4; cube
+  // 40,960 129 and 133; sphere 20,011, few rows per group, whole product 58.7 and 64.7). The
+  // rule looks at the group alone, so that batches and shards sum every row as its matrix does.
   for (const VGroup &g : p.vgroups) {
+    const int32_t lane_vecs = p.vec == 2 ? 16 : g.rows >= 512 ? 4 : 8;
     int32_t nv = g.stride / p.vec, lanes = 1;
     while (lanes * lane_vecs < nv && lanes < 32) lanes *= 2;
     const int64_t row_bytes = static_cast<int64_t>(g.stride) * esize;
