@@ -500,13 +500,13 @@ __global__ void __launch_bounds__(kDuWarps * 32, multi_ctas<T, kDuWarps>()) du_m
       slice_product<T, W, mt.value>(a.panels + U.data_off, U.ld, U.m, U.ld, warp, kDuWarps, a.xt,
                                     dyn_smem + warp * 2 * stage_bytes<T, W>(),
                                     [&](int c) { return c < U.ncols ? __ldg(map + c) : -1; }, acc);
-      if (tid == 0) s_ticket = next;
       sum_warps<T, W, kDuWarps, mt.value, true>(
           acc, U.m, dyn_smem,
           [&](int row, int q, T s) {
             if (q < a.nr) a.y[a.tmap0[U.row0 + row] + q * a.ldy] = s;
           });
     });
+    if (tid == 0) s_ticket = next;  // (the one before was read by all warps before sum_warps' barriers)
     __syncthreads();  // the sums are read, the stages may be filled again
     u = s_ticket;
   }
