@@ -439,6 +439,7 @@ __global__ void __launch_bounds__(kThreads, 6) du_rows_kernel(DuArgs<T> a) {
       }
     }
     if (DIRECT) break;  // a unit per CTA
+    if (d.ld == 0) __syncthreads();  // no columns, no barrier above: all warps have read the ticket before
     if (tid == 0) s_ticket = next;
     __syncthreads();  // the entries and segments are no longer read
     u = s_ticket;

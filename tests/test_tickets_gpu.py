@@ -59,3 +59,19 @@ def test_short_tiles_several_columns(gpu, precision, tol, nrhs):
     assert np.linalg.norm(first.double().cpu().numpy() - want) <= tol * np.linalg.norm(want)
     for _ in range(50):
         assert torch.equal(H * Xd, first)
+
+
+@pytest.mark.parametrize("precision,tol", [("f64", 1e-12), ("f32", 1e-5), ("mixed", 1e-5)])
+def test_tiles_without_columns_one_column(gpu, precision, tol):
+    """Tiles covered by rank-0 blocks alone come one after another, at the end of the list."""
+    import torch
+    flat, ref = _thin(9 * 6000, 9, 4, seed=7)
+    H = hmgpu.HMatrix.from_flat(*flat, precision=precision)
+    x = np.random.default_rng(8).standard_normal((H.shape[1], 1)).astype(np.float32).astype(np.float64)
+    want = ref(x)[:, 0]
+    xd = torch.tensor(x[:, 0], dtype=torch.float64 if precision == "f64" else torch.float32, device=gpu)
+    first = H * xd
+    assert np.linalg.norm(first.double().cpu().numpy() - want) <= tol * np.linalg.norm(want)
+    assert (first.cpu().numpy()[want == 0.0] == 0.0).all()
+    for _ in range(50):
+        assert torch.equal(H * xd, first)
