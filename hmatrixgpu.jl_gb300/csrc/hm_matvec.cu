@@ -13,6 +13,7 @@
 // and stay in L2.
 #include <cuda_runtime.h>
 
+#include <cstdint>
 #include <type_traits>
 
 #include "hm_device.h"
@@ -466,11 +467,20 @@ int occupancy_du(bool f64, bool comp) {
   return n > 0 ? n : 1;
 }
 
+// Whether n elements at x and m elements at y have memory in common.
+template <typename T>
+static bool overlaps(const T *x, int64_t n, const T *y, int64_t m) {
+  const uintptr_t x0 = reinterpret_cast<uintptr_t>(x), y0 = reinterpret_cast<uintptr_t>(y);
+  return x0 < y0 + m * sizeof(T) && y0 < x0 + n * sizeof(T);
+}
+
 template <typename T, bool COMP>
 static cudaError_t run(const DevPlan &p, const T *panels, const T *vdata, T *xt, const T *x, T *y,
                        int grid_v, int grid_du, cudaStream_t s, cudaEvent_t *ev, int *launches) {
   const bool overlap = may_overlap(sizeof(T) == 8, p.entries, 1);
-  const bool direct = p.nvunits <= grid_v * (kThreads / 32) && p.nunits <= grid_du;
+  // x is read while y is written: not where they share memory (y = H y in place), which the
+  // permuted copy allows
+  const bool direct = p.nvunits <= grid_v * (kThreads / 32) && p.nunits <= grid_du && !overlaps(x, p.n, y, p.m);
   int nl = 0;
   cudaError_t e = cudaSuccess;
   if (ev) cudaEventRecord(ev[0], s);
