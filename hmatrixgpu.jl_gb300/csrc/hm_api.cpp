@@ -588,11 +588,16 @@ extern "C" int hmgpu_matvec(hmgpu_hmatrix *h, const void *x, void *y, int64_t nr
       H.dp.mcolmap = reinterpret_cast<int32_t *>(map);
     }
     if (!tc && !H.p_multi && H.plan.p_rows > 0 && (rc = H.dalloc(&H.p_multi, H.plan.p_rows * per * es))) return rc;
+    // a pass reads its columns of x before it writes those of y: where the two share memory other
+    // than column by column, passes are as wide as they can be
+    const uintptr_t x0 = reinterpret_cast<uintptr_t>(x), y0 = reinterpret_cast<uintptr_t>(y);
+    const bool shared = x0 < y0 + ((nrhs - 1) * ldy + H.bs.m) * es && y0 < x0 + ((nrhs - 1) * ldx + H.bs.n) * es &&
+                        !(x == y && ldx == ldy);
     for (int64_t k0 = 0, nr = 0; k0 < nrhs; k0 += nr) {
       cudaEvent_t *ev;
       if ((rc = next_events(&ev))) return rc;
-      nr = tc ? std::min<int64_t>(per, nrhs - k0)
-              : hm::multi_pass_columns(f64, nrhs - k0, H.dp.entries, H.num_sms);
+      nr = tc || shared ? std::min<int64_t>(per, nrhs - k0)
+                        : hm::multi_pass_columns(f64, nrhs - k0, H.dp.entries, H.num_sms);
       int nl = 0;
       cudaError_t e;
       if (tc)  // scaled FP16 (hi, lo) splits on the tensor cores

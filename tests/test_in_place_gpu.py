@@ -52,3 +52,23 @@ def test_one_column(gpu, n, precision):
     own = S.mul_permuted(torch.empty(rows, device=gpu, dtype=x.dtype), xp)
     z = xp.clone()
     assert torch.equal(S.mul_permuted(z[:rows], z), own)
+
+
+@pytest.mark.parametrize("precision", ["f64", "f32", "mixed"])
+@pytest.mark.parametrize("nrhs", [2, 3, 18])
+def test_several_columns(gpu, precision, nrhs):
+    """In place, and (from three columns on) with y two columns behind x in one array."""
+    import torch
+    H, _ = _matrix(700, precision, gpu)
+    n = H.shape[1]
+    dt = torch.float64 if precision == "f64" else torch.float32
+    X = torch.randn(nrhs, n, device=gpu, dtype=dt, generator=torch.Generator(gpu).manual_seed(nrhs)).t()
+    want = H * X
+    Z = X.clone(memory_format=torch.preserve_format)
+    hmgpu.mul_(Z, H, Z)
+    assert torch.equal(Z, want)
+    if nrhs >= 3:
+        buf = torch.zeros(nrhs + 2, n, device=gpu, dtype=dt).t()
+        buf[:, :nrhs].copy_(X)
+        hmgpu.mul_(buf[:, 2:], H, buf[:, :nrhs])
+        assert torch.equal(buf[:, 2:], want)
