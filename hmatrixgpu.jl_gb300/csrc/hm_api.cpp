@@ -159,7 +159,7 @@ int upload_plan(HMatrix &H, const std::vector<int32_t> &tmap0, const std::vector
       }
       if (static_cast<int64_t>(mu.size()) >= want) break;
     }
-    if ((rc = upload(H, &H.dp.munits, mu))) return rc;
+    if ((rc = upload(H, &H.dp.munits, mu)) || (rc = upload(H, &H.dp.mcol0, map0))) return rc;
     H.dp.nmunits = static_cast<int32_t>(mu.size());
   }
   {  // device order: by first XT row, so pieces reading the same x rows share them in L2
@@ -544,6 +544,24 @@ extern "C" int hmgpu_matvec(hmgpu_hmatrix *h, const void *x, void *y, int64_t nr
     *ev = H.prof_ev[H.prof_used++].data();
     return HMGPU_OK;
   };
+  // The one-time contents of scratch that this call allocates: on the caller's stream, or, while
+  // that is captured, on a stream of its own and waited for. In the graph they would run with
+  // its replays only, and a product before the first replay would read scratch without contents.
+  auto first_fill = [](cudaStream_t on, auto fill) -> int {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(on, &st) != cudaSuccess) cudaGetLastError();  // the launches that follow fail, too
+    cudaError_t e = cudaSuccess;
+    if (st == cudaStreamCaptureStatusNone) {
+      e = fill(on);
+    } else {
+      cudaStream_t own = nullptr;
+      e = cudaStreamCreateWithFlags(&own, cudaStreamNonBlocking);
+      if (e == cudaSuccess) e = fill(own);
+      if (e == cudaSuccess) e = cudaStreamSynchronize(own);
+      if (own) cudaStreamDestroy(own);
+    }
+    return e == cudaSuccess ? HMGPU_OK : hm::cuda_fail(e, "preparing the multi-RHS scratch");
+  };
   if (nrhs >= H.multi_from) {
     // several right-hand sides: one pass per rhs_per_pass() columns, the
     // matrix read once per pass (hm_multi.cu); for mixed precision one pass
@@ -555,10 +573,10 @@ extern "C" int hmgpu_matvec(hmgpu_hmatrix *h, const void *x, void *y, int64_t nr
     if (tc && !H.tc.prow) {
       const size_t sb = 2 * static_cast<size_t>(H.tc.nmem) * hm::kTcMaxRhs * sizeof(float);
       if ((rc = H.dalloc(reinterpret_cast<void **>(&H.tc.xscale), sb)) ||
+          (rc = first_fill(s, [&](cudaStream_t q) { return cudaMemsetAsync(H.tc.xscale, 0, sb, q); })) ||
           (rc = H.dalloc(reinterpret_cast<void **>(&H.tc.prow),
                          std::max<int64_t>(H.plan.p_rows, 1) * hm::kTcMaxRhs * 4)))
         return rc;
-      cudaMemsetAsync(H.tc.xscale, 0, sb, s);
     }
     // the XTS of every width that this call's passes have
     for (int64_t left = nrhs; tc && left > 0; left -= std::min<int64_t>(left, per)) {
@@ -567,25 +585,24 @@ extern "C" int hmgpu_matvec(hmgpu_hmatrix *h, const void *x, void *y, int64_t nr
       if (xts) continue;
       const int64_t xb = H.plan.xt_len * 2 * w * 2;
       if ((rc = H.dalloc(reinterpret_cast<void **>(&xts), xb))) return rc;
-      cudaMemsetAsync(xts, 0, xb, s);
-      if (cudaError_t e = hm::encode_xts_map(H.tc, w)) return hm::cuda_fail(e, "tensor map of XTS");
-    }
-    if (!tc && !H.dp.mcolmap) {  // one allocation: an allocation costs more than the kernel
-      std::vector<int64_t> col0(H.plan.tiles.size());
-      int64_t ncm = 0;
-      for (size_t t = 0; t < col0.size(); t++) {
-        col0[t] = ncm;
-        ncm += H.plan.tiles[t].ncols;
+      rc = first_fill(s, [&](cudaStream_t q) { return cudaMemsetAsync(xts, 0, xb, q); });
+      if (cudaError_t e = rc ? cudaSuccess : hm::encode_xts_map(H.tc, w)) rc = hm::cuda_fail(e, "tensor map of XTS");
+      if (rc) {
+        H.dfree(xts);
+        xts = nullptr;
+        return rc;
       }
-      const int64_t mb = (ncm * static_cast<int64_t>(sizeof(int32_t)) + 7) & ~int64_t(7);
-      char *map = nullptr;
-      if ((rc = H.dalloc(reinterpret_cast<void **>(&map), mb + col0.size() * sizeof(int64_t)))) return rc;
-      int64_t *first = reinterpret_cast<int64_t *>(map + mb);
-      cudaError_t e = cudaMemcpyAsync(first, col0.data(), col0.size() * sizeof(int64_t), cudaMemcpyHostToDevice, s);
-      if (e == cudaSuccess)
-        e = hm::launch_colmap(H.dp.tiles, H.dp.ntiles, H.dp.segs, first, reinterpret_cast<int32_t *>(map), s);
-      if (e != cudaSuccess) return hm::cuda_fail(e, "column map");
-      H.dp.mcolmap = reinterpret_cast<int32_t *>(map);
+    }
+    if (!tc && !H.dp.mcolmap) {
+      int64_t ncm = 0;
+      for (const hm::TileDesc &d : H.plan.tiles) ncm += d.ncols;
+      int32_t *map = nullptr;
+      if ((rc = H.dalloc(reinterpret_cast<void **>(&map), ncm * sizeof(int32_t))) ||
+          (rc = first_fill(s, [&](cudaStream_t q) {
+             return hm::launch_colmap(H.dp.tiles, H.dp.ntiles, H.dp.segs, H.dp.mcol0, map, q);
+           })))
+        return rc;
+      H.dp.mcolmap = map;
     }
     if (!tc && !H.p_multi && H.plan.p_rows > 0 && (rc = H.dalloc(&H.p_multi, H.plan.p_rows * per * es))) return rc;
     // a pass reads its columns of x before it writes those of y: where the two share memory other
@@ -611,8 +628,11 @@ extern "C" int hmgpu_matvec(hmgpu_hmatrix *h, const void *x, void *y, int64_t nr
         const int w = hm::multi_width(f64, static_cast<int>(nr));
         void *&xt = w == per ? H.xt_multi : H.xt_multi_w[w == 4 ? 0 : w == 8 ? 1 : 2];
         if (!xt) {
-          if ((rc = H.dalloc(&xt, H.plan.xt_len * w * es))) return rc;
-          cudaMemsetAsync(xt, 0, H.plan.xt_len * w * es, s);
+          void *t = nullptr;
+          const int64_t xb = H.plan.xt_len * w * es;
+          if ((rc = H.dalloc(&t, xb)) || (rc = first_fill(s, [&](cudaStream_t q) { return cudaMemsetAsync(t, 0, xb, q); })))
+            return rc;
+          xt = t;
         }
         e = hm::launch_matvec_multi(f64, H.dp, H.panels, H.vdata, xt, H.p_multi,
                                     static_cast<const char *>(x) + k0 * ldx * es, ldx, static_cast<int>(nr),

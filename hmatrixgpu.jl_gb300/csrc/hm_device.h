@@ -16,6 +16,7 @@ struct DevPlan {
   int32_t nunits = 0;
   MUnit *munits = nullptr;       // multi-RHS near/U work: at most 64 rows of a tile, widest tiles first
   int32_t nmunits = 0;
+  int64_t *mcol0 = nullptr;      // first entry of each tile in mcolmap
   int32_t *mcolmap = nullptr;    // XT row of every tile column, tile after tile (first multi-RHS product)
   VUnit *vunits = nullptr;
   int32_t nvunits = 0;
