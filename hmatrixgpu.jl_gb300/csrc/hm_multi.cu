@@ -25,6 +25,7 @@
 
 #include "hm_device.h"
 #include "hm_launch.cuh"
+#include "hm_per_device.h"
 
 namespace hm {
 
@@ -513,27 +514,29 @@ __global__ void __launch_bounds__(kDuWarps * 32, multi_ctas<T, kDuWarps>()) du_m
 }
 
 template <typename T, int W>
-static void multi_attrs() {
-  static bool done = false;  // once per process (the attribute is per function)
-  if (done) return;
-  cudaFuncSetAttribute(v_multi_kernel<T, W>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       static_cast<int>(multi_smem<T, W, kVWarps>()));
-  cudaFuncSetAttribute(du_multi_kernel<T, W>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       static_cast<int>(multi_smem<T, W, kDuWarps>()));
-  done = true;
+static cudaError_t multi_attrs() {
+  static PerDevice once;
+  return once([] {
+    const cudaError_t e = cudaFuncSetAttribute(v_multi_kernel<T, W>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               static_cast<int>(multi_smem<T, W, kVWarps>()));
+    if (e != cudaSuccess) return e;
+    return cudaFuncSetAttribute(du_multi_kernel<T, W>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                static_cast<int>(multi_smem<T, W, kDuWarps>()));
+  });
 }
 
 template <typename T, int W>
 static cudaError_t run_multi(const DevPlan &p, const T *panels, const T *vdata, T *xt, T *P, const T *X,
                              int64_t ldx, int nr, T *Y, int64_t ldy, int num_sms,
                              cudaStream_t s, cudaEvent_t *ev, int *launches) {
-  multi_attrs<T, W>();
+  cudaError_t e = multi_attrs<T, W>();
+  if (e != cudaSuccess) return e;
   int gp = static_cast<int>((p.n_src + 63) / 64);
   if (gp > 2048) gp = 2048;
   const bool overlap = may_overlap(sizeof(T) == 8, p.entries, W);
   int nl = 0;
   if (ev) cudaEventRecord(ev[0], s);
-  cudaError_t e = launch_pdl(overlap, permute_multi_kernel<T, W>, gp, kThreads, 0, s, X, ldx, nr, p.sinv0, p.n_src, xt, p.counter);
+  e = launch_pdl(overlap, permute_multi_kernel<T, W>, gp, kThreads, 0, s, X, ldx, nr, p.sinv0, p.n_src, xt, p.counter);
   nl++;
   if (ev) cudaEventRecord(ev[1], s);
   if (e == cudaSuccess && p.nmv > 0) {

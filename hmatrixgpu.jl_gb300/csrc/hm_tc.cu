@@ -71,6 +71,7 @@
 
 #include "hm_device.h"
 #include "hm_launch.cuh"
+#include "hm_per_device.h"
 
 namespace hm {
 
@@ -1025,13 +1026,13 @@ static size_t smem_bytes() {
 }
 int tc_width(int nr) { return nr <= 16 ? 16 : nr <= 32 ? 32 : 64; }
 
-static void tc_attrs() {
-  static bool done = false;
-  if (done) return;
-  cudaFuncSetAttribute(tc_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem_bytes<16>()));
-  cudaFuncSetAttribute(tc_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem_bytes<32>()));
-  cudaFuncSetAttribute(tc_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem_bytes<64>()));
-  done = true;
+template <int R>
+static cudaError_t tc_attrs() {
+  static PerDevice once;
+  return once([] {
+    return cudaFuncSetAttribute(tc_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                static_cast<int>(smem_bytes<R>()));
+  });
 }
 
 cudaError_t encode_xts_map(DevTc &t, int R) {
@@ -1069,6 +1070,8 @@ template <int R>
 static cudaError_t run_tc(const DevPlan &p, const DevTc &t, const float *X, int64_t ldx, int nr, float *Y, int64_t ldy,
                           cudaStream_t s, cudaEvent_t *ev, int *nl) {
   using Sh = TcShape<R>;
+  cudaError_t e = tc_attrs<R>();
+  if (e != cudaSuccess) return e;
   uint16_t *xts = t.xts[R / 32];
   int gp = static_cast<int>((p.n_src + 63) / 64);
   if (gp > 8192) gp = 8192;
@@ -1078,7 +1081,7 @@ static cudaError_t run_tc(const DevPlan &p, const DevTc &t, const float *X, int6
   unsigned *xmax = reinterpret_cast<unsigned *>(t.xscale);
   float *xs_inv = t.xscale + nm64;
   const dim3 gx(static_cast<unsigned>((p.n_src + kXmaxSpan - 1) / kXmaxSpan), static_cast<unsigned>((nr + 7) / 8));
-  cudaError_t e = launch_pdl(true, xmax_kernel, gx, 256, 0, s, X, ldx, nr, p.n_src, t.mcol0, t.nmem, xmax);
+  e = launch_pdl(true, xmax_kernel, gx, 256, 0, s, X, ldx, nr, p.n_src, t.mcol0, t.nmem, xmax);
   if (e == cudaSuccess)
     e = launch_pdl(true, permute_split_kernel<R>, gp, 256, 0, s, X, ldx, nr, p.sinv0, p.n_src, xts, p.counter + 2,
                    t.mcol0, t.nmem, xmax, xs_inv);
@@ -1151,7 +1154,6 @@ cudaError_t launch_matvec_tc(const DevPlan &p, const DevTc &t, const float *X, i
                              float *Y, int64_t ldy, cudaStream_t s, cudaEvent_t *ev, int *launches) {
   if (nr < 1 || nr > 64 || !t.xts[tc_width(nr) / 32] || !t.xscale || !t.mcol0 || t.nmem < 1)
     return cudaErrorInvalidValue;
-  tc_attrs();
   int nl = 0;
   const int w = tc_width(nr);
   const cudaError_t e = w == 64   ? run_tc<64>(p, t, X, ldx, nr, Y, ldy, s, ev, &nl)
