@@ -477,6 +477,8 @@ static bool overlaps(const T *x, int64_t n, const T *y, int64_t m) {
 template <typename T, bool COMP>
 static cudaError_t run(const DevPlan &p, const T *panels, const T *vdata, T *xt, const T *x, T *y,
                        int grid_v, int grid_du, cudaStream_t s, cudaEvent_t *ev, int *launches) {
+  if (launches) *launches = 0;
+  if (p.nunits == 0) return cudaSuccess;  // a shard without rows
   const bool overlap = may_overlap(sizeof(T) == 8, p.entries, 1);
   // x is read while y is written: not where they share memory (y = H y in place), which the
   // permuted copy allows
