@@ -1,7 +1,10 @@
 // Programmatic dependent launch, shared by the product kernels: a kernel of a
 // product may start while the one before it ends. It calls pdl_wait() before it
 // touches anything that earlier kernels write (or still read), which returns when
-// they are complete, and then pdl_trigger(), from which the next may start.
+// they are complete, and then pdl_trigger(), from which the next may start. What earlier
+// kernels write (x too: it may be the y of the product before) changes while the kernel is
+// already running, so it is not read through the read-only path: no __ldg, and no
+// __restrict__ from which the compiler would take it to be constant or move a load up.
 #pragma once
 #include <cuda_runtime.h>
 

@@ -50,6 +50,24 @@ __device__ __forceinline__ double2 ld_stream(const double2 *p) {
   return v;
 }
 
+// 16 bytes of XT, which the kernel before writes while this one may already run. Volatile, so that it
+// stays after pdl_wait(), like the loads of V beside it (left to the compiler, these loads
+// come later: V pass of the film of 2^20 points 539 us, 511 so).
+__device__ __forceinline__ float4 ld_x(const float4 *p) {
+  float4 v;
+  asm volatile("ld.global.v4.f32 {%0,%1,%2,%3}, [%4];"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+               : "l"(p));
+  return v;
+}
+__device__ __forceinline__ double2 ld_x(const double2 *p) {
+  double2 v;
+  asm volatile("ld.global.v2.f64 {%0,%1}, [%2];"
+               : "=d"(v.x), "=d"(v.y)
+               : "l"(p));
+  return v;
+}
+
 __device__ __forceinline__ float fma_(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 __device__ __forceinline__ double fma_(double a, double b, double c) { return __fma_rn(a, b, c); }
 
@@ -115,12 +133,12 @@ struct XSrc {
 // 16 bytes of the x region at entry e (a multiple of the vector), through the source map
 __device__ __forceinline__ float4 gather_x(const XSrc<float> &s, int32_t e) {
   const int4 i = __ldg(reinterpret_cast<const int4 *>(s.smap0 + e));
-  return make_float4(i.x >= 0 ? __ldg(s.x + i.x) : 0.0f, i.y >= 0 ? __ldg(s.x + i.y) : 0.0f,
-                     i.z >= 0 ? __ldg(s.x + i.z) : 0.0f, i.w >= 0 ? __ldg(s.x + i.w) : 0.0f);
+  return make_float4(i.x >= 0 ? s.x[i.x] : 0.0f, i.y >= 0 ? s.x[i.y] : 0.0f,
+                     i.z >= 0 ? s.x[i.z] : 0.0f, i.w >= 0 ? s.x[i.w] : 0.0f);
 }
 __device__ __forceinline__ double2 gather_x(const XSrc<double> &s, int32_t e) {
   const int2 i = __ldg(reinterpret_cast<const int2 *>(s.smap0 + e));
-  return make_double2(i.x >= 0 ? __ldg(s.x + i.x) : 0.0, i.y >= 0 ? __ldg(s.x + i.y) : 0.0);
+  return make_double2(i.x >= 0 ? s.x[i.x] : 0.0, i.y >= 0 ? s.x[i.y] : 0.0);
 }
 
 // ---------------------------------------------------------------------------
@@ -128,9 +146,8 @@ __device__ __forceinline__ double2 gather_x(const XSrc<double> &s, int32_t e) {
 // Also re-arms the unit ticket of the near/U pass.
 // ---------------------------------------------------------------------------
 template <typename T>
-__global__ void permute_x_kernel(const T *__restrict__ x, const int32_t *__restrict__ smap0,
-                                 int64_t x_len, T *__restrict__ xt,
-                                 int32_t *__restrict__ counter) {
+__global__ void permute_x_kernel(const T *x, const int32_t *__restrict__ smap0, int64_t x_len, T *xt,
+                                 int32_t *counter) {
   int64_t j = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
   pdl_wait();
   pdl_trigger();
@@ -156,7 +173,7 @@ __global__ void permute_x_kernel(const T *__restrict__ x, const int32_t *__restr
 // Six CTAs per SM (40 registers) and four loads in flight per lane: the pass
 // is bound by memory latency, like the near/U pass.
 template <typename T>
-__device__ __forceinline__ void v_unit(const T *__restrict__ V, const VUnit U, T *__restrict__ xt, int lane) {
+__device__ __forceinline__ void v_unit(const T *__restrict__ V, const VUnit U, T *xt, int lane) {
   using VT = typename Vec16<T>::type;
   constexpr int VEC = Vec16<T>::N;
   const int g = U.lanes, slot = lane / g, sub = lane - slot * g, per = 32 / g;
@@ -171,7 +188,7 @@ __device__ __forceinline__ void v_unit(const T *__restrict__ V, const VUnit U, T
       for (; p + 3 * g < nv; p += 4 * g) {  // four 16-byte loads of V in flight per lane
         VT a0 = ld_stream(row + p), a1 = ld_stream(row + p + g);
         VT a2 = ld_stream(row + p + 2 * g), a3 = ld_stream(row + p + 3 * g);
-        VT b0 = __ldg(X + p), b1 = __ldg(X + p + g), b2 = __ldg(X + p + 2 * g), b3 = __ldg(X + p + 3 * g);
+        VT b0 = ld_x(X + p), b1 = ld_x(X + p + g), b2 = ld_x(X + p + 2 * g), b3 = ld_x(X + p + 3 * g);
         const T *ea0 = reinterpret_cast<const T *>(&a0), *eb0 = reinterpret_cast<const T *>(&b0);
         const T *ea1 = reinterpret_cast<const T *>(&a1), *eb1 = reinterpret_cast<const T *>(&b1);
         const T *ea2 = reinterpret_cast<const T *>(&a2), *eb2 = reinterpret_cast<const T *>(&b2);
@@ -187,7 +204,7 @@ __device__ __forceinline__ void v_unit(const T *__restrict__ V, const VUnit U, T
       }
       for (; p + g < nv; p += 2 * g) {
         VT a0 = ld_stream(row + p), a1 = ld_stream(row + p + g);
-        VT b0 = __ldg(X + p), b1 = __ldg(X + p + g);
+        VT b0 = ld_x(X + p), b1 = ld_x(X + p + g);
         const T *ea0 = reinterpret_cast<const T *>(&a0), *eb0 = reinterpret_cast<const T *>(&b0);
         const T *ea1 = reinterpret_cast<const T *>(&a1), *eb1 = reinterpret_cast<const T *>(&b1);
 #pragma unroll
@@ -197,7 +214,7 @@ __device__ __forceinline__ void v_unit(const T *__restrict__ V, const VUnit U, T
       }
       if (p < nv) {
         VT a0 = ld_stream(row + p);
-        VT b0 = __ldg(X + p);
+        VT b0 = ld_x(X + p);
         const T *ea0 = reinterpret_cast<const T *>(&a0), *eb0 = reinterpret_cast<const T *>(&b0);
 #pragma unroll
         for (int q = 0; q < VEC; q++) acc = fma_(ea0[q], eb0[q], acc);
@@ -211,7 +228,7 @@ __device__ __forceinline__ void v_unit(const T *__restrict__ V, const VUnit U, T
 // The same unit with x read through the source map (the sums in the same order).
 template <typename T>
 __device__ __forceinline__ void v_unit_direct(const T *__restrict__ V, const VUnit U, const XSrc<T> &src,
-                                              T *__restrict__ xt, int lane) {
+                                              T *xt, int lane) {
   using VT = typename Vec16<T>::type;
   constexpr int VEC = Vec16<T>::N;
   const int g = U.lanes, slot = lane / g, sub = lane - slot * g, per = 32 / g;
@@ -250,7 +267,7 @@ template <typename T>
 __global__ void __launch_bounds__(kThreads, 6) v_pass_kernel(const T *__restrict__ V,
                                                           const VUnit *__restrict__ units,
                                                           const int32_t *__restrict__ warp_begin,
-                                                          T *__restrict__ xt) {
+                                                          T *xt) {
   const int warp = static_cast<int>((blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x) >> 5);
   const int lane = threadIdx.x & 31;
   const int u0 = warp_begin[warp], u1 = warp_begin[warp + 1];
@@ -263,8 +280,7 @@ __global__ void __launch_bounds__(kThreads, 6) v_pass_kernel(const T *__restrict
 template <typename T>
 __global__ void __launch_bounds__(kThreads, 6) v_pass_dyn_kernel(const T *__restrict__ V,
                                                               const VUnit *__restrict__ units,
-                                                              int32_t nunits, T *__restrict__ xt,
-                                                              int32_t *__restrict__ ticket) {
+                                                              int32_t nunits, T *xt, int32_t *ticket) {
   const int lane = threadIdx.x & 31;
   const int nwarps = static_cast<int>((gridDim.x * blockDim.x) >> 5);
   int u = static_cast<int>((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
@@ -283,7 +299,7 @@ __global__ void __launch_bounds__(kThreads, 6) v_pass_dyn_kernel(const T *__rest
 template <typename T>
 __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 6 : 5) v_pass_direct_kernel(const T *__restrict__ V,
                                                                 const VUnit *__restrict__ units, int32_t nunits,
-                                                                const XSrc<T> src, T *__restrict__ xt) {
+                                                                const XSrc<T> src, T *xt) {
   const int u = static_cast<int>((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
   if (u >= nunits) return;
   const VUnit U = units[u];

@@ -51,9 +51,9 @@ __device__ constexpr int kTicket[kTickets] = {0, 1, 8};
 // whole; the x-region rows that no source index maps to stay zero (every pass
 // width has its own XT, zeroed once). Also re-arms the ticket counters.
 template <typename T, int W>
-__global__ void permute_multi_kernel(const T *__restrict__ X, int64_t ldx, int nr,
+__global__ void permute_multi_kernel(const T *X, int64_t ldx, int nr,
                                      const int32_t *__restrict__ sinv0, int64_t n_src,
-                                     T *__restrict__ xt, int32_t *__restrict__ counter) {
+                                     T *xt, int32_t *counter) {
   __shared__ T tile[64][W + 1];
   pdl_wait();
   pdl_trigger();
@@ -217,7 +217,7 @@ struct Sums<float, TR, TN> {
 // stage, one stage ahead. `buf`: the warp's two stages.
 template <typename T, int W, int MT, typename RowOf>
 __device__ __forceinline__ void slice_product(const T *A, int64_t lda, int m, int ncols, int first, int step,
-                                              const T *__restrict__ xt, unsigned char *buf, RowOf row_of,
+                                              const T *xt, unsigned char *buf, RowOf row_of,
                                               Sums<T, LaneTile<T, W, MT>::TR, LaneTile<T, W, MT>::TN> &acc) {
   constexpr int SETS = sum_sets<T, W>();
   Sums<T, LaneTile<T, W, MT>::TR, LaneTile<T, W, MT>::TN> set[SETS];
@@ -353,7 +353,7 @@ template <typename T, int W>
 __global__ void __launch_bounds__(kVWarps * 32, multi_ctas<T, kVWarps>()) v_multi_kernel(const T *__restrict__ V,
                                                                             const MVItem *__restrict__ items,
                                                                             int32_t nbig, int32_t nitems,
-                                                                            T *__restrict__ xt, T *__restrict__ P,
+                                                                            T *xt, T *P,
                                                                             int32_t *counter) {
   extern __shared__ __align__(16) unsigned char dyn_smem[];
   __shared__ int32_t s_ticket;
@@ -407,8 +407,7 @@ __global__ void __launch_bounds__(kVWarps * 32, multi_ctas<T, kVWarps>()) v_mult
 
 // t rows of cut groups: pieces summed in order (one warp per row, lane = RHS).
 template <typename T, int W>
-__global__ void reduce_multi_kernel(const MVReduce *__restrict__ red, int32_t nred, const T *__restrict__ P,
-                                    T *__restrict__ xt) {
+__global__ void reduce_multi_kernel(const MVReduce *__restrict__ red, int32_t nred, const T *P, T *xt) {
   const int lane = threadIdx.x & 31;
   pdl_wait();
   pdl_trigger();

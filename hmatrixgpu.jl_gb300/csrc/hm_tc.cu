@@ -745,10 +745,18 @@ __global__ void __launch_bounds__(TcShape<R>::kThreads, 1) tc_kernel(const __gri
       for (int c = 0; c < H; c++) v[c] *= f;
       if (I.kind == 0) {
         float *yr = a.y + yrow;
-        const float *xs = a.xs_inv + mem * kTcMaxRhs + keep;  // its member's
+        const float4 *xs = reinterpret_cast<const float4 *>(a.xs_inv + mem * kTcMaxRhs + keep);  // its member's
+#pragma unroll
+        for (int q = 0; q < H / 4; q++) {
+          const float4 g = xs[q];
+          v[4 * q] *= g.x;
+          v[4 * q + 1] *= g.y;
+          v[4 * q + 2] *= g.z;
+          v[4 * q + 3] *= g.w;
+        }
 #pragma unroll
         for (int c = 0; c < H; c++)
-          if (keep + c < a.nr) yr[(keep + c) * a.ldy] = v[c] * __ldg(xs + c);
+          if (keep + c < a.nr) yr[(keep + c) * a.ldy] = v[c];
       } else if (I.kind == 1) {
         uint4 *dst = reinterpret_cast<uint4 *>(a.xts_out + static_cast<int64_t>(I.out + row) * (2 * R)) + keep / 8;
 #pragma unroll
@@ -791,8 +799,8 @@ __device__ __forceinline__ int member_of(const int64_t *col0, int nmem, int64_t 
 // kXmaxSpan), its warp w right-hand side 8 y + w: coalesced loads along the
 // indices, eight in flight per lane, one atomic per member met.
 constexpr int kXmaxSpan = 2048;
-__global__ void xmax_kernel(const float *__restrict__ X, int64_t ldx, int nr, int64_t n_src,
-                            const int64_t *__restrict__ col0, int nmem, unsigned *__restrict__ xmax) {
+__global__ void xmax_kernel(const float *X, int64_t ldx, int nr, int64_t n_src,
+                            const int64_t *__restrict__ col0, int nmem, unsigned *xmax) {
   const int lane = threadIdx.x & 31;
   const int r = blockIdx.y * (blockDim.x >> 5) + (threadIdx.x >> 5);
   pdl_wait();  // x is there, the maxima are cleared
@@ -825,12 +833,12 @@ __global__ void xmax_kernel(const float *__restrict__ X, int64_t ldx, int nr, in
 // written whole; x-region rows that no source index maps to stay zero from the allocation.
 // Also writes 1 / sigma per member and right-hand side, and re-arms the two item tickets.
 template <int R>
-__global__ void __launch_bounds__(256) permute_split_kernel(const float *__restrict__ X, int64_t ldx, int nr,
+__global__ void __launch_bounds__(256) permute_split_kernel(const float *X, int64_t ldx, int nr,
                                                             const int32_t *__restrict__ sinv0, int64_t n_src,
-                                                            uint16_t *__restrict__ xts, int32_t *__restrict__ tickets,
+                                                            uint16_t *xts, int32_t *tickets,
                                                             const int64_t *__restrict__ col0, int nmem,
-                                                            const unsigned *__restrict__ xmax,
-                                                            float *__restrict__ xs_inv) {
+                                                            const unsigned *xmax,
+                                                            float *xs_inv) {
   __shared__ float tile[64][R + 1];
   __shared__ float s0[R];  // sigma of the block's first member
   __shared__ int mem[64];
@@ -880,8 +888,7 @@ __global__ void __launch_bounds__(256) permute_split_kernel(const float *__restr
 // summed in order; one warp per row, lane = right-hand side (and lane + 32 in
 // a 64-wide pass).
 template <int R>
-__global__ void reduce_split_kernel(const MVReduce *__restrict__ red, int32_t nred, const float *__restrict__ P,
-                                    uint16_t *__restrict__ xts) {
+__global__ void reduce_split_kernel(const MVReduce *__restrict__ red, int32_t nred, const float *P, uint16_t *xts) {
   const int lane = threadIdx.x & 31;
   pdl_wait();
   pdl_trigger();
