@@ -547,12 +547,15 @@ extern "C" int hmgpu_matvec(hmgpu_hmatrix *h, const void *x, void *y, int64_t nr
   // The one-time contents of scratch that this call allocates: on the caller's stream, or, while
   // that is captured, on a stream of its own and waited for. In the graph they would run with
   // its replays only, and a product before the first replay would read scratch without contents.
-  auto first_fill = [](cudaStream_t on, auto fill) -> int {
+  auto capturing = [s]() {
     cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(on, &st) != cudaSuccess) cudaGetLastError();  // the launches that follow fail, too
+    if (cudaStreamIsCapturing(s, &st) != cudaSuccess) cudaGetLastError();  // the launches that follow fail, too
+    return st != cudaStreamCaptureStatusNone;
+  };
+  auto first_fill = [&](auto fill) -> int {
     cudaError_t e = cudaSuccess;
-    if (st == cudaStreamCaptureStatusNone) {
-      e = fill(on);
+    if (!capturing()) {
+      e = fill(s);
     } else {
       cudaStream_t own = nullptr;
       e = cudaStreamCreateWithFlags(&own, cudaStreamNonBlocking);
@@ -573,32 +576,17 @@ extern "C" int hmgpu_matvec(hmgpu_hmatrix *h, const void *x, void *y, int64_t nr
     if (tc && !H.tc.prow) {
       const size_t sb = 2 * static_cast<size_t>(H.tc.nmem) * hm::kTcMaxRhs * sizeof(float);
       if ((rc = H.dalloc(reinterpret_cast<void **>(&H.tc.xscale), sb)) ||
-          (rc = first_fill(s, [&](cudaStream_t q) { return cudaMemsetAsync(H.tc.xscale, 0, sb, q); })) ||
+          (rc = first_fill([&](cudaStream_t q) { return cudaMemsetAsync(H.tc.xscale, 0, sb, q); })) ||
           (rc = H.dalloc(reinterpret_cast<void **>(&H.tc.prow),
                          std::max<int64_t>(H.plan.p_rows, 1) * hm::kTcMaxRhs * 4)))
         return rc;
-    }
-    // the XTS of every width that this call's passes have
-    for (int64_t left = nrhs; tc && left > 0; left -= std::min<int64_t>(left, per)) {
-      const int w = hm::tc_width(static_cast<int>(std::min<int64_t>(left, per)));
-      uint16_t *&xts = H.tc.xts[w / 32];
-      if (xts) continue;
-      const int64_t xb = H.plan.xt_len * 2 * w * 2;
-      if ((rc = H.dalloc(reinterpret_cast<void **>(&xts), xb))) return rc;
-      rc = first_fill(s, [&](cudaStream_t q) { return cudaMemsetAsync(xts, 0, xb, q); });
-      if (cudaError_t e = rc ? cudaSuccess : hm::encode_xts_map(H.tc, w)) rc = hm::cuda_fail(e, "tensor map of XTS");
-      if (rc) {
-        H.dfree(xts);
-        xts = nullptr;
-        return rc;
-      }
     }
     if (!tc && !H.dp.mcolmap) {
       int64_t ncm = 0;
       for (const hm::TileDesc &d : H.plan.tiles) ncm += d.ncols;
       int32_t *map = nullptr;
       if ((rc = H.dalloc(reinterpret_cast<void **>(&map), ncm * sizeof(int32_t))) ||
-          (rc = first_fill(s, [&](cudaStream_t q) {
+          (rc = first_fill([&](cudaStream_t q) {
              return hm::launch_colmap(H.dp.tiles, H.dp.ntiles, H.dp.segs, H.dp.mcol0, map, q);
            })))
         return rc;
@@ -610,31 +598,57 @@ extern "C" int hmgpu_matvec(hmgpu_hmatrix *h, const void *x, void *y, int64_t nr
     const uintptr_t x0 = reinterpret_cast<uintptr_t>(x), y0 = reinterpret_cast<uintptr_t>(y);
     const bool shared = x0 < y0 + ((nrhs - 1) * ldy + H.bs.m) * es && y0 < x0 + ((nrhs - 1) * ldx + H.bs.n) * es &&
                         !(x == y && ldx == ldy);
+    // Each pass width has its own XT or XTS (zeroed once): rows that no pass writes (padding, the
+    // zero row) must read as zero in that width's layout.
+    auto xt_of = [&](int w) -> void *& {
+      return w == per ? H.xt_multi : H.xt_multi_w[w == 4 ? 0 : w == 8 ? 1 : 2];
+    };
+    auto have = [&](int w) { return (tc ? static_cast<void *>(H.tc.xts[w / 32]) : xt_of(w)) != nullptr; };
     for (int64_t k0 = 0, nr = 0; k0 < nrhs; k0 += nr) {
       cudaEvent_t *ev;
       if ((rc = next_events(&ev))) return rc;
       nr = tc || shared ? std::min<int64_t>(per, nrhs - k0)
                         : hm::multi_pass_columns(f64, nrhs - k0, H.dp.entries, H.num_sms);
+      int w = tc ? hm::tc_width(static_cast<int>(nr)) : hm::multi_width(f64, static_cast<int>(nr));
+      if (!have(w) && capturing()) {
+        // most captures forbid allocation: the pass takes a width that is there, a wider one or
+        // else the widest with fewer columns
+        int v = w;
+        while (v <= per && !have(v)) v *= 2;
+        if (v > per)
+          for (v = w / 2; v >= (tc ? 16 : 4) && !have(v);) v /= 2;
+        if (v >= (tc ? 16 : 4)) {
+          w = v;
+          nr = std::min<int64_t>(nr, w);
+        }
+      }
       int nl = 0;
       cudaError_t e;
-      if (tc)  // scaled FP16 (hi, lo) splits on the tensor cores
-        e = hm::launch_matvec_tc(H.dp, H.tc, reinterpret_cast<const float *>(static_cast<const char *>(x) + k0 * ldx * es),
+      if (tc) {  // scaled FP16 (hi, lo) splits on the tensor cores
+        if (uint16_t *&xts = H.tc.xts[w / 32]; !xts) {
+          const int64_t xb = H.plan.xt_len * 2 * w * 2;
+          if ((rc = H.dalloc(reinterpret_cast<void **>(&xts), xb))) return rc;
+          rc = first_fill([&](cudaStream_t q) { return cudaMemsetAsync(xts, 0, xb, q); });
+          if (cudaError_t em = rc ? cudaSuccess : hm::encode_xts_map(H.tc, w)) rc = hm::cuda_fail(em, "tensor map of XTS");
+          if (rc) {
+            H.dfree(xts);
+            xts = nullptr;
+            return rc;
+          }
+        }
+        e = hm::launch_matvec_tc(H.dp, H.tc, w, reinterpret_cast<const float *>(static_cast<const char *>(x) + k0 * ldx * es),
                                  ldx, static_cast<int>(nr),
                                  reinterpret_cast<float *>(static_cast<char *>(y) + k0 * ldy * es), ldy,
                                  s, ev, &nl);
-      else {
-        // each pass width has its own XT (zeroed once): rows that no pass
-        // writes (padding, the zero row) must read as zero in that width's layout
-        const int w = hm::multi_width(f64, static_cast<int>(nr));
-        void *&xt = w == per ? H.xt_multi : H.xt_multi_w[w == 4 ? 0 : w == 8 ? 1 : 2];
-        if (!xt) {
+      } else {
+        if (void *&xt = xt_of(w); !xt) {
           void *t = nullptr;
           const int64_t xb = H.plan.xt_len * w * es;
-          if ((rc = H.dalloc(&t, xb)) || (rc = first_fill(s, [&](cudaStream_t q) { return cudaMemsetAsync(t, 0, xb, q); })))
+          if ((rc = H.dalloc(&t, xb)) || (rc = first_fill([&](cudaStream_t q) { return cudaMemsetAsync(t, 0, xb, q); })))
             return rc;
           xt = t;
         }
-        e = hm::launch_matvec_multi(f64, H.dp, H.panels, H.vdata, xt, H.p_multi,
+        e = hm::launch_matvec_multi(f64, H.dp, w, H.panels, H.vdata, xt_of(w), H.p_multi,
                                     static_cast<const char *>(x) + k0 * ldx * es, ldx, static_cast<int>(nr),
                                     static_cast<char *>(y) + k0 * ldy * es, ldy, H.num_sms, s, ev, &nl);
       }

@@ -120,16 +120,17 @@ cudaError_t launch_tc_scales(const VGroup *groups, int64_t ngroups, const float 
 cudaError_t launch_pack_tc(const TcPack *jobs, int64_t njobs, const float *src, void *adata, const int32_t *colmap,
                            const float *colsc, const float *nu, const float *gam, cudaStream_t s);
 // permutation + split of X, V pass, reduction of pieces, near/U pass over
-// nr <= 64 columns (the XTS of their width must exist); ev (optional) gets 4
+// nr <= width columns, width 16, 32 or 64 (its XTS must exist); ev (optional) gets 4
 // events as launch_matvec_multi.
-cudaError_t launch_matvec_tc(const DevPlan &p, const DevTc &t, const float *X, int64_t ldx, int nr,
+cudaError_t launch_matvec_tc(const DevPlan &p, const DevTc &t, int width, const float *X, int64_t ldx, int nr,
                              float *Y, int64_t ldy, cudaStream_t s, cudaEvent_t *ev, int *launches);
 
 // XT row of every tile column (tile t's at colmap[col0[t]]...), from the segments.
 cudaError_t launch_colmap(const TileDesc *tiles, int32_t ntiles, const Seg *segs, const int64_t *col0, int32_t *colmap,
                           cudaStream_t s);
 // P: partial rows of cut V groups (p_rows x rhs_per_pass() values).
-cudaError_t launch_matvec_multi(bool f64, const DevPlan &p, const void *panels, const void *vdata,
+// xt: the XT of that width, nr <= width columns.
+cudaError_t launch_matvec_multi(bool f64, const DevPlan &p, int width, const void *panels, const void *vdata,
                                 void *xt, void *P, const void *X, int64_t ldx, int nr, void *Y,
                                 int64_t ldy, int num_sms, cudaStream_t s, cudaEvent_t *ev,
                                 int *launches);

@@ -588,30 +588,32 @@ int multi_pass_columns(bool f64, int64_t left, int64_t entries, int num_sms) {
 }
 
 template <typename T>
-static cudaError_t run_multi_w(const DevPlan &p, const T *panels, const T *vdata, T *xt, T *P, const T *X,
+static cudaError_t run_multi_w(const DevPlan &p, int width, const T *panels, const T *vdata, T *xt, T *P, const T *X,
                                int64_t ldx, int nr, T *Y, int64_t ldy, int num_sms, cudaStream_t s,
                                cudaEvent_t *ev, int *launches) {
-  switch (multi_width(sizeof(T) == 8, nr)) {
+  if (nr > width) return cudaErrorInvalidValue;
+  switch (width) {
     case 4:
       if constexpr (sizeof(T) == 8)
         return run_multi<T, 4>(p, panels, vdata, xt, P, X, ldx, nr, Y, ldy, num_sms, s, ev, launches);
       return cudaErrorInvalidValue;
     case 8: return run_multi<T, 8>(p, panels, vdata, xt, P, X, ldx, nr, Y, ldy, num_sms, s, ev, launches);
     case 16: return run_multi<T, 16>(p, panels, vdata, xt, P, X, ldx, nr, Y, ldy, num_sms, s, ev, launches);
-    default: return run_multi<T, kRhs>(p, panels, vdata, xt, P, X, ldx, nr, Y, ldy, num_sms, s, ev, launches);
+    case kRhs: return run_multi<T, kRhs>(p, panels, vdata, xt, P, X, ldx, nr, Y, ldy, num_sms, s, ev, launches);
+    default: return cudaErrorInvalidValue;
   }
 }
 
-cudaError_t launch_matvec_multi(bool f64, const DevPlan &p, const void *panels, const void *vdata,
+cudaError_t launch_matvec_multi(bool f64, const DevPlan &p, int width, const void *panels, const void *vdata,
                                 void *xt, void *P, const void *X, int64_t ldx, int nr, void *Y,
                                 int64_t ldy, int num_sms, cudaStream_t s, cudaEvent_t *ev,
                                 int *launches) {
   if (f64)
-    return run_multi_w<double>(p, static_cast<const double *>(panels), static_cast<const double *>(vdata),
+    return run_multi_w<double>(p, width, static_cast<const double *>(panels), static_cast<const double *>(vdata),
                              static_cast<double *>(xt), static_cast<double *>(P),
                              static_cast<const double *>(X), ldx, nr, static_cast<double *>(Y), ldy,
                              num_sms, s, ev, launches);
-  return run_multi_w<float>(p, static_cast<const float *>(panels), static_cast<const float *>(vdata),
+  return run_multi_w<float>(p, width, static_cast<const float *>(panels), static_cast<const float *>(vdata),
                           static_cast<float *>(xt), static_cast<float *>(P), static_cast<const float *>(X),
                           ldx, nr, static_cast<float *>(Y), ldy, num_sms, s, ev, launches);
 }

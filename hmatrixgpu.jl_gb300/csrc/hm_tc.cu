@@ -1157,15 +1157,15 @@ cudaError_t launch_pack_tc(const TcPack *jobs, int64_t njobs, const float *src, 
   return cudaGetLastError();
 }
 
-cudaError_t launch_matvec_tc(const DevPlan &p, const DevTc &t, const float *X, int64_t ldx, int nr,
+cudaError_t launch_matvec_tc(const DevPlan &p, const DevTc &t, int width, const float *X, int64_t ldx, int nr,
                              float *Y, int64_t ldy, cudaStream_t s, cudaEvent_t *ev, int *launches) {
-  if (nr < 1 || nr > 64 || !t.xts[tc_width(nr) / 32] || !t.xscale || !t.mcol0 || t.nmem < 1)
+  if ((width != 16 && width != 32 && width != 64) || nr < 1 || nr > width || !t.xts[width / 32] || !t.xscale ||
+      !t.mcol0 || t.nmem < 1)
     return cudaErrorInvalidValue;
   int nl = 0;
-  const int w = tc_width(nr);
-  const cudaError_t e = w == 64   ? run_tc<64>(p, t, X, ldx, nr, Y, ldy, s, ev, &nl)
-                        : w == 32 ? run_tc<32>(p, t, X, ldx, nr, Y, ldy, s, ev, &nl)
-                                  : run_tc<16>(p, t, X, ldx, nr, Y, ldy, s, ev, &nl);
+  const cudaError_t e = width == 64   ? run_tc<64>(p, t, X, ldx, nr, Y, ldy, s, ev, &nl)
+                        : width == 32 ? run_tc<32>(p, t, X, ldx, nr, Y, ldy, s, ev, &nl)
+                                      : run_tc<16>(p, t, X, ldx, nr, Y, ldy, s, ev, &nl);
   if (launches) *launches = nl;
   return e != cudaSuccess ? e : cudaGetLastError();
 }
