@@ -677,7 +677,7 @@ def mul_(y, H, x, stream=None):
         if x.dtype != want or y.dtype != want:
             raise TypeError(f"x and y must be {want} for this H-matrix")
         two = x.dim() == 2
-        nrhs = x.shape[1] if two else 1
+        nrhs = 1 if x.dim() == 1 else x.shape[1]
         if x.shape[0] != n or y.shape[0] != m or (two and y.shape[1] != nrhs):
             raise ValueError("dimension mismatch")
         if two and (x.stride(0) != 1 or y.stride(0) != 1):
