@@ -111,7 +111,7 @@ struct VUnit {
   int32_t x_off;   // XT offset (aligned) matching stored position 0
   int32_t t_off;   // XT offset of the first output
   int32_t lanes;   // lanes per row (power of two <= 32)
-  int32_t pad;
+  int32_t sums;    // sums per lane, 1 or 2: its vectors in turn
 };
 static_assert(sizeof(VUnit) == 32, "VUnit layout");
 

@@ -173,6 +173,15 @@ __global__ void permute_x_kernel(const T *x, const int32_t *__restrict__ smap0, 
 // Six CTAs per SM (40 registers) and four loads in flight per lane: the pass
 // is bound by memory latency, like the near/U pass.
 template <typename T>
+__device__ __forceinline__ void add_vec(T &acc, const typename Vec16<T>::type &a, const typename Vec16<T>::type &b) {
+  const T *ea = reinterpret_cast<const T *>(&a), *eb = reinterpret_cast<const T *>(&b);
+#pragma unroll
+  for (int q = 0; q < Vec16<T>::N; q++) acc = fma_(ea[q], eb[q], acc);
+}
+
+// The lane's vectors go to its SUMS sums in turn, so that a row of half as many lanes with two
+// sums each adds the same numbers in the same order.
+template <typename T, int SUMS>
 __device__ __forceinline__ void v_unit(const T *__restrict__ V, const VUnit U, T *xt, int lane) {
   using VT = typename Vec16<T>::type;
   constexpr int VEC = Vec16<T>::N;
@@ -181,7 +190,7 @@ __device__ __forceinline__ void v_unit(const T *__restrict__ V, const VUnit U, T
   const VT *X = reinterpret_cast<const VT *>(xt + U.x_off);
   for (int k0 = 0; k0 < U.nrows; k0 += per) {
     const int k = k0 + slot;
-    T acc = T(0);
+    T acc[2] = {T(0), T(0)};
     if (k < U.nrows) {
       const VT *row = reinterpret_cast<const VT *>(V + U.v_off + static_cast<int64_t>(k) * U.stride);
       int p = sub;
@@ -189,44 +198,31 @@ __device__ __forceinline__ void v_unit(const T *__restrict__ V, const VUnit U, T
         VT a0 = ld_stream(row + p), a1 = ld_stream(row + p + g);
         VT a2 = ld_stream(row + p + 2 * g), a3 = ld_stream(row + p + 3 * g);
         VT b0 = ld_x(X + p), b1 = ld_x(X + p + g), b2 = ld_x(X + p + 2 * g), b3 = ld_x(X + p + 3 * g);
-        const T *ea0 = reinterpret_cast<const T *>(&a0), *eb0 = reinterpret_cast<const T *>(&b0);
-        const T *ea1 = reinterpret_cast<const T *>(&a1), *eb1 = reinterpret_cast<const T *>(&b1);
-        const T *ea2 = reinterpret_cast<const T *>(&a2), *eb2 = reinterpret_cast<const T *>(&b2);
-        const T *ea3 = reinterpret_cast<const T *>(&a3), *eb3 = reinterpret_cast<const T *>(&b3);
-#pragma unroll
-        for (int q = 0; q < VEC; q++) acc = fma_(ea0[q], eb0[q], acc);
-#pragma unroll
-        for (int q = 0; q < VEC; q++) acc = fma_(ea1[q], eb1[q], acc);
-#pragma unroll
-        for (int q = 0; q < VEC; q++) acc = fma_(ea2[q], eb2[q], acc);
-#pragma unroll
-        for (int q = 0; q < VEC; q++) acc = fma_(ea3[q], eb3[q], acc);
+        add_vec<T>(acc[0], a0, b0);
+        add_vec<T>(acc[SUMS - 1], a1, b1);
+        add_vec<T>(acc[0], a2, b2);
+        add_vec<T>(acc[SUMS - 1], a3, b3);
       }
       for (; p + g < nv; p += 2 * g) {
         VT a0 = ld_stream(row + p), a1 = ld_stream(row + p + g);
         VT b0 = ld_x(X + p), b1 = ld_x(X + p + g);
-        const T *ea0 = reinterpret_cast<const T *>(&a0), *eb0 = reinterpret_cast<const T *>(&b0);
-        const T *ea1 = reinterpret_cast<const T *>(&a1), *eb1 = reinterpret_cast<const T *>(&b1);
-#pragma unroll
-        for (int q = 0; q < VEC; q++) acc = fma_(ea0[q], eb0[q], acc);
-#pragma unroll
-        for (int q = 0; q < VEC; q++) acc = fma_(ea1[q], eb1[q], acc);
+        add_vec<T>(acc[0], a0, b0);
+        add_vec<T>(acc[SUMS - 1], a1, b1);
       }
       if (p < nv) {
         VT a0 = ld_stream(row + p);
         VT b0 = ld_x(X + p);
-        const T *ea0 = reinterpret_cast<const T *>(&a0), *eb0 = reinterpret_cast<const T *>(&b0);
-#pragma unroll
-        for (int q = 0; q < VEC; q++) acc = fma_(ea0[q], eb0[q], acc);
+        add_vec<T>(acc[0], a0, b0);
       }
     }
-    for (int o = g >> 1; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if (sub == 0 && k < U.nrows) xt[U.t_off + k] = acc;
+    T sum = SUMS == 2 ? acc[0] + acc[1] : acc[0];
+    for (int o = g >> 1; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    if (sub == 0 && k < U.nrows) xt[U.t_off + k] = sum;
   }
 }
 
 // The same unit with x read through the source map (the sums in the same order).
-template <typename T>
+template <typename T, int SUMS>
 __device__ __forceinline__ void v_unit_direct(const T *__restrict__ V, const VUnit U, const XSrc<T> &src,
                                               T *xt, int lane) {
   using VT = typename Vec16<T>::type;
@@ -235,7 +231,7 @@ __device__ __forceinline__ void v_unit_direct(const T *__restrict__ V, const VUn
   const int nv = U.stride / VEC;
   for (int k0 = 0; k0 < U.nrows; k0 += per) {
     const int k = k0 + slot;
-    T acc = T(0);
+    T acc[2] = {T(0), T(0)};
     if (k < U.nrows) {
       const VT *row = reinterpret_cast<const VT *>(V + U.v_off + static_cast<int64_t>(k) * U.stride);
       // n vectors in flight, and no FMA that is predicated off (the FP64 pipe would be as busy with it)
@@ -247,20 +243,26 @@ __device__ __forceinline__ void v_unit_direct(const T *__restrict__ V, const VUn
           b[z] = gather_x(src, U.x_off + (p + z * g) * VEC);
         }
 #pragma unroll
-        for (int z = 0; z < n.value; z++) {
-          const T *ea = reinterpret_cast<const T *>(&a[z]), *eb = reinterpret_cast<const T *>(&b[z]);
-#pragma unroll
-          for (int q = 0; q < VEC; q++) acc = fma_(ea[q], eb[q], acc);
-        }
+        for (int z = 0; z < n.value; z++) add_vec<T>(acc[z % SUMS], a[z], b[z]);
       };
       int p = sub;
       for (; p + 3 * g < nv; p += 4 * g) some(std::integral_constant<int, 4>(), p);
       for (; p + g < nv; p += 2 * g) some(std::integral_constant<int, 2>(), p);
       if (p < nv) some(std::integral_constant<int, 1>(), p);
     }
-    for (int o = g >> 1; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if (sub == 0 && k < U.nrows) xt[U.t_off + k] = acc;
+    T sum = SUMS == 2 ? acc[0] + acc[1] : acc[0];
+    for (int o = g >> 1; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    if (sub == 0 && k < U.nrows) xt[U.t_off + k] = sum;
   }
+}
+
+// FP64 lanes have one sum.
+template <typename T>
+__device__ __forceinline__ void v_unit_any(const T *__restrict__ V, const VUnit U, T *xt, int lane) {
+  if (sizeof(T) == 4 && U.sums == 2)
+    v_unit<T, 2>(V, U, xt, lane);
+  else
+    v_unit<T, 1>(V, U, xt, lane);
 }
 
 template <typename T>
@@ -274,7 +276,7 @@ __global__ void __launch_bounds__(kThreads, 6) v_pass_kernel(const T *__restrict
   if (u0 >= u1) return;
   pdl_wait();  // XT holds the permuted x
   pdl_trigger();
-  for (int u = u0; u < u1; u++) v_unit(V, units[u], xt, lane);
+  for (int u = u0; u < u1; u++) v_unit_any(V, units[u], xt, lane);
 }
 
 template <typename T>
@@ -290,7 +292,7 @@ __global__ void __launch_bounds__(kThreads, 6) v_pass_dyn_kernel(const T *__rest
   while (u < nunits) {
     int next = 0;
     if (lane == 0) next = nwarps + atomicAdd(ticket, 1);
-    v_unit(V, units[u], xt, lane);
+    v_unit_any(V, units[u], xt, lane);
     u = __shfl_sync(0xffffffffu, next, 0);
   }
 }
@@ -305,7 +307,10 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 6 : 5) v_pass_direc
   const VUnit U = units[u];
   pdl_wait();  // x is there, and t no longer read
   pdl_trigger();
-  v_unit_direct(V, U, src, xt, threadIdx.x & 31);
+  if (sizeof(T) == 4 && U.sums == 2)
+    v_unit_direct<T, 2>(V, U, src, xt, threadIdx.x & 31);
+  else
+    v_unit_direct<T, 1>(V, U, src, xt, threadIdx.x & 31);
 }
 
 // ---------------------------------------------------------------------------

@@ -64,6 +64,12 @@ static int32_t default_unit_rows(Plan &p, int nwarps) {
   return 16;
 }
 
+// FP32 V rows of up to this many bytes in all: half the lanes per row. Product in us with all
+// lanes / half of them: sphere 20,011 (0.08 GB) 67 / 61, 131,072 (0.94 GB) 368 / 354; batch of 12
+// spheres (1.0 GB) 434 / 425; film 2^19 (1.4 GB) 825 / 831; 131,072-point cube at 1e-4 (2.9 GB)
+// 1511 / 1658; batches of 16 and 32 spheres (3.4 and 7.1 GB) 1287 / 1352 and 2675 / 2852.
+static constexpr int64_t kHalfLanesBytes = int64_t(2) << 30;
+
 void make_vunits(Plan &p, int64_t unit_bytes, int nwarps) {
   const int esize = 16 / p.vec;
   p.vunits.clear();
@@ -77,20 +83,22 @@ void make_vunits(Plan &p, int64_t unit_bytes, int nwarps) {
   // none on small matrices (V pass of a 20,011-point sphere 96 us, now 31 us).
   const int64_t share = bytes / std::max(1, nwarps);
   unit_bytes = std::min(unit_bytes, std::max<int64_t>(1024, std::min(share, std::max<int64_t>(8192, share / 4))));
-  // Lanes per row: a power of two leaving each lane at least this many 16-byte
-  // vectors of the row (at most a warp per row). Fewer lanes per row leave less
-  // idle at the row's end and in the sum over the lanes; in FP64 that counts
-  // more, since the FP64 pipe takes as long for one active lane as for 32. V pass
-  // in us with 4 / 8 / 16 vectors a lane: film 2^20 FP32 580 / 507 / 512, batch of
-  // 12 spheres 113 / 77 / 81; 40,960-point cube FP64 673 / 497 / 372.
-  // FP32 groups of many rank rows (volumes) take 4: their matrices are large, and longer
-  // runs of each row per load count more (cube 2^18 at 1e-6 2245 us with 8, 1894 with 4; cube
-  // 40,960 129 and 133; sphere 20,011, few rows per group, whole product 58.7 and 64.7). The
-  // rule looks at the group alone, so that batches and shards sum every row as its matrix does.
+  // Sums of a row: a power of two, each of at least this many 16-byte vectors of the row in turn
+  // (at most 32), and as many lanes. Fewer lanes per row leave less idle at the row's end and
+  // in the sum over the lanes; in FP64 that counts more, since the FP64 pipe takes as long for
+  // one active lane as for 32: V pass of the 40,960-point cube in us with 4 / 8 / 16 vectors a sum
+  // 673 / 497 / 372. In FP32 half as many lanes may hold two sums each: the same sums, added in
+  // the same order, so that a row does not depend on how many lanes it has, which is
+  // chosen by the size of the whole (a batch, a shard and a matrix differ there).
+  const int32_t sum_vecs = p.vec == 2 ? 16 : 4;
+  const bool halve = p.vec == 4 && bytes <= kHalfLanesBytes;
   for (const VGroup &g : p.vgroups) {
-    const int32_t lane_vecs = p.vec == 2 ? 16 : g.rows >= 512 ? 4 : 8;
-    int32_t nv = g.stride / p.vec, lanes = 1;
-    while (lanes * lane_vecs < nv && lanes < 32) lanes *= 2;
+    int32_t nv = g.stride / p.vec, lanes = 1, sums = 1;
+    while (lanes * sum_vecs < nv && lanes < 32) lanes *= 2;
+    if (halve && lanes > 1 && lanes * sum_vecs >= nv) {  // (rows so long that all lanes have more: a warp each)
+      lanes /= 2;
+      sums = 2;
+    }
     const int64_t row_bytes = static_cast<int64_t>(g.stride) * esize;
     // whole steps of 32 / lanes rows
     const int32_t step = 32 / lanes;
@@ -103,6 +111,7 @@ void make_vunits(Plan &p, int64_t unit_bytes, int nwarps) {
       u.x_off = g.x_off;
       u.t_off = g.t_off + k0;
       u.lanes = lanes;
+      u.sums = sums;
       p.vunits.push_back(u);
       uweight.push_back(row_bytes * u.nrows + 256);
     }
