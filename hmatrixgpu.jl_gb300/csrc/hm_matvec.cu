@@ -18,6 +18,7 @@
 
 #include "hm_device.h"
 #include "hm_launch.cuh"
+#include "hm_per_device.h"
 
 namespace hm {
 
@@ -488,6 +489,19 @@ int occupancy_du(bool f64, bool comp) {
   return n > 0 ? n : 1;
 }
 
+// The ticket form of the V pass runs with a quarter of an SM's L1 as shared memory, of which it needs
+// none. Left to the driver it gets the split of the kernel before it, when the two overlap, and
+// all of the L1 when they do not: a product was faster or slower by up to 0.12 ms in a graph than
+// launched directly (batch of 32 spheres, us launched / in a graph: 2690 / 2615 left to the
+// driver, 2619 / 2615 so; film of 2^20 points 1761 and 1747 launched).
+template <typename T>
+static cudaError_t v_dyn_attrs() {
+  static PerDevice once;
+  return once([] {
+    return cudaFuncSetAttribute(v_pass_dyn_kernel<T>, cudaFuncAttributePreferredSharedMemoryCarveout, 25);
+  });
+}
+
 // Whether n elements at x and m elements at y have memory in common.
 template <typename T>
 static bool overlaps(const T *x, int64_t n, const T *y, int64_t m) {
@@ -517,6 +531,7 @@ static cudaError_t run(const DevPlan &p, const T *panels, const T *vdata, T *xt,
   const XSrc<T> src{xt, x, p.smap0, static_cast<int32_t>(p.x_len)};
   if (ev) cudaEventRecord(ev[1], s);
   if (!p.warp_begin_empty) {
+    if (!direct && p.v_dynamic && (e = v_dyn_attrs<T>()) != cudaSuccess) return e;
     if (direct)
       e = launch_pdl(overlap, v_pass_direct_kernel<T>, (p.nvunits + kThreads / 32 - 1) / (kThreads / 32), kThreads, 0, s,
                      vdata, p.vunits, p.nvunits, src, xt);
