@@ -317,7 +317,7 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 6 : 5) v_pass_direc
 // ---------------------------------------------------------------------------
 // Near/U pass. CTAs take row units (rows of one tile) from a ticket counter
 // (the first one is the CTA's own number, its tables are read while the V pass
-// ends, and the next ticket is drawn while the current unit streams), tiles
+// ends; the next ticket is drawn when a unit is done), tiles
 // with the most columns first. The CTA gathers the tile's vector
 // entries (x for dense columns, t for rank columns) into shared memory once
 // per unit (once per 16 rows when the tile needs several chunks of entries);
@@ -369,8 +369,6 @@ __global__ void __launch_bounds__(kThreads, 6) du_rows_kernel(DuArgs<T> a) {
       pdl_wait();  // t is complete, the ticket is zero
       pdl_trigger();
     }
-    int32_t next = 0;
-    if (!DIRECT && tid == 0) next = static_cast<int32_t>(gridDim.x) + atomicAdd(a.counter, 1);
     // Rows 16 at a time (a warp per row pair); a unit has more than 16 rows
     // only when its tile fits one chunk of entries, which are then gathered
     // once for all its rows.
@@ -463,7 +461,7 @@ __global__ void __launch_bounds__(kThreads, 6) du_rows_kernel(DuArgs<T> a) {
     }
     if (DIRECT) break;  // a unit per CTA
     if (d.ld == 0) __syncthreads();  // no columns, no barrier above: all warps have read the ticket before
-    if (tid == 0) s_ticket = next;
+    if (tid == 0) s_ticket = next_unit(a.counter, gridDim.x, a.nunits);
     __syncthreads();  // the entries and segments are no longer read
     u = s_ticket;
   }

@@ -366,9 +366,6 @@ __global__ void __launch_bounds__(kVWarps * 32, multi_ctas<T, kVWarps>()) v_mult
   bool big = u < nbig;
   if (!big) u = nbig + u * kVWarps + warp;
   while (u < nitems) {  // one loop for both kinds, so that the micro-kernels' code is there once
-    int32_t next = 0;
-    if (big ? tid == 0 : lane == 0)
-      next = (big ? ctas : nbig + ctas * kVWarps) + atomicAdd(counter + kTicket[big ? 1 : 2], 1);
     const MVItem I = items[u];
     T *out = (I.kind == 0 ? xt : P) + static_cast<int64_t>(I.out) * W;
     with_rows<T, W>(I.nrows, [&](auto mt) {
@@ -392,7 +389,7 @@ __global__ void __launch_bounds__(kVWarps * 32, multi_ctas<T, kVWarps>()) v_mult
       }
     });
     if (big) {
-      if (tid == 0) s_ticket = next;
+      if (tid == 0) s_ticket = next_unit(counter + kTicket[1], ctas, nbig);
       __syncthreads();  // the sums are read, the stages may be filled again
       u = s_ticket;
       if (u >= nbig) {
@@ -400,6 +397,8 @@ __global__ void __launch_bounds__(kVWarps * 32, multi_ctas<T, kVWarps>()) v_mult
         u = nbig + static_cast<int32_t>(blockIdx.x) * kVWarps + warp;
       }
     } else {
+      int32_t next = 0;
+      if (lane == 0) next = nbig + next_unit(counter + kTicket[2], ctas * kVWarps, nitems - nbig);
       u = __shfl_sync(0xffffffffu, next, 0);
     }
   }
@@ -491,8 +490,6 @@ __global__ void __launch_bounds__(kDuWarps * 32, multi_ctas<T, kDuWarps>()) du_m
   pdl_trigger();
   for (int32_t u = static_cast<int32_t>(blockIdx.x); u < a.nunits;) {
     const MUnit U = a.units[u];
-    int32_t next = 0;
-    if (tid == 0) next = static_cast<int32_t>(gridDim.x) + atomicAdd(a.counter + kTicket[0], 1);
     const int32_t *map = a.colmap + U.map;
     with_rows<T, W>(U.m, [&](auto mt) {
       using L = LaneTile<T, W, mt.value>;
@@ -506,7 +503,8 @@ __global__ void __launch_bounds__(kDuWarps * 32, multi_ctas<T, kDuWarps>()) du_m
             if (q < a.nr) a.y[a.tmap0[U.row0 + row] + q * a.ldy] = s;
           });
     });
-    if (tid == 0) s_ticket = next;  // (the one before was read by all warps before sum_warps' barriers)
+    // (the ticket before was read by all warps before sum_warps' barriers)
+    if (tid == 0) s_ticket = next_unit(a.counter + kTicket[0], gridDim.x, a.nunits);
     __syncthreads();  // the sums are read, the stages may be filled again
     u = s_ticket;
   }
