@@ -202,6 +202,7 @@ void make_plan(const BlockSet &bs, int vec, int nwarps, const std::vector<int64_
 // units of about `unit_bytes` with their static split over `nwarps` warps: both
 // only partition the stored layout, so they can be rebuilt at any time.
 void make_units(Plan &p, int32_t unit_rows);
+int32_t default_unit_rows(Plan &p, int nwarps);
 void make_vunits(Plan &p, int64_t unit_bytes, int nwarps);
 
 // Plan and block set of the block-diagonal batch of several H-matrices (see

@@ -56,7 +56,7 @@ void make_units(Plan &p, int32_t unit_rows) {
 // that still give each of the resident CTAs two units; 16, two rows per warp, at
 // least. Near/U pass in us with 16 / 64 rows: film 2^20 1427 / 1284, batch of 12
 // spheres 125 / 107; with 24 tiles (1000 points, FP64) 8.2 / 14.
-static int32_t default_unit_rows(Plan &p, int nwarps) {
+int32_t default_unit_rows(Plan &p, int nwarps) {
   for (int32_t rows : {64, 32}) {
     make_units(p, rows);
     if (static_cast<int64_t>(p.units.size()) >= 2 * (nwarps / 8)) return rows;

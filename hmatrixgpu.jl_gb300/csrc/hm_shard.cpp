@@ -111,7 +111,9 @@ static int make_shard(const HMatrix &H, int32_t rank, int32_t world, HMatrix &S)
   std::iota(q.tile_order.begin(), q.tile_order.end(), 0);
   std::stable_sort(q.tile_order.begin(), q.tile_order.end(),
                    [&](int32_t a, int32_t b) { return q.tiles[a].ncols > q.tiles[b].ncols; });
-  make_units(q, p.unit_rows);
+  // the matrix's rows per unit, or fewer: an eighth of its units would leave CTAs idle (last of 8
+  // shards of a film of 300,000 points, in us with 64 / 16 rows: FP64 534 / 512, mixed 174 / 165)
+  make_units(q, std::min(p.unit_rows, default_unit_rows(q, p.nwarps)));
   make_vunits(q, p.vunit_bytes, p.nwarps);
   // ---- device data -------------------------------------------------------------------
   int rc;
@@ -131,9 +133,8 @@ static int make_shard(const HMatrix &H, int32_t rank, int32_t world, HMatrix &S)
   std::vector<int32_t> smap0(static_cast<size_t>(n)), tmap0(static_cast<size_t>(m), -1);
   std::iota(smap0.begin(), smap0.end(), 0);
   for (int64_t r = S.shard_row0; r < S.shard_row1; r++) tmap0[r] = static_cast<int32_t>(r - S.shard_row0);
-  S.dp.v_dynamic = H.dp.v_dynamic;
+  S.dp.v_dynamic = H.dp.v_dynamic && q.v_len * static_cast<int64_t>(es) > kDynamicVBytes;
   if ((rc = upload_plan(S, tmap0, smap0, H.dp.zero_row))) return rc;
-  S.plan.unit_rows = p.unit_rows;
   return setup_grids(S);
 }
 
