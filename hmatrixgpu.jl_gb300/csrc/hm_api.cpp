@@ -159,8 +159,11 @@ int upload_plan(HMatrix &H, const std::vector<int32_t> &tmap0, const std::vector
       }
       if (static_cast<int64_t>(mu.size()) >= want) break;
     }
-    if ((rc = upload(H, &H.dp.munits, mu)) || (rc = upload(H, &H.dp.mcol0, map0))) return rc;
     H.dp.nmunits = static_cast<int32_t>(mu.size());
+    mu.resize(mu.size() + (map0.size() * sizeof(int64_t) + sizeof(MUnit) - 1) / sizeof(MUnit));  // one upload
+    if (!map0.empty()) std::memcpy(static_cast<void *>(mu.data() + H.dp.nmunits), map0.data(), map0.size() * sizeof(int64_t));
+    if ((rc = upload(H, &H.dp.munits, mu))) return rc;
+    H.dp.mcol0 = reinterpret_cast<int64_t *>(H.dp.munits + H.dp.nmunits);
   }
   {  // device order: by first XT row, so pieces reading the same x rows share them in L2
     std::vector<MVItem> ms = p.mv_items;

@@ -660,9 +660,10 @@ static int persistent_grid(F kernel) {
   return std::max(1, sms) * std::max(1, occ);
 }
 
-// The Jacobi SVDs of a batch (or r = k without SVD). `table`: kJacTable + njobs words.
-static cudaError_t launch_jacobi(const AcaJob *jobs, int32_t njobs, double eps, int svd, double *ws, AcaRes *res,
-                                 int32_t *table) {
+// The Jacobi SVDs of a batch of blocks of kmin to kmax terms (or r = k without SVD). `table`: kJacTable +
+// njobs words. Only the launches that some block may need: each costs a lone small block 2 us.
+static cudaError_t launch_jacobi(const AcaJob *jobs, int32_t njobs, int32_t kmin, int32_t kmax, double eps, int svd,
+                                 double *ws, AcaRes *res, int32_t *table) {
   int32_t *ids = table + kJacTable, *ticket = table + 2 * kJacBins;
   jacobi_bins_kernel<<<1, 1024>>>(njobs, svd, res, table, ids);
   if (!svd) return cudaGetLastError();
@@ -670,15 +671,21 @@ static cudaError_t launch_jacobi(const AcaJob *jobs, int32_t njobs, double eps, 
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-  cudaFuncAttributes fa;
-  cudaError_t e = cudaFuncGetAttributes(&fa, jacobi_cta_kernel);
-  if (e != cudaSuccess) return e;
-  const int64_t cap = (most - static_cast<int64_t>(fa.sharedSizeBytes)) / 8;
-  e = cudaFuncSetAttribute(jacobi_cta_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(cap * 8));
-  if (e != cudaSuccess) return e;
-  jacobi_cta_kernel<<<sms, kBuildThreads, cap * 8>>>(jobs, eps, cap, ws, res, table, ids, ticket);
+  cudaError_t e = cudaSuccess;
+  bool behind = false;  // a Jacobi launch, which is complete before it ends, stands before the next
+  if (kmax > kJacGroupMax) {
+    cudaFuncAttributes fa;
+    e = cudaFuncGetAttributes(&fa, jacobi_cta_kernel);
+    if (e != cudaSuccess) return e;
+    const int64_t cap = (most - static_cast<int64_t>(fa.sharedSizeBytes)) / 8;
+    e = cudaFuncSetAttribute(jacobi_cta_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(cap * 8));
+    if (e != cudaSuccess) return e;
+    jacobi_cta_kernel<<<sms, kBuildThreads, cap * 8>>>(jobs, eps, cap, ws, res, table, ids, ticket);
+    behind = true;
+  }
   // The group launches read nothing of one another, nor of the kernel above: each may start as
-  // soon as the CTAs of the one before have started, and takes the SMs as they fall idle.
+  // soon as the CTAs of the one before have started, and takes the SMs as they fall idle. The first
+  // Jacobi launch starts after the bins are there.
   auto words = [](int c) {  // a CTA's groups of k terms hold 2 k (k | 1) + k doubles each
     int64_t w = 0;
     for (int k = jac_class_max(c + 1) + 1; k <= jac_class_max(c); k++)
@@ -693,11 +700,13 @@ static cudaError_t launch_jacobi(const AcaJob *jobs, int32_t njobs, double eps, 
     e = cudaFuncSetAttribute(jacobi_group_kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
                              cudaSharedmemCarveoutMaxShared);
   for (int c = 0; c < kJacClasses && e == cudaSuccess; c++) {
+    if (jac_class_max(c + 1) >= kmax || jac_class_max(c) < kmin) continue;
     int occ = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, jacobi_group_kernel, kJacThreads, words(c) * 8);
     const int64_t grid = std::min<int64_t>(static_cast<int64_t>(sms) * std::max(1, occ), njobs);
-    e = launch_pdl(true, jacobi_group_kernel, dim3(static_cast<unsigned>(grid)), kJacThreads, words(c) * 8, nullptr,
+    e = launch_pdl(behind, jacobi_group_kernel, dim3(static_cast<unsigned>(grid)), kJacThreads, words(c) * 8, nullptr,
                    jobs, jac_class_max(c + 1) + 1, jac_class_max(c), eps, ws, res, table, ids, ticket + 1 + c);
+    behind = true;
   }
   if (e != cudaSuccess) return e;
   return cudaGetLastError();
@@ -793,7 +802,7 @@ struct Compressor {
   int run(std::vector<AcaJob> &jobs, std::vector<AcaRes> &res, const std::vector<int> &sel,
           Keep keep, Place place, After after) {
     size_t pos = 0;
-    DevBuf ws, djobs, dres, dtick, dbins, duo, dvo, dcj, dcr;
+    DevBuf ws, djobs, dres, dtick, duo, dvo, dcj, dcr;
     if (int rc = dtick.alloc(8 * sizeof(int32_t))) return rc;
     const int64_t fill = budget;
     if (resume)  // a quarter more than the batches fill, for the continued blocks
@@ -834,7 +843,7 @@ struct Compressor {
       ws_bytes += used * static_cast<int64_t>(sizeof(double));
       int rc;
       if ((rc = ws.reserve(used * sizeof(double))) || (rc = djobs.reserve(nb * sizeof(AcaJob))) ||
-          (rc = dres.reserve(nb * sizeof(AcaRes))) || (rc = dbins.reserve((kJacTable + nb) * sizeof(int32_t))))
+          (rc = dres.reserve(nb * sizeof(AcaRes) + (kJacTable + nb) * sizeof(int32_t))))  // and the bins
         return rc;
       cudaMemcpy(djobs.p, batch.data(), nb * sizeof(AcaJob), cudaMemcpyHostToDevice);
       cudaMemset(dres.p, 0, nb * sizeof(AcaRes));
@@ -846,8 +855,10 @@ struct Compressor {
       if (resume && (rc = continue_full(batch, used, ws, djobs, dres, dcj, dcr, tk + 6))) return rc;
       qr_kernel<<<grid_qr, kBuildThreads>>>(djobs.as<AcaJob>(), nbig, nb, svd, ws.as<double>(), dres.as<AcaRes>(),
                                          tk + 2);
-      cudaError_t e = launch_jacobi(djobs.as<AcaJob>(), nb, eps_svd, svd, ws.as<double>(), dres.as<AcaRes>(),
-                                    dbins.as<int32_t>());
+      int32_t kmax = 1;
+      for (const AcaJob &j : batch) kmax = std::max(kmax, j.kcap);
+      cudaError_t e = launch_jacobi(djobs.as<AcaJob>(), nb, 1, kmax, eps_svd, svd, ws.as<double>(), dres.as<AcaRes>(),
+                                    reinterpret_cast<int32_t *>(dres.as<AcaRes>() + nb));
       if (e != cudaSuccess) return cuda_fail(e, "Jacobi launch");
       std::vector<AcaRes> hr(nb);
       e = cudaMemcpy(hr.data(), dres.p, nb * sizeof(AcaRes), cudaMemcpyDeviceToHost);
@@ -1304,12 +1315,11 @@ extern "C" int hmgpu_svd_recompress(int64_t m, int64_t n, int64_t k, const doubl
     *r_out = 0;
     return HMGPU_OK;
   }
-  DevBuf dj, dr, dws, dtk, dbins, duo, dvo, dus, dvs;
+  DevBuf dj, dr, dws, dtk, duo, dvo, dus, dvs;
   int rc;
-  if ((rc = dj.alloc(sizeof(AcaJob))) || (rc = dr.alloc(sizeof(AcaRes))) || (rc = dtk.alloc(16)) ||
-      (rc = dws.alloc(ws_doubles(m, n, k) * 8)) || (rc = duo.alloc(8)) || (rc = dvo.alloc(8)) ||
-      (rc = dus.alloc(m * k * 8)) || (rc = dvs.alloc(k * n * 8)) ||
-      (rc = dbins.alloc((kJacTable + 1) * sizeof(int32_t))))
+  if ((rc = dj.alloc(sizeof(AcaJob))) || (rc = dr.alloc(sizeof(AcaRes) + (kJacTable + 1) * sizeof(int32_t))) ||
+      (rc = dtk.alloc(16)) || (rc = dws.alloc(ws_doubles(m, n, k) * 8)) || (rc = duo.alloc(8)) || (rc = dvo.alloc(8)) ||
+      (rc = dus.alloc(m * k * 8)) || (rc = dvs.alloc(k * n * 8)))
     return rc;
   std::vector<double> w(static_cast<size_t>(m * k + k * n));
   for (int64_t i = 0; i < m * k; i++) w[i] = U[i];
@@ -1327,7 +1337,9 @@ extern "C" int hmgpu_svd_recompress(int64_t m, int64_t n, int64_t k, const doubl
   cudaMemcpy(dvo.p, &zero, 8, cudaMemcpyHostToDevice);
   const int big = team_job(j) ? 1 : 0;
   qr_kernel<<<1, kBuildThreads>>>(dj.as<AcaJob>(), big, 1, 1, dws.as<double>(), dr.as<AcaRes>(), dtk.as<int32_t>());
-  cudaError_t e = launch_jacobi(dj.as<AcaJob>(), 1, eps, 1, dws.as<double>(), dr.as<AcaRes>(), dbins.as<int32_t>());
+  const int32_t terms = static_cast<int32_t>(k);
+  cudaError_t e = launch_jacobi(dj.as<AcaJob>(), 1, terms, terms, eps, 1, dws.as<double>(), dr.as<AcaRes>(),
+                                reinterpret_cast<int32_t *>(dr.as<AcaRes>() + 1));
   if (e != cudaSuccess) return cuda_fail(e, "Jacobi launch");
   form_kernel<<<1, kBuildThreads>>>(dj.as<AcaJob>(), big, 1, 1, dws.as<double>(), dr.as<AcaRes>(),
                                     duo.as<int64_t>(), dvo.as<int64_t>(), dus.as<double>(), dvs.as<double>(),
