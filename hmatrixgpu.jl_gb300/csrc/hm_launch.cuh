@@ -18,10 +18,14 @@ __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.lau
 // Whether the kernels of a pass of `columns` right-hand sides over `entries` stored entries may
 // overlap: always in FP32. The CTAs of a kernel that starts while another ends land where there is
 // room, several on one SM while others get none; that is made good where memory bounds the
-// kernel, but not the FP64 pipe of the SMs (product of a 5266-point cube with 6 right-hand sides 805
-// us with overlap, 452 without; 1000 points on a circle 15.2 and 18.8). So in FP64 only while the
-// pipe's time, 2 FMAs per clock and SM, is short beside the launches.
-inline bool may_overlap(bool f64, int64_t entries, int columns) { return !f64 || entries * columns < 6000000; }
+// kernel, but not the FP64 pipe of the SMs. So in FP64 only while the launches are a good part of the
+// time. Product in us with / without overlap, one column: 1000-point cube (0.99 M entries) 14.1 / 18.5,
+// film of 2000 (1.8 M) 17.6 / 22.6, sphere of 4000 (5.8 M) 41.8 / 30.8, 3000-point cube (7.3 M) 62.3 /
+// 38.3; passes 4 to 32 wide, entries times width: 22 M 93.0 / 98.4, 29 M 79.5 / 85.9, 43 M 179.7 / 129.1, 81 M
+// 341 / 219.
+inline bool may_overlap(bool f64, int64_t entries, int columns) {
+  return !f64 || entries * columns < (columns == 1 ? 2000000 : 30000000);
+}
 
 // A launch that may overlap the end of the kernel before it (`overlap`).
 template <typename... P, typename... A>

@@ -101,10 +101,12 @@ struct RowAcc {
   }
 };
 
-// The vector that the two passes read: XT = [x permuted | t], or, for a matrix whose V
-// and near/U units all fit the resident warps and CTAs (DIRECT), x itself through the source map
-// in place of its permuted copy: one launch less, where launches are most of the time (1000
-// points, FP64: 9.1 us, 11.6 with the permutation), and no tickets, since every unit has a warp or CTA of its own.
+// The vector that the two passes read: XT = [x permuted | t], or, for a matrix with no more V units
+// than resident warps of the V pass and no more near/U units than resident CTAs (DIRECT), x itself
+// through the source map in place of its permuted copy: one launch less, where launches are most of
+// the time (1000 points, FP64: 9.1 us, 11.6 with the permutation), and no tickets, since every
+// unit has a warp or CTA of its own. (In FP64 the direct V kernel has five CTAs per SM, not six: the last
+// few may start later, and nothing waits for them but the near/U pass.)
 template <typename T>
 struct XSrc {
   const T *xt;

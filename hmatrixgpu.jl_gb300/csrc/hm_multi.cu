@@ -564,8 +564,10 @@ int multi_width(bool f64, int nr) { return nr <= 4 && f64 ? 4 : nr <= 8 ? 8 : nr
 
 // FP32 passes are as wide as they can be: they read the matrix once. In FP64 a pass's time is
 // that of the FP64 pipe, in proportion to its width, beside some 12 us of launches and latency, so the
-// columns are split into the widths with the least sum of both (18 columns of a million
-// entries or more: 16 and 4 wide, not 32). A row's sum does not depend on the width.
+// columns are split into the widths with the least sum of both. 18 columns in one 32-wide pass / as
+// chosen, in us: 2000 points on a circle (0.47 M entries) 104 / one pass, 1000-point cube (0.99 M) 94 / 73
+// (16 and 4 wide), film of 30,000 (59 M) 4043 / 2609. The worst seen: circle of 20,000, where V rows are long
+// and the pipe is not the bound, 28 columns 911 / 951. A row's sum does not depend on the width.
 int multi_pass_columns(bool f64, int64_t left, int64_t entries, int num_sms) {
   if (!f64 || left >= kRhs) return static_cast<int>(left < kRhs ? left : kRhs);
   const double column = static_cast<double>(entries) / (2.0 * num_sms * 1900.0);  // us of the FP64 pipe per column
