@@ -34,8 +34,8 @@ METRIC = "H-matvec/s at N=2^20, 1 & 32 RHS: mixed vs plain FP32 at equal err; HB
 WORKLOAD = "film-2^20 Laplace leaf64 eta2 tol1e-4, 1 RHS, FP32 storage"
 GRID, LEAF, ETA, TOL = 1024, 64, 2.0, 1e-4
 # DRAM traffic / algorithmic bytes of the near/U kernel, from an ncu capture on
-# film 512 x 512 (1983.5 MB of dram__bytes_read + write for 1952.3 MB algorithmic)
-TRAFFIC_RATIO = 1983.5 / 1952.3
+# film 512 x 512 (1984.2 MB of dram__bytes_read + write for 1952.3 MB algorithmic)
+TRAFFIC_RATIO = 1984.2 / 1952.3
 
 
 def peaks():
@@ -768,7 +768,7 @@ def run_gpu(args):
                      "peak_source": src, "algorithmic_bytes_per_launch": du_bytes,
                      "traffic": du_bytes * TRAFFIC_RATIO,
                      "traffic_source": "ncu dram__bytes_read+write of du_rows_kernel on film 512x512 "
-                                       "(1983.5 MB for 1952.3 MB algorithmic), scaled by algorithmic bytes "
+                                       "(1984.2 MB for 1952.3 MB algorithmic), scaled by algorithmic bytes "
                                        "(profiles/du_rows_v_pass_film512.md)"},
         "cpu_baseline": {"value": cpu_runs[1]["value"], "unit": "matvec/s", "cores": 1, "kind": "port",
                          "sample": cpu_desc + f"; {cpu_runs[1]['steps']} timed products on one core",

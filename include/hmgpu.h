@@ -205,7 +205,8 @@ int hmgpu_hmatrix_build(const hmgpu_options *opt, const hmgpu_kernel *K, const h
 /* mul!(y, H, x) (src/mult.jl:159-189) for nrhs right-hand sides: x is n x nrhs
  * and y is m x nrhs, column-major with leading dimensions ldx >= n and
  * ldy >= m, device pointers of the mode's element type (double for HMGPU_F64,
- * float otherwise).  y is overwritten in the original (unpermuted) order.
+ * float otherwise).  y is overwritten in the original (unpermuted) order; it may
+ * be x itself (with ldy = ldx).
  * Stream-ordered on `stream` (a cudaStream_t; NULL = the legacy default
  * stream); returns without synchronising. */
 int hmgpu_matvec(hmgpu_hmatrix *H, const void *x, void *y, int64_t nrhs, int64_t ldx,
