@@ -474,10 +474,10 @@ int occupancy_du(bool f64, bool comp) {
 }
 
 // The ticket form of the V pass runs with a quarter of an SM's L1 as shared memory, of which it needs
-// none. Left to the driver it gets the split of the kernel before it, when the two overlap, and
+// none. Left unset it gets the split of the kernel before it, when the two overlap, and
 // all of the L1 when they do not: a product was faster or slower by up to 0.12 ms in a graph than
-// launched directly (batch of 32 spheres, us launched / in a graph: 2690 / 2615 left to the
-// driver, 2619 / 2615 so; film of 2^20 points 1761 and 1747 launched).
+// launched directly (batch of 32 spheres, us launched / in a graph: 2690 / 2615 left
+// unset, 2619 / 2615 so; film of 2^20 points 1761 and 1747 launched).
 template <typename T>
 static cudaError_t v_dyn_attrs() {
   static PerDevice once;

@@ -18,7 +18,7 @@
 // Measured on a film of 262,144 points (633 M stored entries, FP32), us per product with 32,
 // 16 and 8 right-hand sides: 1039, 647 and 558, against 2336 for the form before (CTA-wide
 // stages, 4 x 8 or 2 x 16 tiles, panel entries straight from global memory: L1-bound). The
-// FMAs alone take 580 at the card's FP32 rate, the entries' bytes 374.
+// FMAs alone take 633 at 32 TFMA/s, the entries' bytes 374.
 #include <cuda_runtime.h>
 
 #include <type_traits>
