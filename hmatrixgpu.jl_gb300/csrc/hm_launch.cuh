@@ -20,11 +20,11 @@ __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.lau
 // room, several on one SM while others get none; that is made good where memory bounds the
 // kernel, but not the FP64 pipe of the SMs. So in FP64 only while the launches are a good part of the
 // time. Product in us with / without overlap, one column: 1000-point cube (0.99 M entries) 14.1 / 18.5,
-// film of 2000 (1.8 M) 17.6 / 22.6, sphere of 4000 (5.8 M) 41.8 / 30.8, 3000-point cube (7.3 M) 62.3 /
-// 38.3; passes 4 to 32 wide, entries times width: 22 M 93.0 / 98.4, 29 M 79.5 / 85.9, 43 M 179.7 / 129.1, 81 M
-// 341 / 219.
+// film of 3000 (2.7 M) 19.6 / 21.7, 1800-point cube (2.88 M) 23.1 / 24.6, sphere of 2500 (3.00 M) 31.9 / 23.6,
+// 2500-point cube (5.0 M) 49.8 / 32.1; passes 4 to 32 wide, entries times width: 22 M 93.0 / 98.4, 29 M 79.5 /
+// 85.9, 43 M 179.7 / 129.1 and 123.0 / 127.1, 81 M 341 / 219.
 inline bool may_overlap(bool f64, int64_t entries, int columns) {
-  return !f64 || entries * columns < (columns == 1 ? 2000000 : 30000000);
+  return !f64 || entries * columns < (columns == 1 ? 2900000 : 30000000);
 }
 
 // A launch that may overlap the end of the kernel before it (`overlap`).
